@@ -88,6 +88,12 @@ static void axis_tables(int n, int count, std::vector<float>& q2, std::vector<fl
   }
 }
 
+// Strides of kx and z in the mixed-space arrays Sm, D and J (y contiguous).
+static void mixed_strides(int Nx, int Ny, int Nz, int& ks, int& zs) {
+  ks = Ny * Nz;
+  zs = Ny;
+}
+
 struct DevTables {
   void* base = nullptr;
   Shape sh;
@@ -119,6 +125,7 @@ static int build_tables(int Nx, int Ny, int Nz, DevTables& t) {
   Shape& s = t.sh;
   s.Nx = Nx; s.Ny = Ny; s.Nz = Nz; s.Kx = Kx;
   s.plane0 = 0;
+  mixed_strides(Nx, Ny, Nz, s.ks, s.zs);
   s.pref_yz = 0;
   s.par = 0;
   s.twM = (const float2*)(b + off_tw[0]);
@@ -176,11 +183,11 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // Tensor map over a run's mixed-space state Sm [nF][Kx][Nz][Ny] (8-byte
 // complex elements) with box {wy rows, 1 z, Kx, 1 field}: one TMA copy brings
 // the half spectra of wy rows of one field at one z.
-static int encode_sm_map(void* Sm, int Ny, int Nz, int Kx, int nF, int wy, CUtensorMap* out) {
+static int encode_sm_map(void* Sm, int Ny, int Nz, int Kx, int nF, int ks, int zs, int wy, CUtensorMap* out) {
   const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
   if (!fn) return fail(PF_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const cuuint64_t dims[4] = {(cuuint64_t)Ny, (cuuint64_t)Nz, (cuuint64_t)Kx, (cuuint64_t)nF};
-  const cuuint64_t strides[3] = {(cuuint64_t)Ny * 8, (cuuint64_t)Ny * Nz * 8, (cuuint64_t)Kx * Ny * Nz * 8};
+  const cuuint64_t strides[3] = {(cuuint64_t)zs * 8, (cuuint64_t)ks * 8, (cuuint64_t)Kx * Ny * Nz * 8};
   const cuuint32_t box[4] = {(cuuint32_t)wy, 1, (cuuint32_t)Kx, 1};
   const cuuint32_t es[4] = {1, 1, 1, 1};
   const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, Sm, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -533,7 +540,7 @@ static bool x_ok(pf_batch* b, const XKernels& k) {
     const size_t sb = k.bulk_smem(b->nF);
     CUtensorMap probe;
     if (sb > kMaxSmem || (k.wy * 8) % 16 != 0 || b->Kx > 256 ||
-        encode_sm_map(b->hrp[0].Sm, b->Ny, b->Nz, b->Kx, b->nF, k.wy, &probe) != PF_OK ||
+        encode_sm_map(b->hrp[0].Sm, b->Ny, b->Nz, b->Kx, b->nF, b->tab.sh.ks, b->tab.sh.zs, k.wy, &probe) != PF_OK ||
         !raise_smem((const void*)k.bulk, sb))
       return false;
   }
@@ -591,7 +598,7 @@ static void apply_xj(pf_batch* b, const XKernels& k) {
 static int write_tensor_maps(pf_batch* b, int wy) {
   for (int r = 0; r < b->nruns; ++r) {
     CUtensorMap m;
-    const int rc = encode_sm_map(b->hrp[r].Sm, b->Ny, b->Nz, b->Kx, b->nF, wy, &m);
+    const int rc = encode_sm_map(b->hrp[r].Sm, b->Ny, b->Nz, b->Kx, b->nF, b->tab.sh.ks, b->tab.sh.zs, wy, &m);
     if (rc) return rc;
     b->tmaps[r] = m;
   }

@@ -42,7 +42,21 @@ PF_HD float2 csub(float2 a, float2 b) {
   return make_float2(a.x - b.x, a.y - b.y);
 #endif
 }
-PF_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// s * a and s * a + b: one packed instruction each on the device
+PF_HD float2 cscale(float2 a, float s) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  return __fmul2_rn(a, make_float2(s, s));
+#else
+  return make_float2(a.x * s, a.y * s);
+#endif
+}
+PF_HD float2 cfma(float s, float2 a, float2 b) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+  return __ffma2_rn(make_float2(s, s), a, b);
+#else
+  return make_float2(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y));
+#endif
+}
 PF_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 // a * b
 PF_HD float2 cmul(float2 a, float2 b) {
@@ -154,7 +168,7 @@ struct Dft<3> {
     float2 a = v[0];
     float2 t1 = cadd(v[1], v[2]);
     float2 t2 = csub(v[1], v[2]);
-    float2 m = make_float2(fmaf(-0.5f, t1.x, a.x), fmaf(-0.5f, t1.y, a.y));
+    float2 m = cfma(-0.5f, t1, a);
     float2 s = cscale(t2, PF_SQRT3_2);
     v[0] = cadd(a, t1);
     v[1] = cadd(m, cmul_mi(s));
@@ -193,10 +207,10 @@ struct Dft<5> {
     const float2 x0 = v[0];
     const float2 t1 = cadd(v[1], v[4]), d1 = csub(v[1], v[4]);
     const float2 t2 = cadd(v[2], v[3]), d2 = csub(v[2], v[3]);
-    const float2 a1 = make_float2(fmaf(c2, t2.x, fmaf(c1, t1.x, x0.x)), fmaf(c2, t2.y, fmaf(c1, t1.y, x0.y)));
-    const float2 a2 = make_float2(fmaf(c1, t2.x, fmaf(c2, t1.x, x0.x)), fmaf(c1, t2.y, fmaf(c2, t1.y, x0.y)));
-    const float2 b1 = make_float2(fmaf(s2, d2.x, s1 * d1.x), fmaf(s2, d2.y, s1 * d1.y));
-    const float2 b2 = make_float2(fmaf(-s1, d2.x, s2 * d1.x), fmaf(-s1, d2.y, s2 * d1.y));
+    const float2 a1 = cfma(c2, t2, cfma(c1, t1, x0));
+    const float2 a2 = cfma(c1, t2, cfma(c2, t1, x0));
+    const float2 b1 = cfma(s2, d2, cscale(d1, s1));
+    const float2 b2 = cfma(-s1, d2, cscale(d1, s2));
     v[0] = cadd(x0, cadd(t1, t2));
     v[1] = cadd(a1, cmul_mi(b1));
     v[4] = cadd(a1, cmul_pi(b1));
@@ -231,8 +245,8 @@ struct Dft<17> {
         const int m = (j * k) % 17;
         const int mm = m <= 8 ? m : 17 - m;
         const float sn = m <= 8 ? S[mm] : -S[mm];
-        a = make_float2(fmaf(C[mm], t[j].x, a.x), fmaf(C[mm], t[j].y, a.y));
-        b = make_float2(fmaf(sn, d[j].x, b.x), fmaf(sn, d[j].y, b.y));
+        a = cfma(C[mm], t[j], a);
+        b = cfma(sn, d[j], b);
       }
       out[k] = make_float2(a.x + b.y, a.y - b.x);
       out[17 - k] = make_float2(a.x - b.y, a.y + b.x);
@@ -242,6 +256,30 @@ struct Dft<17> {
     for (int k = 1; k < 17; ++k) v[k] = out[k];
   }
 };
+
+// v * W_R^j (INV: its conjugate) for a j known after unrolling.  Multiples of
+// a quarter turn cost no arithmetic and odd eighths two adds and a packed
+// multiply; left to a general complex multiply they cost four instructions
+// each, since the compiler may not drop a product with zero.  They are 3 of
+// DFT_8's 3 twiddles and 5 of DFT_16's 9.
+template <int R, bool INV>
+PF_HD float2 rot(float2 v, int j) {
+  const int e = (INV ? R - j % R : j % R) % R;  // e / R turns, clockwise
+  if (8 * e % R != 0) {
+    const float2 w = wconst<R>(j);
+    return INV ? cmulc(v, w) : cmul(v, w);
+  }
+  switch (8 * e / R) {
+    case 0: return v;
+    case 1: return cscale(make_float2(v.x + v.y, v.y - v.x), PF_SQRT1_2);
+    case 2: return cmul_mi(v);
+    case 3: return cscale(make_float2(v.y - v.x, -v.x - v.y), PF_SQRT1_2);
+    case 4: return make_float2(-v.x, -v.y);
+    case 5: return cscale(make_float2(-v.x - v.y, v.x - v.y), PF_SQRT1_2);
+    case 6: return cmul_pi(v);
+    default: return cscale(make_float2(v.x - v.y, v.x + v.y), PF_SQRT1_2);
+  }
+}
 
 // Composite R = R1*R2 in registers: x[n1 + R1*n2] -> X[k2 + R2*k1]
 template <int R1, int R2>
@@ -258,10 +296,7 @@ struct DftComposite {
       if constexpr (INV) dft_inv<R2>(c);
       else Dft<R2>::fwd(c);
 #pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) {
-        float2 w = wconst<R>(n1 * k2);
-        t[n1 + R1 * k2] = (n1 * k2 == 0) ? c[k2] : (INV ? cmulc(c[k2], w) : cmul(c[k2], w));
-      }
+      for (int k2 = 0; k2 < R2; ++k2) t[n1 + R1 * k2] = rot<R, INV>(c[k2], n1 * k2);
     }
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) {

@@ -89,6 +89,7 @@ struct Shape {
   int nblk_x;   // blocks of the x pass per run
   int nblk_yz;  // blocks of the yz pass per run
   int plane0;   // first (field, kx) plane of a yz-pass launch (a launch may cover a subset)
+  int ks, zs;   // strides of kx and z in Sm, D and J (y contiguous; see mixed_strides)
   // L2 prefetch distance in CTAs of the yz variants that prefetch: the CTAs
   // resident at once, so that CTA b fetches into L2 what CTA b + pref (which
   // starts about when b ends) will read; 0: none
@@ -175,30 +176,27 @@ __device__ __forceinline__ float warp_max(float v) {
 // so that IDFT_M(Z') = N z.  Frequencies k and M-k always sit in mirrored
 // runs of the four-step layout, so one thread owns both halves of every pair.
 // ---------------------------------------------------------------------------
-// inverse pre-processing of the pair (k, M-k), 0 < k < M.  With
-// s = x_k + conj(x_m), d = x_k - conj(x_m):
-//   z_k = s + i d conj(w_k),   z_m = conj(s) + i (-conj(d)) conj(w_m);
-// the rotated products are formed directly in their final component order so
-// that the sums are packed FP32-pair instructions.
-__device__ __forceinline__ void pre_pair(float2 xk, float2 xm, float2 wk, float2 wm, float2& zk, float2& zm) {
+// Since W_N^(M-k) = -conj(W_N^k), the two halves of a pair share one product:
+// inverse pre-processing of the pair (k, M-k), 0 < k < M, with
+// s = x_k + conj(x_m), d = x_k - conj(x_m), e = i d conj(w_k):
+//   z_k = s + e,   z_m = conj(s - e)
+// (one twiddle and 9 instructions a pair; two products took two and 12).
+__device__ __forceinline__ void pre_pair(float2 xk, float2 xm, float2 wk, float2& zk, float2& zm) {
   const float2 s = __ffma2_rn(xm, make_float2(1.f, -1.f), xk);
   const float2 d = __ffma2_rn(xm, make_float2(-1.f, 1.f), xk);
-  const float2 ie = make_float2(fmaf(d.x, wk.y, -d.y * wk.x), fmaf(d.x, wk.x, d.y * wk.y));     // i d conj(wk)
-  const float2 ie2 = make_float2(fmaf(-d.y, wm.x, -d.x * wm.y), fmaf(-d.x, wm.x, d.y * wm.y));  // i (-conj d) conj(wm)
-  zk = __fadd2_rn(s, ie);
-  zm = __ffma2_rn(s, make_float2(1.f, -1.f), ie2);
+  const float2 e = make_float2(fmaf(d.x, wk.y, -d.y * wk.x), fmaf(d.x, wk.x, d.y * wk.y));  // i d conj(wk)
+  zk = __fadd2_rn(s, e);
+  zm = make_float2(s.x - e.x, e.y - s.y);
 }
 // forward post-processing of the pair (k, M-k), 0 < k < M, scaled by h = scale/2:
-//   x_k = h (s - i d w_k),   x_m = h (conj(s) - i (-conj(d)) w_m),
-// s = z_k + conj(z_m), d = z_k - conj(z_m).
-__device__ __forceinline__ void post_pair(float2 zk, float2 zm, float2 wk, float2 wm, float h, float2& xk, float2& xm) {
-  const float2 hh = make_float2(h, h);
+// with s = z_k + conj(z_m), d = z_k - conj(z_m), e = -i d w_k:
+//   x_k = h (s + e),   x_m = h conj(s - e).
+__device__ __forceinline__ void post_pair(float2 zk, float2 zm, float2 wk, float h, float2& xk, float2& xm) {
   const float2 s = __ffma2_rn(zm, make_float2(1.f, -1.f), zk);
   const float2 d = __ffma2_rn(zm, make_float2(-1.f, 1.f), zk);
-  const float2 mie = make_float2(fmaf(d.x, wk.y, d.y * wk.x), fmaf(-d.x, wk.x, d.y * wk.y));    // -i d wk
-  const float2 mie2 = make_float2(fmaf(-d.x, wm.y, d.y * wm.x), fmaf(d.x, wm.x, d.y * wm.y));   // -i (-conj d) wm
-  xk = __fmul2_rn(__fadd2_rn(s, mie), hh);
-  xm = __fmul2_rn(__ffma2_rn(s, make_float2(1.f, -1.f), mie2), hh);
+  const float2 e = make_float2(fmaf(d.x, wk.y, d.y * wk.x), fmaf(-d.x, wk.x, d.y * wk.y));  // -i d wk
+  xk = __fmul2_rn(__fadd2_rn(s, e), make_float2(h, h));
+  xm = __fmul2_rn(make_float2(s.x - e.x, e.y - s.y), make_float2(h, h));
 }
 
 // Factorization of the x pass's lines (M = Nx/2 complex points): the plan's,
@@ -224,36 +222,68 @@ __device__ __forceinline__ float2 ldtw(const float2* p) {
   else return __ldg(p);
 }
 
+// One pass-A item: the N2 elements of column n1 of the line at p (column
+// included), twiddles w(k2) = W_L^(n1 k2).
+template <int N1, int N2, int STRIDE, bool INV, class Tw>
+__device__ __forceinline__ void passA_item(float2* p, const Tw& w) {
+  float2 v[N2];
+  if (!INV) {
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[n2 * STRIDE];
+    Dft<N2>::fwd(v);
+#pragma unroll
+    for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmul(v[k2], w(k2));
+  } else {
+    v[0] = p[0];
+#pragma unroll
+    for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmulc(p[k2 * STRIDE], w(k2));
+    dft_inv<N2>(v);
+  }
+#pragma unroll
+  for (int k = 0; k < N2; ++k) p[k * STRIDE] = v[k];
+}
+
 // pass A over a runtime number of lines (pitch P, T threads).  A warp takes 32
 // consecutive lines at one column n1: with an odd pitch those 32 accesses hit
-// distinct bank pairs.
+// distinct bank pairs.  Where the CTA's warps are a multiple of N1, a warp
+// keeps one column and loads its twiddles once; the lines beyond the last
+// whole 32 are spread over (line, column), so that they cost rem N1 / 32
+// warp items instead of N1 (17 fields x 8 rows: 136 lines, 34 items, not 40).
 template <int L, int P, int T, bool INV, bool TWS = false>
 __device__ __forceinline__ void passA_rt(float2* buf, int NL, const float2* __restrict__ tw) {
-  constexpr int N1 = XLine<L>::N1, N2 = XLine<L>::N2;
-  const int nlb = (NL + 31) >> 5;  // groups of 32 lines
-  const int items = nlb * 32 * N1;
-  for (int it = threadIdx.x; it < items; it += T) {
-    const int lo = it & 31, rest = it >> 5;
-    const int n1 = rest % N1, l = (rest / N1) * 32 + lo;
-    if (l >= NL) continue;
-    float2* p = buf + l * P + n1;
-    float2 v[N2];
-    if (!INV) {
+  constexpr int N1 = XLine<L>::N1, N2 = XLine<L>::N2, NW = T / 32;
+  if constexpr (NW % N1 == 0) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n1 = w % N1;
+    float2 wt[N2];
 #pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[n2 * (N1 + 1)];
-      Dft<N2>::fwd(v);
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmul(v[k2], ldtw<TWS>(tw + n1 * k2));
-    } else {
-      v[0] = p[0];
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmulc(p[k2 * (N1 + 1)], ldtw<TWS>(tw + n1 * k2));
-      dft_inv<N2>(v);
+    for (int k2 = 1; k2 < N2; ++k2) wt[k2] = ldtw<TWS>(tw + n1 * k2);
+    const int full = NL & ~31;
+    for (int l = (w / N1) * 32 + lane; l < full; l += 32 * (NW / N1))
+      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + n1, [&](int k2) { return wt[k2]; });
+    const int rem = NL - full;
+    if ((int)threadIdx.x < rem * N1) {
+      const int m1 = threadIdx.x / rem, l = full + (int)threadIdx.x - m1 * rem;
+      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + m1, [&](int k2) { return ldtw<TWS>(tw + m1 * k2); });
     }
-#pragma unroll
-    for (int k = 0; k < N2; ++k) p[k * (N1 + 1)] = v[k];
+  } else {
+    const int nlb = (NL + 31) >> 5;  // groups of 32 lines
+    const int items = nlb * 32 * N1;
+    for (int it = threadIdx.x; it < items; it += T) {
+      const int lo = it & 31, rest = it >> 5;
+      const int n1 = rest % N1, l = (rest / N1) * 32 + lo;
+      if (l >= NL) continue;
+      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + n1, [&](int k2) { return ldtw<TWS>(tw + n1 * k2); });
+    }
   }
 }
+
+// Division of small counts by a count n fixed for the kernel: a multiply
+// (exact for x n < 2^32) instead of about 20 instructions.
+struct FastDiv {
+  unsigned n, magic;
+  __device__ __forceinline__ explicit FastDiv(int n_) : n(n_), magic(0xffffffffu / (unsigned)n_ + 1u) {}
+  __device__ __forceinline__ int operator()(int x) const { return n == 1 ? x : (int)__umulhi((unsigned)x, magic); }
+};
 
 // Where element kx of a line's half spectrum is read from:
 //   SPEC_GLOBAL  src + kx * stride in read-only global memory;
@@ -270,11 +300,12 @@ __device__ __forceinline__ int x_spec_slot(int kx) {
   return kx == M ? N1 : (N1 + 1) * (kx % N2) + kx / N2;
 }
 
+// Element k1 of run r: kx = r + N2 k1, step = N2 strides of kx.
 template <int SRC, int M>
-__device__ __forceinline__ float2 ld_spec(const float2* src, size_t stride, int kx) {
-  if constexpr (SRC == SPEC_INPLACE) return src[x_spec_slot<M>(kx)];
-  else if constexpr (SRC == SPEC_SMEM) return src[(size_t)kx * stride];
-  else return __ldg(src + (size_t)kx * stride);
+__device__ __forceinline__ float2 ld_spec(const float2* src, int step, int r, int k1) {
+  if constexpr (SRC == SPEC_INPLACE) return src[(XLine<M>::N1 + 1) * r + k1];
+  else if constexpr (SRC == SPEC_SMEM) return src[k1 * step];
+  else return __ldg(src + (ptrdiff_t)k1 * step);
 }
 
 // Run pair of item group q of a line (x_inv_runs / x_fwd_runs), q < N2/2 + 1:
@@ -292,22 +323,25 @@ __device__ __forceinline__ int x_run_pair(int q) {
 // for the run pair `pr` (from where SRC says), pre-process, inverse DFT_N1 of
 // each run, store the runs (pass B' output) into the padded line.
 template <int M, int SRC = SPEC_GLOBAL, bool TWS = false>
-__device__ __forceinline__ void x_inv_runs(const float2* src, size_t plane, float2* line, int pr,
+__device__ __forceinline__ void x_inv_runs(const float2* src, int ks, float2* line, int pr,
                                            const float2* __restrict__ twN) {  // src may be line (in place)
   constexpr int N1 = XLine<M>::N1, N2 = XLine<M>::N2;
+  const int step = N2 * ks;
+  const auto run = [&](int r) { return SRC == SPEC_INPLACE ? src : src + r * ks; };
   if (pr > 0 && 2 * pr < N2) {
     const int ra = pr, rb = N2 - pr;
+    const float2 *sa = run(ra), *sb = run(rb);
     float2 a[N1], b[N1];
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) {
-      a[k1] = ld_spec<SRC, M>(src, plane, ra + N2 * k1);
-      b[k1] = ld_spec<SRC, M>(src, plane, rb + N2 * k1);
+      a[k1] = ld_spec<SRC, M>(sa, step, ra, k1);
+      b[k1] = ld_spec<SRC, M>(sb, step, rb, k1);
     }
     float2 za[N1], zb[N1];
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) {
       const int k = ra + N2 * k1;
-      pre_pair(a[k1], b[N1 - 1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), za[k1], zb[N1 - 1 - k1]);
+      pre_pair(a[k1], b[N1 - 1 - k1], ldtw<TWS>(twN + k), za[k1], zb[N1 - 1 - k1]);
     }
     dft_inv<N1>(za);
     dft_inv<N1>(zb);
@@ -319,15 +353,15 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, size_t plane, floa
   } else if (pr == 0) {
     float2 a[N1];
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) a[k1] = ld_spec<SRC, M>(src, plane, N2 * k1);
-    const float2 xM = ld_spec<SRC, M>(src, plane, M);
+    for (int k1 = 0; k1 < N1; ++k1) a[k1] = ld_spec<SRC, M>(src, step, 0, k1);
+    const float2 xM = ld_spec<SRC, M>(src, step, 0, N1);  // kx = M
     float2 z[N1];
     z[0] = make_float2(a[0].x + xM.x, a[0].x - xM.x);
 #pragma unroll
     for (int k1 = 1; k1 <= N1 / 2; ++k1) {
       const int k = N2 * k1;
       float2 zk, zm;
-      pre_pair(a[k1], a[N1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), zk, zm);
+      pre_pair(a[k1], a[N1 - k1], ldtw<TWS>(twN + k), zk, zm);
       z[k1] = zk;
       if (k1 != N1 - k1) z[N1 - k1] = zm;
     }
@@ -336,14 +370,15 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, size_t plane, floa
     for (int n1 = 0; n1 < N1; ++n1) line[n1] = z[n1];
   } else {  // pr == N2/2: the run pairs with itself, element k1 with N1-1-k1
     const int ra = N2 / 2;
+    const float2* sa = run(ra);
     float2 a[N1];
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) a[k1] = ld_spec<SRC, M>(src, plane, ra + N2 * k1);
+    for (int k1 = 0; k1 < N1; ++k1) a[k1] = ld_spec<SRC, M>(sa, step, ra, k1);
     float2 z[N1];
 #pragma unroll
     for (int k1 = 0; k1 < N1 / 2; ++k1) {
       const int k = ra + N2 * k1;
-      pre_pair(a[k1], a[N1 - 1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), z[k1], z[N1 - 1 - k1]);
+      pre_pair(a[k1], a[N1 - 1 - k1], ldtw<TWS>(twN + k), z[k1], z[N1 - 1 - k1]);
     }
     dft_inv<N1>(z);
 #pragma unroll
@@ -354,9 +389,10 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, size_t plane, floa
 // Forward x transform, last half: forward DFT_N1 of the run pair `pr` (pass
 // B), post-process, store the half spectrum (scaled) to global.
 template <int M, bool TWS = false>
-__device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, size_t plane, const float2* line, int pr,
+__device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, const float2* line, int pr,
                                            float scale, const float2* __restrict__ twN) {
   constexpr int N1 = XLine<M>::N1, N2 = XLine<M>::N2;
+  const int step = N2 * ks;
   const float h = 0.5f * scale;
   if (pr > 0 && 2 * pr < N2) {
     const int ra = pr, rb = N2 - pr;
@@ -368,13 +404,14 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, size_t plan
     }
     Dft<N1>::fwd(za);
     Dft<N1>::fwd(zb);
+    float2 *da = dst + ra * ks, *db = dst + rb * ks;
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) {
       const int k = ra + N2 * k1;
       float2 xk, xm;
-      post_pair(za[k1], zb[N1 - 1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), h, xk, xm);
-      dst[(size_t)k * plane] = xk;
-      dst[(size_t)(M - k) * plane] = xm;
+      post_pair(za[k1], zb[N1 - 1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
+      da[(ptrdiff_t)k1 * step] = xk;
+      db[(ptrdiff_t)(N1 - 1 - k1) * step] = xm;  // kx = M - k
     }
   } else if (pr == 0) {
     float2 z[N1];
@@ -382,17 +419,18 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, size_t plan
     for (int n1 = 0; n1 < N1; ++n1) z[n1] = line[n1];
     Dft<N1>::fwd(z);
     dst[0] = make_float2((z[0].x + z[0].y) * scale, 0.f);
-    dst[(size_t)M * plane] = make_float2((z[0].x - z[0].y) * scale, 0.f);
+    dst[(ptrdiff_t)N1 * step] = make_float2((z[0].x - z[0].y) * scale, 0.f);  // kx = M
 #pragma unroll
     for (int k1 = 1; k1 <= N1 / 2; ++k1) {
       const int k = N2 * k1;
       float2 xk, xm;
-      post_pair(z[k1], z[N1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), h, xk, xm);
-      dst[(size_t)k * plane] = xk;
-      if (k1 != N1 - k1) dst[(size_t)(M - k) * plane] = xm;
+      post_pair(z[k1], z[N1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
+      dst[(ptrdiff_t)k1 * step] = xk;
+      if (k1 != N1 - k1) dst[(ptrdiff_t)(N1 - k1) * step] = xm;
     }
   } else {
     const int ra = N2 / 2;
+    float2* da = dst + ra * ks;
     float2 z[N1];
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) z[n1] = line[n1 + (N1 + 1) * ra];
@@ -401,9 +439,9 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, size_t plan
     for (int k1 = 0; k1 < N1 / 2; ++k1) {
       const int k = ra + N2 * k1;
       float2 xk, xm;
-      post_pair(z[k1], z[N1 - 1 - k1], ldtw<TWS>(twN + k), ldtw<TWS>(twN + M - k), h, xk, xm);
-      dst[(size_t)k * plane] = xk;
-      dst[(size_t)(M - k) * plane] = xm;
+      post_pair(z[k1], z[N1 - 1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
+      da[(ptrdiff_t)k1 * step] = xk;
+      da[(ptrdiff_t)(N1 - 1 - k1) * step] = xm;
     }
   }
 }
@@ -716,14 +754,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
 __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-// Prefetch [p, p + bytes) into L2 in chunks of at most 4 KB, one per lane of
-// the calling warp.
-__device__ __forceinline__ void prefetch_l2_warp(const void* p, size_t bytes, int lane) {
-  constexpr size_t CH = 4096;
-  for (size_t o = (size_t)lane * CH; o < bytes; o += 32 * CH)
-    prefetch_l2(static_cast<const char*>(p) + o, (unsigned)(bytes - o < CH ? bytes - o : CH));
-}
-
 // ASYNC: the tile's half spectra are copied into the line buffer by cp.async
 // (all of them in flight at once, no registers held) in the in-place slot
 // order, and the inverse transform then runs in place; otherwise each item
@@ -754,12 +784,13 @@ __global__ void __launch_bounds__(T) x_pass_kernel(const RunParams* __restrict__
   const float2* twM = TWS ? stwM : sh.twM;
   const RunParams& rp = runs[blockIdx.y];
   const int nF = (MODE == MODE_XJ) ? 1 : rp.V + 1;
+  const FastDiv by_line(nF * WY);
   const int ny_tiles = sh.Ny / WY;
   const int z = blockIdx.x / ny_tiles;
   const int y0 = (blockIdx.x - z * ny_tiles) * WY;
-  const size_t plane = (size_t)sh.Nz * sh.Ny;
-  const size_t fstride = (size_t)sh.Kx * plane;
-  const size_t row_off = (size_t)z * sh.Ny + y0;
+  const int ks = sh.ks;
+  const size_t fstride = (size_t)sh.Kx * sh.Nz * sh.Ny;
+  const int row_off = z * sh.zs + y0;
   const float2* __restrict__ src = (MODE == MODE_XJ) ? rp.J : rp.Sm;
 
   if (MODE == MODE_IMPORT) {
@@ -780,19 +811,19 @@ __global__ void __launch_bounds__(T) x_pass_kernel(const RunParams* __restrict__
       for (int it = threadIdx.x; it < nF * KX * WY; it += T) {
         const int yy = it % WY, r = it / WY, kx = r % KX, f = r / KX;
         cp_async8(smem + (f * WY + yy) * PM + x_spec_slot<M>(kx),
-                  src + f * fstride + (size_t)kx * plane + row_off + yy);
+                  src + f * fstride + (kx * ks + row_off + yy));
       }
       cp_async_wait_all();
       __syncthreads();
       for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
-        const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
+        const int q = by_line(it), l = it - q * (nF * WY), pr = x_run_pair<M>(q);
         x_inv_runs<M, SPEC_INPLACE, TWS>(smem + l * PM, 0, smem + l * PM, pr, twN);
       }
     } else {
       for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
-        const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
+        const int q = by_line(it), l = it - q * (nF * WY), pr = x_run_pair<M>(q);
         const int f = l / WY, yy = l - f * WY;
-        x_inv_runs<M, SPEC_GLOBAL, TWS>(src + f * fstride + row_off + yy, plane, smem + l * PM, pr, twN);
+        x_inv_runs<M, SPEC_GLOBAL, TWS>(src + f * fstride + row_off + yy, ks, smem + l * PM, pr, twN);
       }
     }
     __syncthreads();
@@ -835,9 +866,9 @@ __global__ void __launch_bounds__(T) x_pass_kernel(const RunParams* __restrict__
   float2* __restrict__ dst = (MODE == MODE_BULK) ? rp.D : (MODE == MODE_XJ ? rp.J : rp.Sm);
   const float scale = 1.0f / (float)NX;
   for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
-    const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
+    const int q = by_line(it), l = it - q * (nF * WY), pr = x_run_pair<M>(q);
     const int f = l / WY, yy = l - f * WY;
-    x_fwd_runs<M, TWS>(dst + f * fstride + row_off + yy, plane, smem + l * PM, pr, scale, twN);
+    x_fwd_runs<M, TWS>(dst + f * fstride + row_off + yy, ks, smem + l * PM, pr, scale, twN);
   }
 
   if (MODE != MODE_BULK) return;
@@ -887,8 +918,8 @@ __global__ void __launch_bounds__(T, MINB) x_pass_tma_kernel(const RunParams* __
   const int ny_tiles = sh.Ny / WY;
   const int ntiles = sh.Nz * ny_tiles;
   const unsigned tile_bytes = (unsigned)(nF * KX * WY * 8);
-  const size_t plane = (size_t)sh.Nz * sh.Ny;
-  const size_t fstride = (size_t)sh.Kx * plane;
+  const int ks = sh.ks;
+  const size_t fstride = (size_t)sh.Kx * sh.Nz * sh.Ny;
   if (threadIdx.x == 0) mbar_init(bar, 1);
   __syncthreads();
   auto issue = [&](int t) {
@@ -902,7 +933,7 @@ __global__ void __launch_bounds__(T, MINB) x_pass_tma_kernel(const RunParams* __
   for (; tile < ntiles; tile += gridDim.x) {
     const int z = tile / ny_tiles;
     const int y0 = (tile - z * ny_tiles) * WY;
-    const size_t row_off = (size_t)z * sh.Ny + y0;
+    const int row_off = z * sh.zs + y0;
     const bool ok = mbar_wait(bar, parity);
     if (!__syncthreads_and(ok)) {  // the tile never arrived: flag the step and stop
       if (threadIdx.x == 0) atomicOr(rp.err, 1u);
@@ -931,7 +962,7 @@ __global__ void __launch_bounds__(T, MINB) x_pass_tma_kernel(const RunParams* __
     for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
       const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
       const int f = l / WY, yy = l - f * WY;
-      x_fwd_runs<M>(rp.D + f * fstride + row_off + yy, plane, smem + l * PM, pr, scale, sh.twN);
+      x_fwd_runs<M>(rp.D + f * fstride + row_off + yy, ks, smem + l * PM, pr, scale, sh.twN);
     }
     // 4. diagnostics of the tile (its block partials; ends with a barrier, so
     //    the lines are free for the next tile afterwards)
@@ -1403,7 +1434,8 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
   const int kx = p - (p / Kx) * Kx;
   const size_t plane_elems = (size_t)NZ * NY;
   const size_t fstride = (size_t)Kx * plane_elems;
-  const size_t poff = f * fstride + kx * plane_elems;
+  const size_t poff = f * fstride + kx * plane_elems;  // k-space state
+  const size_t moff = f * fstride + kx * sh.ks;        // mixed space
   const bool is_c = (f == rp.V);
   const bool var_c = (MODE == YZ_MAIN) && is_c && rp.mobility != MOB_CONST;
   const int z0 = r * G::LA;
@@ -1411,7 +1443,7 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
   // 1. forward y transform of the mixed-space input rows z0..z0+LA
   //    (MAIN/IMPORT: D~ or S~; C2: J~'), first pass straight from global
   {
-    const float2* src = (MODE == YZ_MAIN) ? rp.D + poff : (MODE == YZ_C2 ? rp.J + kx * plane_elems : rp.Sm + poff);
+    const float2* src = (MODE == YZ_MAIN) ? rp.D + moff : (MODE == YZ_C2 ? rp.J + kx * sh.ks : rp.Sm + moff);
     const int n1 = threadIdx.x % N1y;
     float2 w[N2y];
 #pragma unroll
@@ -1422,7 +1454,7 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
       const int it = threadIdx.x + j * T;
       if (ITEMS % T != 0 && it >= ITEMS) break;
       const int zl = it / N1y;
-      const float2* s = src + (size_t)(z0 + zl) * NY + n1;
+      const float2* s = src + (z0 + zl) * sh.zs + n1;
       float2 v[N2y];
 #pragma unroll
       for (int n2 = 0; n2 < N2y; ++n2) v[n2] = __ldg(s + n2 * N1y);
@@ -1448,7 +1480,8 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
       const size_t poff2 = f2 * fstride + kx2 * plane_elems;
       const int lane = threadIdx.x & 31;
       if (threadIdx.x < 32) {
-        prefetch_l2_warp(rp.D + poff2 + (size_t)r2 * G::LA * NY, (size_t)G::LA * NY * 8, lane);
+        const float2* d2 = rp.D + f2 * fstride + kx2 * sh.ks;
+        for (int zl = lane; zl < G::LA; zl += 32) prefetch_l2(d2 + (r2 * G::LA + zl) * sh.zs, NY * 8);
       } else {
         for (int k1 = lane; k1 < N1z; k1 += 32)
           prefetch_l2(rp.Sk + poff2 + (size_t)k1 * NY * N2z + (size_t)r2 * G::LB * N2z, G::LB * N2z * 8);
@@ -1521,7 +1554,7 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
   //    (u~ for the next x pass, or J~ for the variable-mobility chain)
   {
     const bool real_plane = (kx == 0) || (2 * kx == sh.Nx);  // the x-DFT of real data is real there
-    float2* dst = var_c ? rp.J + kx * plane_elems : rp.Sm + poff;
+    float2* dst = var_c ? rp.J + kx * sh.ks : rp.Sm + moff;
     const int n1 = threadIdx.x % N1y;
     float2 w[N2y];
 #pragma unroll
@@ -1538,7 +1571,7 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
 #pragma unroll
       for (int k2 = 1; k2 < N2y; ++k2) v[k2] = cmulc(s[k2 * (N1y + 1)], w[k2]);
       dft_inv<N2y>(v);
-      float2* o = dst + (size_t)(z0 + zl) * NY + n1;
+      float2* o = dst + (z0 + zl) * sh.zs + n1;
 #pragma unroll
       for (int n2 = 0; n2 < N2y; ++n2) {
         float2 x = v[n2];
@@ -1573,37 +1606,34 @@ struct YZ1 {
   static constexpr size_t SMEM = (size_t)NZ * PY * sizeof(float2);
 };
 
-// column pass A (forward or inverse) over the NY y positions
+// column pass A (forward or inverse) over the NY y positions.  Where the CTA's
+// warps are a multiple of N1 a warp keeps one column n1 and loads its twiddles
+// once (as broadcast loads of every item they were 7 of 23 shared wavefronts).
 template <int NY, int NZ, int T, bool INV, bool RAWP, bool TWS = false>
 __device__ __forceinline__ void colA(float2* U, const float2* __restrict__ tw) {
-  constexpr int N1 = Line<NZ>::N1, N2 = Line<NZ>::N2, PY = YZ1<NY, NZ, RAWP>::PY;
-  constexpr int ITEMS = NY * N1, ITER = (ITEMS + T - 1) / T;
+  constexpr int N1 = Line<NZ>::N1, N2 = Line<NZ>::N2, PY = YZ1<NY, NZ, RAWP>::PY, NW = T / 32;
+  if constexpr (NW % N1 == 0) {
+    const int w = threadIdx.x >> 5, n1 = w % N1;
+    float2 wt[N2];
+#pragma unroll
+    for (int k2 = 1; k2 < N2; ++k2) wt[k2] = ldtw<TWS>(tw + n1 * k2);
 #pragma unroll 1
-  for (int j = 0; j < ITER; ++j) {
-    const int it = threadIdx.x + j * T;
-    if (ITEMS % T != 0 && it >= ITEMS) break;
-    const int yp = it % NY, n1 = it / NY;
-    float2* p = U + n1 * PY + Line<NY>::phys(yp);
-    float2 v[N2];
-    if (!INV) {
-#pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[n2 * N1 * PY];
-      Dft<N2>::fwd(v);
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmul(v[k2], ldtw<TWS>(tw + n1 * k2));
-    } else {
-      v[0] = p[0];
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmulc(p[k2 * N1 * PY], ldtw<TWS>(tw + n1 * k2));
-      dft_inv<N2>(v);
+    for (int yp = (w / N1) * 32 + (threadIdx.x & 31); yp < NY; yp += 32 * (NW / N1))
+      passA_item<N1, N2, N1 * PY, INV>(U + n1 * PY + Line<NY>::phys(yp), [&](int k2) { return wt[k2]; });
+  } else {
+    constexpr int ITEMS = NY * N1, ITER = (ITEMS + T - 1) / T;
+#pragma unroll 1
+    for (int j = 0; j < ITER; ++j) {
+      const int it = threadIdx.x + j * T;
+      if (ITEMS % T != 0 && it >= ITEMS) break;
+      const int yp = it % NY, n1 = it / NY;
+      passA_item<N1, N2, N1 * PY, INV>(U + n1 * PY + Line<NY>::phys(yp), [&](int k2) { return ldtw<TWS>(tw + n1 * k2); });
     }
-#pragma unroll
-    for (int k = 0; k < N2; ++k) p[k * N1 * PY] = v[k];
   }
 }
 
-template <int NY, int NZ, int T, int MODE, bool RAWP = false>
-__global__ void __launch_bounds__(T) yz1_kernel(const RunParams* __restrict__ runs, const Shape sh) {
+template <int NY, int NZ, int T, int MODE, bool RAWP = false, int MINB = 0, int UC = Line<NZ>::N1>
+__global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restrict__ runs, const Shape sh) {
   using LY = Line<NY>;
   using LZ = Line<NZ>;
   constexpr int N1y = LY::N1, N2y = LY::N2, N1z = LZ::N1, N2z = LZ::N2;
@@ -1625,13 +1655,14 @@ __global__ void __launch_bounds__(T) yz1_kernel(const RunParams* __restrict__ ru
   const int f = (MODE == YZ_C2) ? rp.V : p / Kx;
   const int kx = p - (p / Kx) * Kx;
   const size_t plane_elems = (size_t)NZ * NY;
-  const size_t poff = ((size_t)f * Kx + kx) * plane_elems;
+  const size_t poff = ((size_t)f * Kx + kx) * plane_elems;          // k-space state
+  const size_t moff = (size_t)f * Kx * plane_elems + kx * sh.ks;  // mixed space
   const bool is_c = (f == rp.V);
   const bool var_c = (MODE == YZ_MAIN) && is_c && rp.mobility != MOB_CONST;
 
   // 1. forward y transform of all NZ rows, first pass straight from global
   {
-    const float2* src = (MODE == YZ_MAIN) ? rp.D + poff : (MODE == YZ_C2 ? rp.J + kx * plane_elems : rp.Sm + poff);
+    const float2* src = (MODE == YZ_MAIN) ? rp.D + moff : (MODE == YZ_C2 ? rp.J + kx * sh.ks : rp.Sm + moff);
     // twiddles: preloaded when every iteration of a thread has the same n1
     constexpr bool FIXED = (T % N1y) == 0;
     float2 wt[N2y];
@@ -1645,7 +1676,7 @@ __global__ void __launch_bounds__(T) yz1_kernel(const RunParams* __restrict__ ru
       const int it = threadIdx.x + j * T;
       if (ITEMS % T != 0 && it >= ITEMS) break;
       const int z = it / N1y, n1 = it - z * N1y;
-      const float2* s = src + (size_t)z * NY + n1;
+      const float2* s = src + z * sh.zs + n1;
       float2 v[N2y];
 #pragma unroll
       for (int n2 = 0; n2 < N2y; ++n2) v[n2] = __ldg(s + n2 * N1y);
@@ -1713,7 +1744,7 @@ __global__ void __launch_bounds__(T) yz1_kernel(const RunParams* __restrict__ ru
   // 3. last inverse y pass straight to the mixed-space output
   {
     const bool real_plane = (kx == 0) || (2 * kx == sh.Nx);  // the x-DFT of real data is real there
-    float2* dst = var_c ? rp.J + kx * plane_elems : rp.Sm + poff;
+    float2* dst = var_c ? rp.J + kx * sh.ks : rp.Sm + moff;
     constexpr bool FIXED = (T % N1y) == 0;
     float2 wt[N2y];
     if constexpr (FIXED) {
@@ -1732,7 +1763,7 @@ __global__ void __launch_bounds__(T) yz1_kernel(const RunParams* __restrict__ ru
 #pragma unroll
       for (int k2 = 1; k2 < N2y; ++k2) v[k2] = cmulc(sp[k2 * (N1y + 1)], FIXED ? wt[k2] : __ldg(sh.twY + n1 * k2));
       dft_inv<N2y>(v);
-      float2* o = dst + (size_t)z * NY + n1;
+      float2* o = dst + z * sh.zs + n1;
 #pragma unroll
       for (int n2 = 0; n2 < N2y; ++n2) {
         float2 x = v[n2];
@@ -1841,9 +1872,9 @@ __global__ void __launch_bounds__(T) x_pass_cl_kernel(const RunParams* __restric
   const int ny_tiles = sh.Ny / WY;
   const int z = bp / ny_tiles;
   const int y0 = (bp - z * ny_tiles) * WY;
-  const size_t plane = (size_t)sh.Nz * sh.Ny;
-  const size_t fstride = (size_t)sh.Kx * plane;
-  const size_t row_off = (size_t)z * sh.Ny + y0;
+  const int ks = sh.ks;
+  const size_t fstride = (size_t)sh.Kx * sh.Nz * sh.Ny;
+  const int row_off = z * sh.zs + y0;
   float2* lines = smem;                          // nloc * WY lines
   float2* A = smem + (size_t)h * WY * PM;        // the same offset in both CTAs
   const uint32_t peer_A = map_rank(smem_addr(A), peer);
@@ -1853,7 +1884,7 @@ __global__ void __launch_bounds__(T) x_pass_cl_kernel(const RunParams* __restric
   for (int it = threadIdx.x; it < nloc * WY * NP; it += T) {
     const int l = it % (nloc * WY), pr = x_run_pair<M>(it / (nloc * WY));
     const int fl = l / WY, yy = l - fl * WY;
-    x_inv_runs<M>(rp.Sm + (fbase + fl) * fstride + row_off + yy, plane, lines + l * PM, pr, sh.twN);
+    x_inv_runs<M>(rp.Sm + (fbase + fl) * fstride + row_off + yy, ks, lines + l * PM, pr, sh.twN);
   }
   __syncthreads();
   passA_rt<M, PM, T, true>(lines, nloc * WY, sh.twM);
@@ -1984,7 +2015,7 @@ __global__ void __launch_bounds__(T) x_pass_cl_kernel(const RunParams* __restric
   for (int it = threadIdx.x; it < nloc * WY * NP; it += T) {
     const int l = it % (nloc * WY), pr = x_run_pair<M>(it / (nloc * WY));
     const int fl = l / WY, yy = l - fl * WY;
-    x_fwd_runs<M>(rp.D + (fbase + fl) * fstride + row_off + yy, plane, lines + l * PM, pr, scale, sh.twN);
+    x_fwd_runs<M>(rp.D + (fbase + fl) * fstride + row_off + yy, ks, lines + l * PM, pr, scale, sh.twN);
   }
   if (!rank) return;
 
