@@ -2,8 +2,6 @@
 // construction, CUDA-graph step driver and host<->device field transfer for
 // the fused FP32 path.  The FP64 plain path and the Fortran shims live in
 // pf_plain64.cu, the host-side RNG in pf_host.cpp.
-#include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched through the runtime)
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -126,7 +124,6 @@ static int build_tables(int Nx, int Ny, int Nz, DevTables& t) {
   s.Nx = Nx; s.Ny = Ny; s.Nz = Nz; s.Kx = Kx;
   s.plane0 = 0;
   mixed_strides(Nx, Ny, Nz, s.ks, s.zs);
-  s.pref_yz = 0;
   s.par = 0;
   s.twM = (const float2*)(b + off_tw[0]);
   s.twN = (const float2*)(b + off_tw[1]);
@@ -163,39 +160,6 @@ static const size_t kMaxSmem = 227 * 1024;
 // diagnostics reduction's arrays (under 1 KB).  Both count against kMaxSmem.
 static size_t x_static_smem(int nx) { return (nx >= 96 ? (size_t)(nx + nx / 2) * sizeof(float2) : 0) + 1024; }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry points (no link
-// against the driver library).
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else
-      cudaGetLastError();
-  });
-  return fn;
-}
-
-// Tensor map over a run's mixed-space state Sm [nF][Kx][Nz][Ny] (8-byte
-// complex elements) with box {wy rows, 1 z, Kx, 1 field}: one TMA copy brings
-// the half spectra of wy rows of one field at one z.
-static int encode_sm_map(void* Sm, int Ny, int Nz, int Kx, int nF, int ks, int zs, int wy, CUtensorMap* out) {
-  const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
-  if (!fn) return fail(PF_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  const cuuint64_t dims[4] = {(cuuint64_t)Ny, (cuuint64_t)Nz, (cuuint64_t)Kx, (cuuint64_t)nF};
-  const cuuint64_t strides[3] = {(cuuint64_t)zs * 8, (cuuint64_t)ks * 8, (cuuint64_t)Kx * Ny * Nz * 8};
-  const cuuint32_t box[4] = {(cuuint32_t)wy, 1, (cuuint32_t)Kx, 1};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, Sm, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(PF_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return PF_OK;
-}
 // order parameters per run; the x pass must also fit (var+1) field lines of
 // its rows in shared memory (checked below)
 static const int kMaxVar = 255;
@@ -210,8 +174,11 @@ static int validate(const pf_config* c) {
     return fail(PF_EINVAL, "(Ny, Nz)=(%d, %d) not supported by the fused FP32 path", c->ny, c->nz);
   if (c->var < 1 || c->var > kMaxVar) return fail(PF_EINVAL, "var=%d outside [1, %d]", c->var, kMaxVar);
   bool fits = false;
-  for (int i = 0; i < nxv; ++i)
-    fits = fits || (c->ny % xv[i].wy == 0 && x_smem(c->nx, c->var + 1, xv[i].wy) + x_static_smem(c->nx) <= kMaxSmem);
+  for (int i = 0; i < nxv; ++i) {
+    // at Nx = 32 the 8-row tiles set the limit on var: the 4-row ones are there for latency
+    const int wy = c->nx == 32 ? std::max(xv[i].wy, 8) : xv[i].wy;
+    fits = fits || (c->ny % wy == 0 && x_smem(c->nx, c->var + 1, wy) + x_static_smem(c->nx) <= kMaxSmem);
+  }
   if (!fits) return fail(PF_EINVAL, "var=%d with Nx=%d, Ny=%d does not fit the x pass", c->var, c->nx, c->ny);
   if (c->mobility != PF_MOB_REFERENCE && c->mobility != PF_MOB_C1MC)
     return fail(PF_EINVAL, "unknown mobility form %d", c->mobility);
@@ -240,9 +207,8 @@ struct pf_batch {
   XKernels xk{};
   XKernels xjk{};              // variant of the xj pass (one field: its best rows per CTA differ)
   YZKernels yk{};
-  size_t smem_x = 0, smem_xj = 0, smem_bulk = 0;
+  size_t smem_x = 0, smem_xj = 0;
   std::vector<RunParams> hrp;
-  std::vector<CUtensorMap> tmaps;  // host copies of the runs' tensor maps (TMA x pass)
   RunParams* drp = nullptr;
   void* mem = nullptr;         // all per-run buffers
   float* fin = nullptr;        // float staging [nF][Nz][Ny][Nx]
@@ -257,8 +223,6 @@ struct pf_batch {
   cudaStream_t rec = nullptr;         // the step records of the multi-step graph
   cudaEvent_t ev_yz = nullptr, ev_rec[2] = {nullptr, nullptr};
   int prio_hi = 0;                    // greatest stream priority of the device
-  int nsm = 0;                        // multiprocessors of the device (persistent TMA x pass)
-  int tma_occ = 1;                    // resident CTAs per SM of the chosen TMA x pass
   std::vector<double> hdiag;
   std::vector<int> steps_done;
   std::string variant;  // chosen kernel variants, for reports
@@ -311,34 +275,11 @@ static int launch_xj(pf_batch* b, cudaStream_t s, int prio = 0) {
   return PF_OK;
 }
 
-// The bulk x pass (one CTA per WY rows, or two-CTA clusters sharing the fields).
+// The bulk x pass (one CTA per WY rows).
 static int launch_x_bulk(pf_batch* b, cudaStream_t s) {
-  const int R = b->nruns;
-  const unsigned nblk = (unsigned)(b->Nz * (b->Ny / b->xk.wy));
-  if (b->xk.tma) {  // persistent: as many CTAs as are resident at once, over all runs
-    const unsigned g = (unsigned)std::max(1, std::min((int)nblk, b->nsm * b->tma_occ / R));
-    b->xk.bulk<<<dim3(g, R), b->xk.threads, b->smem_bulk, s>>>(b->drp, b->tab.sh);
-    PF_CUDA(cudaGetLastError());
-    return PF_OK;
-  }
-  if (!b->xk.cl) {
-    b->xk.bulk<<<dim3(nblk, R), b->xk.threads, b->smem_bulk, s>>>(b->drp, b->tab.sh);
-    PF_CUDA(cudaGetLastError());
-    return PF_OK;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = b->xk.cl;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(b->xk.cl * nblk, R);
-  cfg.blockDim = dim3(b->xk.threads);
-  cfg.dynamicSmemBytes = b->smem_bulk;
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  PF_CUDA(cudaLaunchKernelEx(&cfg, b->xk.bulk, (const RunParams*)b->drp, b->tab.sh));
+  const dim3 grid(b->Nz * (b->Ny / b->xk.wy), b->nruns);
+  b->xk.bulk<<<grid, b->xk.threads, b->smem_x, s>>>(b->drp, b->tab.sh);
+  PF_CUDA(cudaGetLastError());
   return PF_OK;
 }
 
@@ -536,38 +477,8 @@ static bool x_ok(pf_batch* b, const XKernels& k) {
   if (b->Ny % k.wy != 0) return false;
   const size_t sm = x_smem(b->Nx, b->nF, k.wy);
   if (sm + x_static_smem(b->Nx) > kMaxSmem) return false;
-  if (k.tma) {  // persistent TMA bulk kernel: staging + lines must fit one CTA; inner TMA box of 16-byte multiples
-    const size_t sb = k.bulk_smem(b->nF);
-    CUtensorMap probe;
-    if (sb > kMaxSmem || (k.wy * 8) % 16 != 0 || b->Kx > 256 ||
-        encode_sm_map(b->hrp[0].Sm, b->Ny, b->Nz, b->Kx, b->nF, b->tab.sh.ks, b->tab.sh.zs, k.wy, &probe) != PF_OK ||
-        !raise_smem((const void*)k.bulk, sb))
-      return false;
-  }
-  if (k.cl) {  // two-CTA bulk: rank 1 must own phi_P and c (var >= 3); the cluster must be schedulable
-    const size_t sb = k.bulk_smem(b->nF);
-    if (b->V < 3 || sb > kMaxSmem || !raise_smem((const void*)k.bulk, sb)) return false;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = k.cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(k.cl * b->Nz * (b->Ny / k.wy), 1);
-    cfg.blockDim = dim3(k.threads);
-    cfg.dynamicSmemBytes = sb;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, (const void*)k.bulk, &cfg) != cudaSuccess || ncl < 1) {
-      cudaGetLastError();
-      return false;
-    }
-  }
-  for (KernelFn f : {k.bulk, k.xj, k.imp, k.exp}) {
-    if ((k.cl || k.tma) && f == k.bulk) continue;
+  for (KernelFn f : {k.bulk, k.xj, k.imp, k.exp})
     if (!raise_smem((const void*)f, sm)) return false;
-  }
   return true;
 }
 
@@ -580,10 +491,8 @@ static bool xj_ok(pf_batch* b, const XKernels& k) {
 
 static void describe_variants(pf_batch* b) {
   char buf[256];
-  snprintf(buf, sizeof buf, "x:wy=%d,threads=%d%s%s yz:cluster=%d,threads=%d%s%s xj:wy=%d,threads=%d%s", b->xk.wy,
-           b->xk.threads, b->xk.cl ? ",cluster=2" : (b->xk.tma ? ",tma" : ""), b->xk.tag, b->yk.cluster,
-           b->yk.threads, b->yk.inpl ? ",in-place" : "", b->yk.pref ? ",L2-prefetch" : "", b->xjk.wy,
-           b->xjk.threads, b->xjk.tag);
+  snprintf(buf, sizeof buf, "x:wy=%d,threads=%d%s yz:cluster=%d,threads=%d xj:wy=%d,threads=%d%s", b->xk.wy,
+           b->xk.threads, b->xk.tag, b->yk.cluster, b->yk.threads, b->xjk.wy, b->xjk.threads, b->xjk.tag);
   b->variant = buf;
 }
 
@@ -593,40 +502,12 @@ static void apply_xj(pf_batch* b, const XKernels& k) {
   describe_variants(b);
 }
 
-// Tensor maps of every run for the TMA x pass with wy rows per tile, written
-// on the batch's stream (in order with the launches that read them).
-static int write_tensor_maps(pf_batch* b, int wy) {
-  for (int r = 0; r < b->nruns; ++r) {
-    CUtensorMap m;
-    const int rc = encode_sm_map(b->hrp[r].Sm, b->Ny, b->Nz, b->Kx, b->nF, b->tab.sh.ks, b->tab.sh.zs, wy, &m);
-    if (rc) return rc;
-    b->tmaps[r] = m;
-  }
-  for (int r = 0; r < b->nruns; ++r)
-    PF_CUDA(cudaMemcpyAsync(const_cast<void*>(b->hrp[r].tmap_sm), &b->tmaps[r], sizeof(CUtensorMap),
-                            cudaMemcpyHostToDevice, b->stream));
-  return PF_OK;
-}
-
 static void apply_variants(pf_batch* b, const XKernels& xk, const YZKernels& yk) {
   b->xk = xk;
   b->yk = yk;
   b->smem_x = x_smem(b->Nx, b->nF, xk.wy);
-  b->smem_bulk = (xk.cl || xk.tma) ? xk.bulk_smem(b->nF) : b->smem_x;
-  if (xk.tma) {
-    write_tensor_maps(b, xk.wy);  // encodable: checked by x_ok
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)xk.bulk, xk.threads, b->smem_bulk) !=
-            cudaSuccess || occ < 1) {
-      cudaGetLastError();
-      occ = 1;
-    }
-    b->tma_occ = std::min(occ, xk.tma);
-  }
   b->tab.sh.nblk_x = b->Nz * (b->Ny / xk.wy);
   b->tab.sh.nblk_yz = yk.cluster * b->nF * b->Kx;
-  // L2 prefetch distance of the yz variants that prefetch: the CTAs resident at once
-  b->tab.sh.pref_yz = yk.pref ? yz_clusters(b, yk) * yk.cluster : 0;
   apply_xj(b, xk);
 }
 
@@ -705,13 +586,11 @@ static int tune_batch(pf_batch* b) {
         if (ty[i] < ty[by]) by = i;
       if (env_int("PFGPU_AUTOTUNE_REPORT", 0)) {  // every variant's best time per step, on stderr
         for (int i : xs)
-          fprintf(stderr, "pfgpu autotune %s x %d wy=%d threads=%d%s%s: %.4f ms/step%s\n", key, i, xv[i].wy,
-                  xv[i].threads, xv[i].cl ? ",cluster=2" : (xv[i].tma ? ",tma" : ""), xv[i].tag, tx[i] / REPS,
-                  i == bx ? " (chosen)" : "");
+          fprintf(stderr, "pfgpu autotune %s x %d wy=%d threads=%d%s: %.4f ms/step%s\n", key, i, xv[i].wy,
+                  xv[i].threads, xv[i].tag, tx[i] / REPS, i == bx ? " (chosen)" : "");
         for (int i : ys)
-          fprintf(stderr, "pfgpu autotune %s yz %d cluster=%d threads=%d%s%s: %.4f ms/step%s\n", key, i,
-                  yv[i].cluster, yv[i].threads, yv[i].inpl ? ",in-place" : "", yv[i].pref ? ",L2-prefetch" : "",
-                  ty[i] / REPS, i == by ? " (chosen)" : "");
+          fprintf(stderr, "pfgpu autotune %s yz %d cluster=%d threads=%d: %.4f ms/step%s\n", key, i, yv[i].cluster,
+                  yv[i].threads, ty[i] / REPS, i == by ? " (chosen)" : "");
       }
       // the xj pass (variable mobility) alone, over every variant that fits one field
       apply_variants(b, xv[bx], yv[by]);
@@ -746,7 +625,7 @@ static int tune_batch(pf_batch* b) {
         PF_CUDA(cudaMemsetAsync(r.Sk, 0, fbytes, b->stream));
         PF_CUDA(cudaMemsetAsync(r.Sm, 0, fbytes, b->stream));
         PF_CUDA(cudaMemsetAsync(r.D, 0, fbytes, b->stream));
-        PF_CUDA(cudaMemsetAsync(r.counter, 0, 256, b->stream));  // step counter, error word
+        PF_CUDA(cudaMemsetAsync(r.counter, 0, 256, b->stream));
       }
       PF_CUDA(cudaStreamSynchronize(b->stream));
       g_tune_cache[key] = std::make_tuple(bx, by, bj);
@@ -871,9 +750,8 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
   const size_t szPx = align((size_t)XD_COUNT * b->Nz * b->Ny * sizeof(double));
   const size_t szPyz = align((size_t)32 * b->nF * b->Kx * sizeof(double));  // 2 parities x 2 x clusters <= 16
   const size_t szDiag = align((size_t)b->ring * DR_COUNT * sizeof(double));
-  const size_t szCnt = 256;   // step counter and error word (one 64-byte line each)
-  const size_t szTmap = 256;  // TMA tensor map of Sm (128 bytes, 64-byte aligned)
-  const size_t per_run = 3 * szS + szMob + szJ + szPx + szPyz + szDiag + szCnt + szTmap;
+  const size_t szCnt = 256;  // step counter
+  const size_t per_run = 3 * szS + szMob + szJ + szPx + szPyz + szDiag + szCnt;
   e = cudaMalloc(&b->mem, per_run * nruns);
   if (e != cudaSuccess)
     return bail(fail(PF_ENOMEM, "cudaMalloc(%zu bytes) for %d runs: %s", per_run * nruns, nruns, cudaGetErrorString(e)));
@@ -884,10 +762,7 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
   e = cudaMalloc(&b->dstage, b->nF * ncell * sizeof(double));
   if (e != cudaSuccess) return bail(fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e)));
   b->hrp.resize(nruns);
-  b->tmaps.resize(nruns);
   b->steps_done.assign(nruns, 0);
-  cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, b->device);
-  if (b->nsm < 1) b->nsm = 1;
   for (int i = 0; i < nruns; ++i) {
     const pf_config& c = cfgs[i];
     char* p = (char*)b->mem + per_run * i;
@@ -902,9 +777,6 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     r.part_yz = (float*)p; p += szPyz;
     r.diag = (double*)p; p += szDiag;
     r.counter = (int*)p;
-    r.err = (unsigned*)(p + 128);
-    p += szCnt;
-    r.tmap_sm = p;
     r.fin = b->fin;
     r.L = (float)c.mob_phi;
     r.kappa_phi = (float)c.grad_coeff_phi;
@@ -963,7 +835,7 @@ static int batch_set_fields(pf_batch* b, int run, const double* phi, const doubl
   b->xk.imp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, b->tab.sh);
   int rc = launch_yz(b, b->yk.imp, b->nF * b->Kx, b->drp + run, 1, b->stream);
   if (rc) return rc;
-  PF_CUDA(cudaMemsetAsync(b->hrp[run].counter, 0, 256, b->stream));  // step counter, error word
+  PF_CUDA(cudaMemsetAsync(b->hrp[run].counter, 0, 256, b->stream));  // step counter
   PF_CUDA(cudaGetLastError());
   PF_CUDA(cudaStreamSynchronize(b->stream));
   b->steps_done[run] = 0;

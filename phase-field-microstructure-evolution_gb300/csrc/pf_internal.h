@@ -13,12 +13,9 @@ typedef void (*KernelFn)(const RunParams*, const Shape);
 // One compiled variant of the x pass (all four modes) ...
 struct XKernels {
   KernelFn bulk, xj, imp, exp;
-  int wy;       // y rows per CTA
-  int threads;  // threads per CTA
-  int cl = 0;   // 2: the bulk kernel runs as clusters of two CTAs sharing the fields (x_pass_cl_kernel)
-  int tma = 0;  // > 0: the bulk kernel is the persistent TMA-staged x_pass_tma_kernel, at most this many CTAs per SM
-  size_t (*bulk_smem)(int nF) = nullptr;  // its dynamic shared memory (cluster and TMA variants)
-  const char* tag = "";  // how the tile is loaded and walked, for reports
+  int wy;           // y rows per CTA
+  int threads;      // threads per CTA
+  const char* tag;  // how the tile is loaded and walked and the CTAs per SM asked for, for reports
 };
 
 // ... and of the yz pass (all three modes).
@@ -27,31 +24,72 @@ struct YZKernels {
   int cluster;   // CTAs per plane
   int threads;   // threads per CTA
   size_t smem;   // dynamic shared memory per CTA
-  int inpl = 0;  // 1: the cluster exchanges the plane in place (one buffer per CTA)
-  int pref = 0;  // 1: the main kernel prefetches the next generation's planes into L2 (Shape::pref_yz)
 };
 
 // Variant lists: each translation unit appends the variants it compiled for a
 // shape to `out` (room for kMaxVariants entries) and returns the new count.  The first variant of a shape is its
 // default; the run-creation autotuner times the others.
-constexpr int kMaxVariants = 20;
+constexpr int kMaxVariants = 8;
 int x_variants_a(int nx, XKernels* out, int n);
 int x_variants_r5(int nx, XKernels* out, int n);
 int yz_variants_small(int ny, int nz, YZKernels* out, int n);
-int yz_variants_128a(int ny, int nz, YZKernels* out, int n);
-int yz_variants_128b(int ny, int nz, YZKernels* out, int n);
-int yz_variants_256a(int ny, int nz, YZKernels* out, int n);
-int yz_variants_256b(int ny, int nz, YZKernels* out, int n);
+int yz_variants_128(int ny, int nz, YZKernels* out, int n);
+int yz_variants_256(int ny, int nz, YZKernels* out, int n);
 int yz_variants_r5(int ny, int nz, YZKernels* out, int n);
+
+// An x-pass variant: WY rows and T threads per CTA, at least MINB CTAs per SM
+// (0: as many registers as the compiler likes).  PHYS: the bulk walk over
+// physical slots; ASYNC: the tile's spectra copied in by cp.async and
+// transformed in place.
+template <int NX, int WY, int T, int MINB = 0, bool PHYS = true, bool ASYNC = false>
+static int add_x(XKernels* out, int n, const char* tag = "") {
+  if (n >= kMaxVariants) return n;
+  XKernels& k = out[n];
+  k.bulk = x_pass_kernel<NX, WY, T, MODE_BULK, PHYS, ASYNC, MINB>;
+  k.xj = x_pass_kernel<NX, WY, T, MODE_XJ, PHYS, ASYNC>;
+  k.imp = x_pass_kernel<NX, WY, T, MODE_IMPORT>;
+  k.exp = x_pass_kernel<NX, WY, T, MODE_EXPORT, PHYS, ASYNC>;
+  k.wy = WY;
+  k.threads = T;
+  k.tag = tag;
+  return n + 1;
+}
+
+// A yz-pass variant with one CTA of T threads per plane (RAWP: unpadded row
+// pitch), at least MINB CTAs per SM, k-space values read UC at a time.
+template <int NY, int NZ, int T, bool RAWP, int MINB = 0, int UC = Line<NZ>::N1>
+static int add_yz1(YZKernels* out, int n) {
+  if (n >= kMaxVariants) return n;
+  YZKernels& k = out[n];
+  k.main = yz1_kernel<NY, NZ, T, YZ_MAIN, RAWP, MINB, UC>;
+  k.c2 = yz1_kernel<NY, NZ, T, YZ_C2, RAWP, MINB, UC>;
+  k.imp = yz1_kernel<NY, NZ, T, YZ_IMPORT, RAWP, MINB, UC>;
+  k.cluster = 1;
+  k.threads = T;
+  k.smem = YZ1<NY, NZ, RAWP>::SMEM;
+  return n + 1;
+}
+
+// ... and with clusters of C CTAs per plane.
+template <int NY, int NZ, int C, int T, int MINB = 0, int UC = Line<NZ>::N1>
+static int add_yz(YZKernels* out, int n) {
+  if (n >= kMaxVariants) return n;
+  YZKernels& k = out[n];
+  k.main = yz_kernel<NY, NZ, C, T, YZ_MAIN, MINB, UC>;
+  k.c2 = yz_kernel<NY, NZ, C, T, YZ_C2, MINB, UC>;
+  k.imp = yz_kernel<NY, NZ, C, T, YZ_IMPORT, MINB, UC>;
+  k.cluster = C;
+  k.threads = T;
+  k.smem = YZ<NY, NZ, C>::SMEM;
+  return n + 1;
+}
 
 inline int get_x_variants(int nx, XKernels* out) { return x_variants_r5(nx, out, x_variants_a(nx, out, 0)); }
 inline int get_yz_variants(int ny, int nz, YZKernels* out) {
   int n = 0;
   n = yz_variants_small(ny, nz, out, n);
-  n = yz_variants_128a(ny, nz, out, n);
-  n = yz_variants_128b(ny, nz, out, n);
-  n = yz_variants_256a(ny, nz, out, n);
-  n = yz_variants_256b(ny, nz, out, n);
+  n = yz_variants_128(ny, nz, out, n);
+  n = yz_variants_256(ny, nz, out, n);
   n = yz_variants_r5(ny, nz, out, n);
   return n;
 }

@@ -66,8 +66,6 @@ struct RunParams {
   float* part_yz;  // [2][2][nblk_yz]: per step parity, hi and lo of each yz CTA's weighted f_int sum
   double* diag;    // [ring][DR_COUNT]
   int* counter;    // step counter (device)
-  unsigned* err;     // bit 0: a TMA tile of the x pass never arrived (the step's record is flagged)
-  const void* tmap_sm;  // TMA tensor map over Sm [nF][Kx][Nz][Ny] (x pass TMA variant), global memory
   float* fin;      // [nF][Nz][Ny][Nx] real fields for import/export
   float L, kappa_phi, kappa_c, dt, D_L, D_gb, sigma1, sigma2, am, ap, c0m, c0p;
   int mobility;
@@ -90,10 +88,6 @@ struct Shape {
   int nblk_yz;  // blocks of the yz pass per run
   int plane0;   // first (field, kx) plane of a yz-pass launch (a launch may cover a subset)
   int ks, zs;   // strides of kx and z in Sm, D and J (y contiguous; see mixed_strides)
-  // L2 prefetch distance in CTAs of the yz variants that prefetch: the CTAs
-  // resident at once, so that CTA b fetches into L2 what CTA b + pref (which
-  // starts about when b ends) will read; 0: none
-  int pref_yz;
   int par;  // parity of the step: which set of diagnostic partials its passes write and its record reads
 };
 
@@ -287,12 +281,11 @@ struct FastDiv {
 
 // Where element kx of a line's half spectrum is read from:
 //   SPEC_GLOBAL  src + kx * stride in read-only global memory;
-//   SPEC_SMEM    src + kx * stride in shared memory (a staging buffer);
 //   SPEC_INPLACE the line itself, kx at run kx % N2, element kx / N2 of the
 //                run (x_spec_slot), and kx = M in the pad slot after run 0.
 // In place, the inputs of a run pair are exactly the slots its outputs go
 // to, so every item reads its inputs into registers and overwrites them.
-enum SpecSrc { SPEC_GLOBAL = 0, SPEC_SMEM = 1, SPEC_INPLACE = 2 };
+enum SpecSrc { SPEC_GLOBAL = 0, SPEC_INPLACE = 1 };
 
 template <int M>
 __device__ __forceinline__ int x_spec_slot(int kx) {
@@ -304,7 +297,6 @@ __device__ __forceinline__ int x_spec_slot(int kx) {
 template <int SRC, int M>
 __device__ __forceinline__ float2 ld_spec(const float2* src, int step, int r, int k1) {
   if constexpr (SRC == SPEC_INPLACE) return src[(XLine<M>::N1 + 1) * r + k1];
-  else if constexpr (SRC == SPEC_SMEM) return src[k1 * step];
   else return __ldg(src + (ptrdiff_t)k1 * step);
 }
 
@@ -690,52 +682,6 @@ __device__ __forceinline__ void bulk_tile(float2* smem, const RunParams& rp, con
 }
 
 // ---------------------------------------------------------------------------
-// TMA (cp.async.bulk.tensor) and mbarrier helpers.  Tensor maps live in
-// global memory (one per run, written by the host before the launch); every
-// copy is a plain tile load from this GPU's own memory (no multicast).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(count)
-               : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(bar)),
-               "r"(bytes)
-               : "memory");
-}
-// Wait for the phase of the given parity to complete, for at most about one
-// second of the global timer: false if it never completed.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-  uint64_t t0;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    uint64_t t1;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-    if (t1 - t0 > 1000000000ull) return false;
-  }
-}
-// 4-D tile load of the box at coordinates (c0 innermost .. c3) into dst,
-// completing on bar.  c0 * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"((uint32_t)__cvta_generic_to_shared(bar))
-      : "memory");
-}
-
-// ---------------------------------------------------------------------------
 // x pass.  MODE_BULK: S -> D (+ mob, diagnostics).  MODE_XJ: J~ -> J~' with the
 // variable-mobility multiply (:947-965).  MODE_IMPORT: real fields -> S.
 // MODE_EXPORT: S -> real fields.
@@ -749,17 +695,12 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
 }
-// Prefetch [p, p + bytes) into L2 (cp.async.bulk.prefetch): no registers, no
-// completion to wait for.  p 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 // ASYNC: the tile's half spectra are copied into the line buffer by cp.async
 // (all of them in flight at once, no registers held) in the in-place slot
 // order, and the inverse transform then runs in place; otherwise each item
 // loads its own inputs from global memory.
-template <int NX, int WY, int T, int MODE, bool PHYS = true, bool ASYNC = false>
-__global__ void __launch_bounds__(T) x_pass_kernel(const RunParams* __restrict__ runs, const Shape sh) {
+template <int NX, int WY, int T, int MODE, bool PHYS = true, bool ASYNC = false, int MINB = 0>
+__global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __restrict__ runs, const Shape sh) {
   constexpr int M = NX / 2;
   using LM = XLine<M>;
   constexpr int PM = LM::PITCH;
@@ -879,99 +820,6 @@ __global__ void __launch_bounds__(T) x_pass_kernel(const RunParams* __restrict__
 
 
 // ---------------------------------------------------------------------------
-// x pass (bulk mode) with TMA-staged loads, persistent over tiles.
-//
-// MINB CTAs per SM (the grid holds as many as are resident at once) walk the
-// tiles (WY rows at one z, all fields) tile = blockIdx.x, blockIdx.x +
-// gridDim.x, ...  The mixed-space half spectra
-// of a tile arrive by TMA -- one box {WY rows, 1 z, Kx, 1 field} per field of
-// the run's tensor map over Sm [nF][Kx][Nz][Ny] -- into a staging buffer
-// [field][kx][row]; as soon as the inverse x transform has consumed them,
-// one thread issues the next tile's boxes, which land while the CTA runs the
-// rest of this tile (inverse pass A, bulk terms, forward transform, stores of
-// D and diagnostics).  The HBM latency that stalls the plain kernel's loads
-// thus overlaps the previous tile's arithmetic.  Results are identical to the
-// plain kernel's (same arithmetic, same per-tile partials).
-// ---------------------------------------------------------------------------
-template <int NX, int WY>
-struct XTMA {
-  static constexpr int M = NX / 2, KX = M + 1, PM = XLine<M>::PITCH;
-  // staging of one field, a multiple of 128 bytes so that every TMA
-  // destination starts on a 128-byte boundary
-  static constexpr int FSTRIDE = ((KX * WY * 8 + 127) / 128) * 16;  // float2 elements
-  static constexpr size_t stage_bytes(int nF) { return (size_t)nF * FSTRIDE * 8; }
-  static constexpr size_t smem(int nF) { return stage_bytes(nF) + (size_t)nF * WY * PM * 8 + 16; }
-};
-
-template <int NX, int WY, int T, int MINB = 1>
-__global__ void __launch_bounds__(T, MINB) x_pass_tma_kernel(const RunParams* __restrict__ runs, const Shape sh) {
-  using G = XTMA<NX, WY>;
-  constexpr int M = G::M, KX = G::KX, PM = G::PM;
-  using LM = XLine<M>;
-  constexpr int NP = LM::N2 / 2 + 1;
-  extern __shared__ __align__(128) unsigned char xsm[];
-  const RunParams& rp = runs[blockIdx.y];
-  const int nF = rp.V + 1;
-  float2* stage = reinterpret_cast<float2*>(xsm);  // [nF][KX][WY], field stride FSTRIDE
-  float2* smem = reinterpret_cast<float2*>(xsm + G::stage_bytes(nF));  // lines [nF * WY][PM]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(xsm + G::stage_bytes(nF) + (size_t)nF * WY * PM * 8);
-  const int ny_tiles = sh.Ny / WY;
-  const int ntiles = sh.Nz * ny_tiles;
-  const unsigned tile_bytes = (unsigned)(nF * KX * WY * 8);
-  const int ks = sh.ks;
-  const size_t fstride = (size_t)sh.Kx * sh.Nz * sh.Ny;
-  if (threadIdx.x == 0) mbar_init(bar, 1);
-  __syncthreads();
-  auto issue = [&](int t) {
-    const int zt = t / ny_tiles, yt = (t - zt * ny_tiles) * WY;
-    mbar_expect_tx(bar, tile_bytes);
-    for (int f = 0; f < nF; ++f) tma_load_4d(stage + (size_t)f * G::FSTRIDE, rp.tmap_sm, yt, zt, 0, f, bar);
-  };
-  int tile = blockIdx.x;
-  if (threadIdx.x == 0 && tile < ntiles) issue(tile);
-  unsigned parity = 0;
-  for (; tile < ntiles; tile += gridDim.x) {
-    const int z = tile / ny_tiles;
-    const int y0 = (tile - z * ny_tiles) * WY;
-    const int row_off = z * sh.zs + y0;
-    const bool ok = mbar_wait(bar, parity);
-    if (!__syncthreads_and(ok)) {  // the tile never arrived: flag the step and stop
-      if (threadIdx.x == 0) atomicOr(rp.err, 1u);
-      return;
-    }
-    parity ^= 1u;
-    // 1. inverse x transform from the staged half spectra (element kx of row yy at [kx][yy])
-    for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
-      const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
-      const int f = l / WY, yy = l - f * WY;
-      x_inv_runs<M, SPEC_SMEM>(stage + (size_t)f * G::FSTRIDE + yy, WY, smem + l * PM, pr, sh.twN);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && tile + (int)gridDim.x < ntiles) issue(tile + gridDim.x);  // staging is free again
-    passA_rt<M, PM, T, true>(smem, nF * WY, sh.twM);
-    __syncthreads();
-    // 2. bulk terms
-    BulkAcc acc;
-    acc.init();
-    bulk_tile<NX, WY, T>(smem, rp, sh, z, y0, acc);
-    __syncthreads();
-    // 3. forward x transform -> D
-    passA_rt<M, PM, T, false>(smem, nF * WY, sh.twM);
-    __syncthreads();
-    const float scale = 1.0f / (float)NX;
-    for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
-      const int l = it % (nF * WY), pr = x_run_pair<M>(it / (nF * WY));
-      const int f = l / WY, yy = l - f * WY;
-      x_fwd_runs<M>(rp.D + f * fstride + row_off + yy, ks, smem + l * PM, pr, scale, sh.twN);
-    }
-    // 4. diagnostics of the tile (its block partials; ends with a barrier, so
-    //    the lines are free for the next tile afterwards)
-    store_block_diag<T>(acc, rp, sh, tile);
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------
 // yz pass.  The state of every field is kept in full k-space,
 //     Sk[f][kx][ypos][zpos] = u_hat (normalised like f_trans, src/f_trans.f90:12),
 // in the digit-transposed position order of the y and z transforms, and is
@@ -994,9 +842,8 @@ struct YZ {
   static constexpr int PZ = Line<NZ>::PITCH;
   static constexpr int UA = LA * PY;
   static constexpr int UB = LB * PZ;
-  static constexpr size_t SMEM = (size_t)(UA + UB) * sizeof(float2);
-  // in-place variant: the A and B layouts share one buffer
-  static constexpr size_t SMEM_INPL = (size_t)(UA > UB ? UA : UB) * sizeof(float2);
+  // the A and B layouts share one buffer
+  static constexpr size_t SMEM = (size_t)(UA > UB ? UA : UB) * sizeof(float2);
   static_assert(NZ % C == 0 && NY % C == 0, "cluster must divide the plane");
 };
 
@@ -1100,6 +947,39 @@ __device__ __forceinline__ void kpoint(const KPlane& P, const KRow& R, const flo
   }
 }
 
+// One run of N1 positions of a z line: last forward pass, update, first inverse
+// pass.  d: the run of the driving term (in), of the new field or J (out);
+// gk: its k-space state, element k1 at gk[k1 * SK1], read UC at a time.
+template <int N1, int N2, int MODE, int UC>
+__device__ __forceinline__ void update_run(float2 (&d)[N1], float2* __restrict__ gk, size_t SK1, const KPlane& P,
+                                           const KRow& R, const float4* qz, const bool is_c, const bool var_c,
+                                           float& fint) {
+  float2 u[UC];
+  if (MODE != YZ_IMPORT) {
+#pragma unroll
+    for (int j = 0; j < UC; ++j) u[j] = gk[j * SK1];
+  }
+  Dft<N1>::fwd(d);
+#pragma unroll
+  for (int k0 = 0; k0 < N1; k0 += UC) {
+    if (MODE != YZ_IMPORT && k0 > 0) {
+#pragma unroll
+      for (int j = 0; j < UC; ++j)
+        if (k0 + j < N1) u[j] = gk[(k0 + j) * SK1];
+    }
+#pragma unroll
+    for (int j = 0; j < UC; ++j) {
+      const int k1 = k0 + j;
+      if (k1 < N1) {
+        kpoint<MODE>(P, R, qz[N2 * k1], is_c, var_c, u[j], d[k1], fint);
+        gk[k1 * SK1] = u[j];
+        if (!var_c) d[k1] = u[j];
+      }
+    }
+  }
+  if (MODE != YZ_IMPORT) dft_inv<N1>(d);
+}
+
 // ---------------------------------------------------------------------------
 // The step's record (src/var_diff.f90:1058-1118): one CTA per run reduces the
 // x-pass partials and the yz pass's f_int partials in a fixed order (the same
@@ -1185,7 +1065,7 @@ __global__ void __launch_bounds__(T) record_kernel(const RunParams* __restrict__
       d[DR_PHIMIN] = m2;
       d[DR_PHIPMAX] = m3;
       d[DR_MASS] = m.value();
-      d[DR_NONFINITE] = nbad + (*rp.err ? 1e9 : 0.0);  // a failed TMA wait flags every later step
+      d[DR_NONFINITE] = nbad;
       *rp.counter = step + 1;
     }
   }
@@ -1215,14 +1095,7 @@ __device__ __forceinline__ void yz_finish(const RunParams& rp, const Shape& sh, 
   }
 }
 
-template <int C>
-__device__ __forceinline__ void cluster_barrier() {
-  if constexpr (C == 1) {
-    __syncthreads();
-  } else {
-    cg::this_cluster().sync();
-  }
-}
+__device__ __forceinline__ void cluster_barrier() { cg::this_cluster().sync(); }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
@@ -1230,81 +1103,10 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
   return r;
 }
-template <int C>
 __device__ __forceinline__ float2 ld_peer(uint32_t a) {
   float2 v;
-  if constexpr (C == 1) {
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  } else {
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  }
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
   return v;
-}
-
-// B[yl][phys_z(z)] <- A_{owner(z)}[z % LA][phys_y(r*LB + yl)], consecutive
-// threads read consecutive y positions of one peer row.
-template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_AB(float2* __restrict__ B, uint32_t A_base, int r) {
-  using G = YZ<NY, NZ, C>;
-  constexpr int TOTAL = G::LB * NZ;
-  static_assert(T % G::LB == 0, "threads must cover whole rows");
-  constexpr int S = T / G::LB;  // z step per iteration
-  constexpr int ITER = (TOTAL + T - 1) / T;
-  const int yl = threadIdx.x % G::LB;
-  const int z0 = threadIdx.x / G::LB;
-  const uint32_t src_off = (uint32_t)(Line<NY>::phys(r * G::LB + yl)) * 8u;
-  constexpr int K = 8;
-#pragma unroll
-  for (int j0 = 0; j0 < ITER; j0 += K) {
-    float2 v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int z = z0 + (j0 + k) * S;
-      if (j0 + k < ITER && z < NZ) {
-        const int owner = z / G::LA, zl = z - owner * G::LA;
-        const uint32_t a = A_base + (uint32_t)(zl * G::PY) * 8u + src_off;
-        v[k] = ld_peer<C>(C == 1 ? a : map_rank(a, owner));
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int z = z0 + (j0 + k) * S;
-      if (j0 + k < ITER && z < NZ) B[yl * G::PZ + Line<NZ>::phys(z)] = v[k];
-    }
-  }
-}
-
-// A[zl][phys_y(y)] <- B_{owner(y)}[y % LB][phys_z(r*LA + zl)], consecutive
-// threads read consecutive z positions of one peer line.
-template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_BA(float2* __restrict__ A, uint32_t B_base, int r) {
-  using G = YZ<NY, NZ, C>;
-  constexpr int TOTAL = G::LA * NY;
-  static_assert(T % G::LA == 0, "threads must cover whole lines");
-  constexpr int S = T / G::LA;
-  constexpr int ITER = (TOTAL + T - 1) / T;
-  const int zl = threadIdx.x % G::LA;
-  const int y0 = threadIdx.x / G::LA;
-  const uint32_t src_off = (uint32_t)(Line<NZ>::phys(r * G::LA + zl)) * 8u;
-  constexpr int K = 8;
-#pragma unroll
-  for (int j0 = 0; j0 < ITER; j0 += K) {
-    float2 v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int y = y0 + (j0 + k) * S;
-      if (j0 + k < ITER && y < NY) {
-        const int owner = y / G::LB, yl = y - owner * G::LB;
-        const uint32_t a = B_base + (uint32_t)(yl * G::PZ) * 8u + src_off;
-        v[k] = ld_peer<C>(C == 1 ? a : map_rank(a, owner));
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int y = y0 + (j0 + k) * S;
-      if (j0 + k < ITER && y < NY) A[zl * G::PY + Line<NY>::phys(y)] = v[k];
-    }
-  }
 }
 
 // In-place exchanges: every thread first reads all the elements it will own
@@ -1313,7 +1115,7 @@ __device__ __forceinline__ void exch_BA(float2* __restrict__ A, uint32_t B_base,
 // CTA overwrites its own buffer with the new layout.  One buffer per CTA
 // instead of two, so a quarter of a 256 x 256 plane (140 KB) fits one CTA.
 template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_AB_inpl(float2* __restrict__ buf, uint32_t A_base, int r) {
+__device__ __forceinline__ void exch_AB(float2* __restrict__ buf, uint32_t A_base, int r) {
   using G = YZ<NY, NZ, C>;
   constexpr int TOTAL = G::LB * NZ;
   static_assert(T % G::LB == 0 && TOTAL % T == 0, "threads must cover whole rows");
@@ -1327,16 +1129,16 @@ __device__ __forceinline__ void exch_AB_inpl(float2* __restrict__ buf, uint32_t 
   for (int k = 0; k < ITER; ++k) {
     const int z = z0 + k * S;
     const int owner = z / G::LA, zl = z - owner * G::LA;
-    v[k] = ld_peer<C>(map_rank(A_base + (uint32_t)(zl * G::PY) * 8u + src_off, owner));
+    v[k] = ld_peer(map_rank(A_base + (uint32_t)(zl * G::PY) * 8u + src_off, owner));
   }
-  cluster_barrier<C>();  // every CTA holds its new layout in registers
+  cluster_barrier();  // every CTA holds its new layout in registers
 #pragma unroll
   for (int k = 0; k < ITER; ++k) buf[yl * G::PZ + Line<NZ>::phys(z0 + k * S)] = v[k];
   __syncthreads();
 }
 
 template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_BA_inpl(float2* __restrict__ buf, uint32_t B_base, int r) {
+__device__ __forceinline__ void exch_BA(float2* __restrict__ buf, uint32_t B_base, int r) {
   using G = YZ<NY, NZ, C>;
   constexpr int TOTAL = G::LA * NY;
   static_assert(T % G::LA == 0 && TOTAL % T == 0, "threads must cover whole lines");
@@ -1350,9 +1152,9 @@ __device__ __forceinline__ void exch_BA_inpl(float2* __restrict__ buf, uint32_t 
   for (int k = 0; k < ITER; ++k) {
     const int y = y0 + k * S;
     const int owner = y / G::LB, yl = y - owner * G::LB;
-    v[k] = ld_peer<C>(map_rank(B_base + (uint32_t)(yl * G::PZ) * 8u + src_off, owner));
+    v[k] = ld_peer(map_rank(B_base + (uint32_t)(yl * G::PZ) * 8u + src_off, owner));
   }
-  cluster_barrier<C>();  // no CTA reads a peer's buffer after this point
+  cluster_barrier();  // no CTA reads a peer's buffer after this point
 #pragma unroll
   for (int k = 0; k < ITER; ++k) buf[zl * G::PY + Line<NY>::phys(y0 + k * S)] = v[k];
   __syncthreads();
@@ -1411,11 +1213,8 @@ __device__ __forceinline__ void passB(float2* buf) {
   }
 }
 
-// PREF (main mode): before its k-space update the CTA prefetches into L2 the
-// D~ rows and k-space block that CTA blockIdx.x + sh.pref_yz (a multiple of C:
-// the same cluster rank, about one generation of resident CTAs later) reads.
-template <int NY, int NZ, int C, int T, int MODE, bool INPL = false, bool PREF = false>
-__global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ runs, const Shape sh) {
+template <int NY, int NZ, int C, int T, int MODE, int MINB = 0, int UC = Line<NZ>::N1>
+__global__ void __launch_bounds__(T, MINB) yz_kernel(const RunParams* __restrict__ runs, const Shape sh) {
   using G = YZ<NY, NZ, C>;
   using LY = Line<NY>;
   using LZ = Line<NZ>;
@@ -1424,10 +1223,9 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
   extern __shared__ float2 smem[];
   __shared__ float4 qzt[NZ];  // kz factors of the k-space update
   stage_kz<NZ, T>(qzt, sh);   // read after the barriers of the forward passes
-  float2* UA = smem;
-  float2* UB = INPL ? smem : smem + G::UA;  // in place: both layouts in one buffer
+  float2 *UA = smem, *UB = smem;  // both layouts share one buffer
   const RunParams& rp = runs[blockIdx.y];
-  const int r = (C == 1) ? 0 : (int)(blockIdx.x % C);
+  const int r = (int)(blockIdx.x % C);
   const int p = sh.plane0 + (int)(blockIdx.x / C);
   const int Kx = sh.Kx;
   const int f = (MODE == YZ_C2) ? rp.V : p / Kx;
@@ -1467,27 +1265,11 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
   }
   __syncthreads();
   passB<NY, G::LA, G::PY, T, false>(UA);
-  cluster_barrier<C>();
-  if constexpr (INPL) exch_AB_inpl<NY, NZ, C, T>(UB, smem_addr(UA), r);
-  else exch_AB<NY, NZ, C, T>(UB, smem_addr(UA), r);
+  cluster_barrier();
+  exch_AB<NY, NZ, C, T>(UB, smem_addr(UA), r);
   __syncthreads();
   passA<NZ, G::LB, G::PZ, T, false>(UB, sh.twZ);
   __syncthreads();
-  if constexpr (PREF && MODE == YZ_MAIN) {
-    const int b2 = (int)blockIdx.x + sh.pref_yz;
-    if (sh.pref_yz > 0 && b2 < (int)gridDim.x && threadIdx.x < 64) {
-      const int p2 = sh.plane0 + b2 / C, f2 = p2 / Kx, kx2 = p2 - f2 * Kx, r2 = b2 % C;
-      const size_t poff2 = f2 * fstride + kx2 * plane_elems;
-      const int lane = threadIdx.x & 31;
-      if (threadIdx.x < 32) {
-        const float2* d2 = rp.D + f2 * fstride + kx2 * sh.ks;
-        for (int zl = lane; zl < G::LA; zl += 32) prefetch_l2(d2 + (r2 * G::LA + zl) * sh.zs, NY * 8);
-      } else {
-        for (int k1 = lane; k1 < N1z; k1 += 32)
-          prefetch_l2(rp.Sk + poff2 + (size_t)k1 * NY * N2z + (size_t)r2 * G::LB * N2z, G::LB * N2z * 8);
-      }
-    }
-  }
 
   // 2. last forward z pass, pointwise k-space update, first inverse z pass,
   //    fused per run of N1z positions
@@ -1509,44 +1291,24 @@ __global__ void __launch_bounds__(T) yz_kernel(const RunParams* __restrict__ run
       // k1 a warp reads and writes consecutive (y position, k2) (coalesced)
       float2* gk = rp.Sk + poff + (size_t)ypos * N2z + k2;
       constexpr size_t SK1 = (size_t)NY * N2z;  // stride of k1
-      float2 d[N1z], u[N1z];
+      float2 d[N1z];
 #pragma unroll
       for (int k1 = 0; k1 < N1z; ++k1) d[k1] = pb[k1];
-      Dft<N1z>::fwd(d);
+      update_run<N1z, N2z, MODE, UC>(d, gk, SK1, P, R, qzt + k2, is_c, var_c, fint);
       if (MODE != YZ_IMPORT) {
 #pragma unroll
-        for (int k1 = 0; k1 < N1z; ++k1) u[k1] = gk[k1 * SK1];
-      }
-#pragma unroll
-      for (int k1 = 0; k1 < N1z; ++k1) kpoint<MODE>(P, R, qzt[k2 + N2z * k1], is_c, var_c, u[k1], d[k1], fint);
-#pragma unroll
-      for (int k1 = 0; k1 < N1z; ++k1) gk[k1 * SK1] = u[k1];
-      if (MODE != YZ_IMPORT) {
-        if (var_c) {
-          dft_inv<N1z>(d);
-#pragma unroll
-          for (int k1 = 0; k1 < N1z; ++k1) pb[k1] = d[k1];
-        } else {
-          dft_inv<N1z>(u);
-#pragma unroll
-          for (int k1 = 0; k1 < N1z; ++k1) pb[k1] = u[k1];
-        }
+        for (int k1 = 0; k1 < N1z; ++k1) pb[k1] = d[k1];
       }
     }
   }
   if (MODE == YZ_IMPORT) {
-    cluster_barrier<C>();  // peers may still read this CTA's A buffer
+    cluster_barrier();  // peers may still read this CTA's A buffer
     return;
   }
   __syncthreads();
   passA<NZ, G::LB, G::PZ, T, true>(UB, sh.twZ);
-  cluster_barrier<C>();
-  if constexpr (INPL) {
-    exch_BA_inpl<NY, NZ, C, T>(UA, smem_addr(UB), r);  // ends after the last peer read
-  } else {
-    exch_BA<NY, NZ, C, T>(UA, smem_addr(UB), r);
-    cluster_barrier<C>();  // no CTA reads a peer's buffers after this point
-  }
+  cluster_barrier();
+  exch_BA<NY, NZ, C, T>(UA, smem_addr(UB), r);  // ends after the last peer read
   passB<NY, G::LA, G::PY, T, true>(UA);
   __syncthreads();
 
@@ -1709,28 +1471,13 @@ __global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restric
       // k1 a warp reads and writes 32 consecutive y positions (coalesced)
       float2* gk = rp.Sk + poff + it;  // it == k2 NY + yp
       constexpr size_t SK1 = (size_t)N2z * NY;  // stride of k1
-      float2 d[N1z], u[N1z];
-      if (MODE != YZ_IMPORT) {
-#pragma unroll
-        for (int k1 = 0; k1 < N1z; ++k1) u[k1] = gk[k1 * SK1];
-      }
+      float2 d[N1z];
 #pragma unroll
       for (int k1 = 0; k1 < N1z; ++k1) d[k1] = pc[k1 * PY];
-      Dft<N1z>::fwd(d);
-#pragma unroll
-      for (int k1 = 0; k1 < N1z; ++k1) kpoint<MODE>(P, R, qzt[k2 + N2z * k1], is_c, var_c, u[k1], d[k1], fint);
-#pragma unroll
-      for (int k1 = 0; k1 < N1z; ++k1) gk[k1 * SK1] = u[k1];
+      update_run<N1z, N2z, MODE, UC>(d, gk, SK1, P, R, qzt + k2, is_c, var_c, fint);
       if (MODE != YZ_IMPORT) {
-        if (var_c) {
-          dft_inv<N1z>(d);
 #pragma unroll
-          for (int k1 = 0; k1 < N1z; ++k1) pc[k1 * PY] = d[k1];
-        } else {
-          dft_inv<N1z>(u);
-#pragma unroll
-          for (int k1 = 0; k1 < N1z; ++k1) pc[k1 * PY] = u[k1];
-        }
+        for (int k1 = 0; k1 < N1z; ++k1) pc[k1 * PY] = d[k1];
       }
     }
   }
@@ -1776,251 +1523,6 @@ __global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restric
   if (MODE == YZ_MAIN) {
     yz_finish<T>(rp, sh, fint, wkx, (size_t)p);
   }
-}
-
-// ---------------------------------------------------------------------------
-// x pass (bulk mode) split over a cluster of two CTAs.
-//
-// With many order parameters the one-CTA x pass holds (P+1) field rows and
-// fits one CTA per SM.  Here the two CTAs of a cluster take the same WY rows
-// and about half of the fields each (rank 0: fields [0, h), rank 1: [h, P+1),
-// h = ceil((P+1)/2); rank 1 owns phi_P and c), so twice as many CTAs fit an
-// SM.  The cross-field terms need per-cell sums over all fields: each CTA
-// forms partial sums over its own fields (sum phi^2, sum phi^4, pair sum,
-// max |phi|), the pair reads the other's partials through distributed shared
-// memory (pairs = pairs_0 + pairs_1 + pre_0 pre_1), and both derive the same
-// per-cell scalars; rank 1 also writes dF/dc, the mobility and the
-// diagnostics.  Cells whose sum of phi^4 is below 1e-30 take the rescaled
-// branch of bulk_slot with a second exchange (sum of (phi/max|phi|)^4).
-// HBM traffic is that of the one-CTA pass.
-// ---------------------------------------------------------------------------
-template <int NX, int WY>
-struct XCL {
-  static constexpr int M = NX / 2;
-  static constexpr int PM = XLine<M>::PITCH;
-  static constexpr int S = WY * M;  // float2 slots (two cells each) per CTA
-  static constexpr int NA = 7;      // per-slot arrays: pre, n4, pairs, mabs (partials), nn (partial), phiP, c
-  static constexpr size_t smem(int nF) { return ((size_t)((nF + 1) / 2) * WY * PM + (size_t)NA * S) * sizeof(float2); }
-};
-
-struct CellOut {
-  float t4a, t4p, invm, dc, mb;
-  int bad;
-};
-
-// per-cell scalars of bulk_slot from the full aggregates of one cell
-__device__ __forceinline__ CellOut cell_terms(float pp, float c, float pre, float n4, float pairs, float mabs, float nn,
-                                              const RunParams& rp, BulkAcc& acc) {
-  const float pp2 = pp * pp;
-  const float S2 = pre + pp2;
-  const float S4 = n4 + pp2 * pp2;
-  float invS4, n4n, sc, im = 1.f;
-  if (S4 >= 1e-30f) {
-    invS4 = 1.f / S4;
-    n4n = n4 * invS4;
-    sc = 4.f;
-  } else if (mabs > 0.f) {
-    im = 1.f / mabs;
-    const float xq = pp * im;
-    const float s4 = nn + (xq * xq) * (xq * xq);
-    invS4 = 1.f / s4;
-    n4n = nn * invS4;
-    sc = 4.f * im;
-  } else {
-    invS4 = 0.f;
-    n4n = 0.f;
-    sc = 0.f;
-  }
-  const float h = n4n;
-  const float dcm = c - rp.c0m, dcp = c - rp.c0p;
-  const float fm = rp.am * dcm * dcm, fp = rp.ap * dcp * dcp;
-  const float dfm = fm - fp;
-  acc.fch += h * fm + (1.f - h) * fp;
-  CellOut o;
-  o.dc = 2.f * h * rp.am * dcm + 2.f * (1.f - h) * rp.ap * dcp;
-  acc.feta += -0.5f * S2 + 0.25f * S4 + rp.sigma1 * pairs + rp.sigma2 * pp2 * pre;
-  acc.mass.add(c);
-  acc.cmin = fminf(acc.cmin, c);
-  acc.cmax = fmaxf(acc.cmax, c);
-  acc.phimin = fminf(acc.phimin, S2);
-  acc.phipmax = fmaxf(acc.phipmax, pp);
-  if (rp.mobility == MOB_REF_VAR) o.mb = 2.f * (1.f - S2) * rp.D_gb;
-  else if (rp.mobility == MOB_C1MC) o.mb = rp.D_L * c * (1.f - c);
-  else o.mb = 0.f;
-  const float qP = pp * im;
-  const float qP2 = qP * qP;
-  const float rP4 = qP2 * qP2 * invS4;
-  o.t4a = sc * invS4 * rP4 * dfm;
-  o.t4p = -sc * (qP * qP2 * invS4) * n4n * dfm;
-  o.invm = im;
-  o.bad = !isfinite(S4 + S2 + pairs + o.dc + o.t4a + o.t4p);
-  return o;
-}
-
-template <int NX, int WY, int T>
-__global__ void __launch_bounds__(T) x_pass_cl_kernel(const RunParams* __restrict__ runs, const Shape sh) {
-  using G = XCL<NX, WY>;
-  constexpr int M = G::M, PM = G::PM, S = G::S;
-  using LM = XLine<M>;
-  constexpr int NP = LM::N2 / 2 + 1;
-  enum { A_PRE = 0, A_N4, A_PAIRS, A_MABS, A_NN, A_PP, A_C };
-  extern __shared__ float2 smem[];
-  const RunParams& rp = runs[blockIdx.y];
-  const int V = rp.V, nF = V + 1, h = (nF + 1) / 2;
-  const int rank = (int)(blockIdx.x & 1), peer = rank ^ 1, bp = (int)(blockIdx.x >> 1);
-  const int fbase = rank ? h : 0, nloc = rank ? nF - h : h;
-  const int ny_tiles = sh.Ny / WY;
-  const int z = bp / ny_tiles;
-  const int y0 = (bp - z * ny_tiles) * WY;
-  const int ks = sh.ks;
-  const size_t fstride = (size_t)sh.Kx * sh.Nz * sh.Ny;
-  const int row_off = z * sh.zs + y0;
-  float2* lines = smem;                          // nloc * WY lines
-  float2* A = smem + (size_t)h * WY * PM;        // the same offset in both CTAs
-  const uint32_t peer_A = map_rank(smem_addr(A), peer);
-  const uint32_t peer_lines = map_rank(smem_addr(lines), peer);
-
-  // 1. inverse x transform of the local fields
-  for (int it = threadIdx.x; it < nloc * WY * NP; it += T) {
-    const int l = it % (nloc * WY), pr = x_run_pair<M>(it / (nloc * WY));
-    const int fl = l / WY, yy = l - fl * WY;
-    x_inv_runs<M>(rp.Sm + (fbase + fl) * fstride + row_off + yy, ks, lines + l * PM, pr, sh.twN);
-  }
-  __syncthreads();
-  passA_rt<M, PM, T, true>(lines, nloc * WY, sh.twM);
-  __syncthreads();
-
-  // 2. partial sums over the local matrix fields (f < V-1), in field order
-  const int fend = min(fbase + nloc, V - 1);
-  for (int it = threadIdx.x; it < S; it += T) {
-    const int m = it % M, yy = it / M;
-    const float2* base = lines + yy * PM + LM::phys(m);
-    float pre0 = 0.f, pre1 = 0.f, n40 = 0.f, n41 = 0.f, pr0 = 0.f, pr1 = 0.f, ma0 = 0.f, ma1 = 0.f;
-    for (int f = fbase; f < fend; ++f) {
-      const float2 p = base[(f - fbase) * WY * PM];
-      const float a0 = p.x * p.x, a1 = p.y * p.y;
-      pr0 = fmaf(a0, pre0, pr0);
-      pr1 = fmaf(a1, pre1, pr1);
-      pre0 += a0;
-      pre1 += a1;
-      n40 = fmaf(a0, a0, n40);
-      n41 = fmaf(a1, a1, n41);
-      ma0 = fmaxf(ma0, fabsf(p.x));
-      ma1 = fmaxf(ma1, fabsf(p.y));
-    }
-    A[A_PRE * S + it] = make_float2(pre0, pre1);
-    A[A_N4 * S + it] = make_float2(n40, n41);
-    A[A_PAIRS * S + it] = make_float2(pr0, pr1);
-    A[A_MABS * S + it] = make_float2(ma0, ma1);
-  }
-  cluster_barrier<2>();
-
-  // full sums (rank 0's part first in both CTAs: both get the same bits)
-  auto totals = [&](int it, float2& pre, float2& n4, float2& pairs, float2& mabs) {
-    float2 a[4], b[4];  // rank 0's and rank 1's partials
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 own = A[k * S + it];
-      const float2 oth = ld_peer<2>(peer_A + (uint32_t)((k * S + it) * 8));
-      a[k] = rank ? oth : own;
-      b[k] = rank ? own : oth;
-    }
-    pre = make_float2(a[0].x + b[0].x, a[0].y + b[0].y);
-    n4 = make_float2(a[1].x + b[1].x, a[1].y + b[1].y);
-    pairs = make_float2(fmaf(a[0].x, b[0].x, a[2].x + b[2].x), fmaf(a[0].y, b[0].y, a[2].y + b[2].y));
-    mabs = make_float2(fmaxf(a[3].x, b[3].x), fmaxf(a[3].y, b[3].y));
-  };
-
-  // 3. phi_P and c from rank 1; the rescaled sum where a cell needs it
-  for (int it = threadIdx.x; it < S; it += T) {
-    const int m = it % M, yy = it / M;
-    const int off_p = ((V - 1 - h) * WY + yy) * PM + LM::phys(m);  // in rank 1's lines
-    const int off_c = ((V - h) * WY + yy) * PM + LM::phys(m);
-    float2 pP, cc;
-    if (rank) {
-      pP = lines[off_p];
-      cc = lines[off_c];
-    } else {
-      pP = ld_peer<2>(peer_lines + (uint32_t)(off_p * 8));
-      cc = ld_peer<2>(peer_lines + (uint32_t)(off_c * 8));
-    }
-    A[A_PP * S + it] = pP;
-    A[A_C * S + it] = cc;
-    float2 pre, n4, pairs, mabs;
-    totals(it, pre, n4, pairs, mabs);
-    float nn[2] = {0.f, 0.f};
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float pp = q ? pP.y : pP.x;
-      const float S4 = (q ? n4.y : n4.x) + (pp * pp) * (pp * pp);
-      const float ma = fmaxf(q ? mabs.y : mabs.x, fabsf(pp));
-      if (S4 < 1e-30f && ma > 0.f) {
-        const float im = 1.f / ma;
-        const float2* base = lines + yy * PM + LM::phys(m);
-        for (int f = fbase; f < fend; ++f) {
-          const float2 p = base[(f - fbase) * WY * PM];
-          const float x = (q ? p.y : p.x) * im;
-          nn[q] = fmaf(x * x, x * x, nn[q]);
-        }
-      }
-    }
-    A[A_NN * S + it] = make_float2(nn[0], nn[1]);
-  }
-  cluster_barrier<2>();
-
-  // 4. per-cell scalars and dF of the local fields, in place
-  BulkAcc acc;
-  acc.init();
-  const float sg1 = rp.sigma1, sg2 = rp.sigma2;
-  for (int it = threadIdx.x; it < S; it += T) {
-    const int m = it % M, yy = it / M;
-    float2 pre, n4, pairs, mabs;
-    totals(it, pre, n4, pairs, mabs);
-    const float2 pP = A[A_PP * S + it], cc = A[A_C * S + it];
-    const float2 own_nn = A[A_NN * S + it];
-    const float2 oth_nn = ld_peer<2>(peer_A + (uint32_t)((A_NN * S + it) * 8));
-    const float2 nn0 = rank ? oth_nn : own_nn, nn1 = rank ? own_nn : oth_nn;
-    CellOut o[2];
-    o[0] = cell_terms(pP.x, cc.x, pre.x, n4.x, pairs.x, fmaxf(mabs.x, fabsf(pP.x)), nn0.x + nn1.x, rp, acc);
-    o[1] = cell_terms(pP.y, cc.y, pre.y, n4.y, pairs.y, fmaxf(mabs.y, fabsf(pP.y)), nn0.y + nn1.y, rp, acc);
-    float2* base = lines + yy * PM + LM::phys(m);
-    for (int f = fbase; f < fbase + nloc; ++f) {
-      float2& slot = base[(f - fbase) * WY * PM];
-      float2 d;
-      if (f < V - 1) {
-        const float2 p = slot;
-        const float g0 = fmaf(sg1, pre.x - p.x * p.x, sg2 * (pP.x * pP.x));
-        const float g1 = fmaf(sg1, pre.y - p.y * p.y, sg2 * (pP.y * pP.y));
-        const float q0 = p.x * o[0].invm, q1 = p.y * o[1].invm;
-        d.x = fmaf(p.x, p.x * p.x, -p.x) + 2.f * p.x * g0 + o[0].t4a * (q0 * q0 * q0);
-        d.y = fmaf(p.y, p.y * p.y, -p.y) + 2.f * p.y * g1 + o[1].t4a * (q1 * q1 * q1);
-      } else if (f == V - 1) {
-        d.x = fmaf(pP.x, pP.x * pP.x, -pP.x) + 2.f * pP.x * (sg2 * pre.x) + o[0].t4p;
-        d.y = fmaf(pP.y, pP.y * pP.y, -pP.y) + 2.f * pP.y * (sg2 * pre.y) + o[1].t4p;
-      } else {
-        d = make_float2(o[0].dc, o[1].dc);
-      }
-      slot = d;
-    }
-    if (rank && rp.mobility != MOB_CONST)
-      *reinterpret_cast<float2*>(rp.mob + ((size_t)z * sh.Ny + y0 + yy) * NX + 2 * m) = make_float2(o[0].mb, o[1].mb);
-    acc.nonfinite += o[0].bad | o[1].bad;
-  }
-  cluster_barrier<2>();  // no distributed-shared-memory access after this point
-
-  // 5. forward x transform of the local fields -> D
-  passA_rt<M, PM, T, false>(lines, nloc * WY, sh.twM);
-  __syncthreads();
-  const float scale = 1.0f / (float)NX;
-  for (int it = threadIdx.x; it < nloc * WY * NP; it += T) {
-    const int l = it % (nloc * WY), pr = x_run_pair<M>(it / (nloc * WY));
-    const int fl = l / WY, yy = l - fl * WY;
-    x_fwd_runs<M>(rp.D + (fbase + fl) * fstride + row_off + yy, ks, lines + l * PM, pr, scale, sh.twN);
-  }
-  if (!rank) return;
-
-  // 6. diagnostics (rank 1): block reduction into the pair's partials
-  store_block_diag<T>(acc, rp, sh, bp);
 }
 
 }  // namespace pf
