@@ -1,10 +1,23 @@
-// Plain FP64 GPU path and the Fortran-signature shims f_trans_, inv_trans_,
-// k_space_.  Each phase of src/var_diff.f90:561-1050 is one kernel (or one
-// cuFFT call) over global memory, in the reference's order, so this path does
-// the reference's 7*var + 9 three-dimensional transforms per step.
+// FP64 GPU path and the Fortran-signature shims f_trans_, inv_trans_, k_space_.
+//
+// The step of src/var_diff.f90:561-1050 in FP64 over global memory, with cuFFT
+// for the transforms.  FP64 arithmetic is what bounds it (a GB300 SM retires
+// about two FP64 operations a clock, and a transform of 100 x 100 x 90 cells
+// needs 45 M of them), so it runs 2 var + 3 transforms a step (2 more with
+// variable mobility) where the reference takes 7 var + 9:
+//   * the gradient energy (:561-678) by Parseval from the spectra that the
+//     update writes anyway, kept as partial sums for the next step's record,
+//     instead of 4 transforms per field;
+//   * phase 14 is linear, so phi - L dt dF/dphi is formed in real space and
+//     transformed once (:1003-1024 transform phi and dF/dphi);
+//   * the mobility correction is skipped where mob - D_mean is zero.
+// The bulk terms use the two values of gamma (sigma_1, sigma_2) and are linear
+// in var.  100 x 100 x 90, 6 order parameters, variable mobility:
+// FIGURES64
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -42,8 +55,13 @@ static int fail64(int code, const char* fmt, ...) {
     if (r_ != CUFFT_SUCCESS) return fail64(PF_ECUDA, "%s: cufft error %d", #call, (int)r_);      \
   } while (0)
 
-static const int NB = 512;  // blocks of the grid-stride reduction kernels
+static const int NB = 608;  // blocks of the grid-stride reduction kernels: four for each of 152 SMs
 static const int NT = 256;
+static const int NREC = 256;  // steps whose records stay on the device
+// Fields are transformed together as long as their spectra stay within this
+// (half of the L2 cache: transform, update and inverse then hit L2); a larger
+// grid goes field by field.
+static const size_t kChunkBytes = (size_t)64 << 20;
 
 enum P64Acc { PA_FINT = 0, PA_FETA, PA_FCH, PA_MASS, PA_CMIN, PA_CMAX, PA_PHIMIN, PA_PHIPMAX, PA_BAD, PA_COUNT };
 
@@ -57,113 +75,119 @@ struct Plain64 {
   pf_config c;
   int device = 0;
   int Nx, Ny, Nz, Kx, V;
+  int B = 1;                 // fields per batched transform
+  bool var_mob = false;      // mob - D_mean can be non-zero
+  bool have_fint = false;    // fint[cur] holds the gradient energy of the present fields
+  int cur = 0;
   size_t ncell, nspec;
   double* phi = nullptr;     // [V][ncell]
   double* con = nullptr;
-  double* dfdphi = nullptr;  // [V][ncell]
+  double* psi = nullptr;     // [V][ncell]: phi - L dt dF/dphi
   double* dfdc = nullptr;
-  double* mob = nullptr;
-  double* work = nullptr;    // 3 real work arrays
-  cufftDoubleComplex* spec = nullptr;  // 5 spectra
-  double* gamma = nullptr;   // [V][V]
+  double* mob = nullptr;     // mobility (variable mobility only)
+  double* work = nullptr;    // real flux (variable mobility only)
+  cufftDoubleComplex* spec = nullptr;   // c_hat, mu_hat (, J_hat)
+  cufftDoubleComplex* chunk = nullptr;  // B spectra; with set / get also the fields' transfer buffer
+  double* dstage = nullptr;  // = chunk
   double* axes = nullptr;
-  double* part = nullptr;    // [PA_COUNT][NB]
-  double* dstage = nullptr;
+  double* part = nullptr;    // [PA_COUNT][NB] of the bulk kernel
+  double* fint = nullptr;    // [2][V + 1][NB]: gradient energy partials of this and the next fields
+  double* rec = nullptr;     // [NREC][PA_COUNT]
+  void* fftwork = nullptr;   // one work area for all plans: they run in turn
   Axes64 ax;
-  cufftHandle fwd = 0, inv = 0;
+  cufftHandle fwd = 0, inv = 0, fwdB = 0, invB = 0;  // one field, B fields
   cudaStream_t stream = nullptr;
   int steps = 0;
 };
 
+// k-space index of element i (at most 2^29 of them: 32-bit division)
 __device__ __forceinline__ void kidx(size_t i, const Axes64& a, int& kx, int& ky, int& kz) {
-  kx = (int)(i % a.Kx);
-  const size_t r = i / a.Kx;
-  ky = (int)(r % a.Ny);
-  kz = (int)(r / a.Ny);
+  const unsigned j = (unsigned)i, r = j / (unsigned)a.Kx;
+  kx = (int)(j - r * (unsigned)a.Kx);
+  kz = (int)(r / (unsigned)a.Ny);
+  ky = (int)(r - (unsigned)kz * (unsigned)a.Ny);
 }
 
-// phase 1/3: out = in * kf_d / N^3   (kf_d = i * Nyquist-zeroed q_d)
-__global__ void p64_grad_spec(const cufftDoubleComplex* __restrict__ in, cufftDoubleComplex* __restrict__ out,
-                              Axes64 a, int d, double scale, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    int kx, ky, kz;
-    kidx(i, a, kx, ky, kz);
-    const double q = (d == 0 ? a.nx[kx] : (d == 1 ? a.ny[ky] : a.nz[kz])) * scale;
-    const cufftDoubleComplex v = in[i];
-    out[i] = make_cuDoubleComplex(-v.y * q, v.x * q);
-  }
-}
-
-// phase 2/4: f_int += 0.5 kappa (gx^2 + gy^2 + gz^2)
-__global__ void p64_fint(const double* __restrict__ g, size_t n, double coef, double* __restrict__ part) {
-  double s = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    s += 0.5 * coef * (g[i] * g[i] + g[n + i] * g[n + i] + g[2 * n + i] * g[2 * n + i]);
-  __shared__ double sh[NT];
-  sh[threadIdx.x] = s;
+__device__ __forceinline__ double block_sum64(double v, double* sh) {
+  sh[threadIdx.x] = v;
   __syncthreads();
   for (int o = NT / 2; o > 0; o >>= 1) {
     if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[PA_FINT * NB + blockIdx.x] += sh[0];
+  const double r = sh[0];
+  __syncthreads();
+  return r;
 }
 
-// phases 5-9 and the mobility of phase 10 (src/var_diff.f90:685-898), with the
-// reference's O(var^2) loops; statistics and mass of the same fields.
-__global__ void p64_bulk(const double* __restrict__ phi, const double* __restrict__ con, const double* __restrict__ gam,
-                         double* __restrict__ dfdphi, double* __restrict__ dfdc, double* __restrict__ mob, int V,
-                         size_t n, pf_config c, int c1mc, double* __restrict__ part) {
+// Weight times |kf|^2 of a k-point (src/var_diff.f90:561-678 by Parseval): the
+// planes 0 < kx < Nx/2 stand for their conjugates too.
+__device__ __forceinline__ double grad_weight(const Axes64& a, int kx, int ky, int kz) {
+  const double gx = a.nx[kx], gy = a.ny[ky], gz = a.nz[kz];
+  return (gx * gx + gy * gy + gz * gz) * ((kx == 0 || 2 * kx == a.Nx) ? 1.0 : 2.0);
+}
+
+// Gradient energy partials of one spectrum (unnormalised): coef sum w |kf|^2 |s|^2
+__global__ void p64_fint(const cufftDoubleComplex* __restrict__ sp, Axes64 a, double coef, size_t n,
+                         double* __restrict__ out) {
+  __shared__ double sh[NT];
+  double s = 0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    int kx, ky, kz;
+    kidx(i, a, kx, ky, kz);
+    const cufftDoubleComplex v = sp[i];
+    s += grad_weight(a, kx, ky, kz) * (v.x * v.x + v.y * v.y);
+  }
+  s = block_sum64(s, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = coef * s;
+}
+
+// phases 5-9 and the mobility of phase 10 (src/var_diff.f90:685-898);
+// statistics and mass of the same fields.  psi_i = phi_i - L dt dF/dphi_i.
+// With a_i = phi_i^2, S = sum over the matrix variants, Gamma_i = sigma_1
+// (S - a_i) + sigma_2 a_P (matrix), sigma_2 S (precipitate).
+__global__ void p64_bulk(const double* __restrict__ phi, const double* __restrict__ con, double* __restrict__ psi,
+                         double* __restrict__ dfdc, double* __restrict__ mob, int V, size_t n, pf_config c, int c1mc,
+                         double* __restrict__ part) {
+  __shared__ double sh[NT];
   double feta = 0, fch = 0, mass = 0;
   double cmin = 1.0, cmax = 0.0, pmin = 1.0, ppmax = 0.0, bad = 0;
   const int P = V - 1;
+  const double Ldt = c.mob_phi * c.t_step;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    double S = 0, num = 0, pairs = 0;
+    for (int iv = 0; iv < P; ++iv) {
+      const double f = phi[iv * n + i], a = f * f;
+      pairs += a * S;
+      S += a;
+      num += a * a;
+    }
+    const double fP = phi[P * n + i], aP = fP * fP, cc = con[i];
+    const double ssq = S + aP, den = num + aP * aP;
     // phase 5
-    for (int iv = 0; iv < V; ++iv) {
-      const double fi = phi[iv * n + i];
-      feta += -0.5 * fi * fi + 0.25 * fi * fi * fi * fi;
-      for (int jv = iv + 1; jv < V; ++jv) {
-        const double fj = phi[jv * n + i];
-        feta += gam[iv * V + jv] * fi * fi * fj * fj;
-      }
-    }
+    feta += -0.5 * ssq + 0.25 * den + c.sigma_1 * pairs + c.sigma_2 * S * aP;
     // phase 6
-    double num = 0, den = 0;
-    for (int iv = 0; iv < V; ++iv) {
-      const double f = phi[iv * n + i];
-      const double f4 = f * f * f * f;
-      if (iv < P) num += f4;
-      den += f4;
-    }
-    const double cc = con[i];
-    const double pm = num / den, pp = 1.0 - pm;
-    fch += pm * c.am * (cc - c.con_0_mat) * (cc - c.con_0_mat) + pp * c.ap * (cc - c.con_0_ppt) * (cc - c.con_0_ppt);
-    const double dc = 2.0 * pm * c.am * (cc - c.con_0_mat) + 2.0 * pp * c.ap * (cc - c.con_0_ppt);
-    dfdc[i] = dc;
-    // phases 7-9
-    const double fmat = c.am * (cc - c.con_0_mat) * (cc - c.con_0_mat);
-    const double fppt = c.ap * (cc - c.con_0_ppt) * (cc - c.con_0_ppt);
-    const double fP = phi[P * n + i];
-    const double t_2 = 4.0 * fP * fP * fP * (den - fP * fP * fP * fP);
-    double ssq = 0;
-    for (int iv = 0; iv < V; ++iv) {
-      const double fi = phi[iv * n + i];
-      ssq += fi * fi;
-      double t2 = 0;
-      for (int jv = 0; jv < V; ++jv)
-        if (jv != iv) {
-          const double fj = phi[jv * n + i];
-          t2 += 2.0 * gam[iv * V + jv] * fi * fj * fj;
-        }
-      const double t1 = fi * fi * fi - fi;
-      double t4;
-      if (iv < P) t4 = 4.0 * fi * fi * fi * fP * fP * fP * fP * (fmat - fppt) / (den * den);
-      else t4 = t_2 * (fppt - fmat) / (den * den);
-      const double d = t1 + t2 + t4;
+    const double rden = 1.0 / den, r2 = rden * rden;
+    const double pm = num * rden, pp = 1.0 - pm;
+    const double dm = cc - c.con_0_mat, dp = cc - c.con_0_ppt;
+    const double fmat = c.am * dm * dm, fppt = c.ap * dp * dp;
+    fch += pm * fmat + pp * fppt;
+    dfdc[i] = 2.0 * (pm * c.am * dm + pp * c.ap * dp);
+    // phases 7-9: dF = phi (phi^2 - 1 + 2 Gamma) + term4
+    const double t4 = 4.0 * (aP * aP) * r2 * (fmat - fppt);
+    const double g0 = 2.0 * c.sigma_2 * aP - 1.0;
+    for (int iv = 0; iv < P; ++iv) {
+      const double f = phi[iv * n + i], a = f * f;
+      const double d = f * (g0 + a * (1.0 + t4) + 2.0 * c.sigma_1 * (S - a));
       if (!isfinite(d)) bad += 1;
-      dfdphi[iv * n + i] = d;
+      psi[iv * n + i] = f - Ldt * d;
     }
-    mob[i] = c1mc ? c.D_L * (1.0 + cc * (1.0 - cc)) : c.D_L + 2.0 * (1.0 - ssq) * c.D_gb;
+    {
+      const double d = fP * (aP - 1.0 + 2.0 * c.sigma_2 * S + 4.0 * aP * num * r2 * (fppt - fmat));
+      if (!isfinite(d)) bad += 1;
+      psi[P * n + i] = fP - Ldt * d;
+    }
+    if (mob) mob[i] = c1mc ? c.D_L * (1.0 + cc * (1.0 - cc)) : c.D_L + 2.0 * (1.0 - ssq) * c.D_gb;
     // statistics of these fields (src/var_diff.f90:1082-1096)
     mass += cc;
     cmin = fmin(cmin, cc);
@@ -171,14 +195,17 @@ __global__ void p64_bulk(const double* __restrict__ phi, const double* __restric
     pmin = fmin(pmin, ssq);
     ppmax = fmax(ppmax, fP);
   }
-  __shared__ double sh[5][NT];
+  const double q[4] = {feta, fch, mass, bad};
+  const int at[4] = {PA_FETA, PA_FCH, PA_MASS, PA_BAD};
+  for (int k = 0; k < 4; ++k) {
+    const double v = block_sum64(q[k], sh);
+    if (threadIdx.x == 0) part[at[k] * NB + blockIdx.x] = v;
+  }
   __shared__ double sm[4][NT];
-  sh[0][threadIdx.x] = feta; sh[1][threadIdx.x] = fch; sh[2][threadIdx.x] = mass; sh[3][threadIdx.x] = bad;
   sm[0][threadIdx.x] = cmin; sm[1][threadIdx.x] = cmax; sm[2][threadIdx.x] = pmin; sm[3][threadIdx.x] = ppmax;
   __syncthreads();
   for (int o = NT / 2; o > 0; o >>= 1) {
     if (threadIdx.x < o) {
-      for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + o];
       sm[0][threadIdx.x] = fmin(sm[0][threadIdx.x], sm[0][threadIdx.x + o]);
       sm[1][threadIdx.x] = fmax(sm[1][threadIdx.x], sm[1][threadIdx.x + o]);
       sm[2][threadIdx.x] = fmin(sm[2][threadIdx.x], sm[2][threadIdx.x + o]);
@@ -187,10 +214,6 @@ __global__ void p64_bulk(const double* __restrict__ phi, const double* __restric
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    part[PA_FETA * NB + blockIdx.x] = sh[0][0];
-    part[PA_FCH * NB + blockIdx.x] = sh[1][0];
-    part[PA_MASS * NB + blockIdx.x] = sh[2][0];
-    part[PA_BAD * NB + blockIdx.x] = sh[3][0];
     part[PA_CMIN * NB + blockIdx.x] = sm[0][0];
     part[PA_CMAX * NB + blockIdx.x] = sm[1][0];
     part[PA_PHIMIN * NB + blockIdx.x] = sm[2][0];
@@ -219,54 +242,85 @@ __global__ void p64_jmob(double* __restrict__ J, const double* __restrict__ mob,
     J[i] = J[i] * (mob[i] - dmean);
 }
 
-// phase 13: c_hat = (c_hat + J'_hat dt G + D K2 dt mu_hat) / (1 + D dt kappa_c K4)
+// phase 13: c_hat = (c_hat + J'_hat dt G + D K2 dt mu_hat) / (1 + D dt kappa_c K4),
+// and the gradient energy partials of the new field (jp: null without the
+// mobility correction)
 __global__ void p64_ch(cufftDoubleComplex* __restrict__ ch, const cufftDoubleComplex* __restrict__ jp,
                        const cufftDoubleComplex* __restrict__ mu, Axes64 a, double dt, double dm, double kc,
-                       double scale, size_t n) {
+                       double scale, double coef, size_t n, double* __restrict__ fint) {
+  __shared__ double sh[NT];
+  double s = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     int kx, ky, kz;
     kidx(i, a, kx, ky, kz);
-    const double g = a.nx[kx] + a.ny[ky] + a.nz[kz];
-    const double k2 = -(a.qx[kx] * a.qx[kx] + a.qy[ky] * a.qy[ky] + a.qz[kz] * a.qz[kz]);
     const double qx2 = a.qx[kx] * a.qx[kx], qy2 = a.qy[ky] * a.qy[ky], qz2 = a.qz[kz] * a.qz[kz];
+    const double k2 = -(qx2 + qy2 + qz2);
     const double k4 = qx2 * qx2 + qy2 * qy2 + qz2 * qz2;
-    const double den = 1.0 + dm * dt * kc * k4;
-    // J'_hat * dt * (i g)
-    const double t11r = -jp[i].y * scale * dt * g, t11i = jp[i].x * scale * dt * g;
-    const double t33 = dm * k2 * dt * scale;
-    ch[i] = make_cuDoubleComplex((ch[i].x * scale + t11r + t33 * mu[i].x) / den,
-                                 (ch[i].y * scale + t11i + t33 * mu[i].y) / den);
+    const double r = scale / (1.0 + dm * dt * kc * k4);
+    const double t33 = dm * k2 * dt;
+    double re = ch[i].x + t33 * mu[i].x, im = ch[i].y + t33 * mu[i].y;
+    if (jp) {  // J'_hat * dt * (i g)
+      const double g = dt * (a.nx[kx] + a.ny[ky] + a.nz[kz]);
+      re -= jp[i].y * g;
+      im += jp[i].x * g;
+    }
+    re *= r;
+    im *= r;
+    ch[i] = make_cuDoubleComplex(re, im);
+    s += grad_weight(a, kx, ky, kz) * (re * re + im * im);
   }
+  s = block_sum64(s, sh);
+  if (threadIdx.x == 0) fint[blockIdx.x] = coef * s;
 }
 
-// phase 14: phi_hat = (phi_hat - L dt dF_hat) / (1 - L kappa dt K2)
-__global__ void p64_ac(cufftDoubleComplex* __restrict__ ph, const cufftDoubleComplex* __restrict__ df, Axes64 a,
-                       double L, double dt, double kp, double scale, size_t n) {
+// phase 14 of `nb` fields: phi_hat = psi_hat / (1 - L kappa dt K2), and the
+// gradient energy partials of the new fields.  A thread takes one k-point of
+// all of them: one division per point.
+__global__ void p64_ac(cufftDoubleComplex* __restrict__ sp, Axes64 a, double Lkdt, double scale, double coef, size_t n,
+                       int nb, double* __restrict__ fint) {
+  __shared__ double sh[NT];
+  double s = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     int kx, ky, kz;
     kidx(i, a, kx, ky, kz);
-    const double k2 = -(a.qx[kx] * a.qx[kx] + a.qy[ky] * a.qy[ky] + a.qz[kz] * a.qz[kz]);
-    const double den = 1.0 - L * kp * dt * k2;
-    ph[i] = make_cuDoubleComplex((ph[i].x - L * dt * df[i].x) * scale / den, (ph[i].y - L * dt * df[i].y) * scale / den);
+    const double q2 = a.qx[kx] * a.qx[kx] + a.qy[ky] * a.qy[ky] + a.qz[kz] * a.qz[kz];
+    const double r = scale / (1.0 + Lkdt * q2);
+    double e = 0;
+    for (int b = 0; b < nb; ++b) {
+      cufftDoubleComplex* p = sp + (size_t)b * n + i;
+      const double re = p->x * r, im = p->y * r;
+      *p = make_cuDoubleComplex(re, im);
+      e += re * re + im * im;
+    }
+    s += grad_weight(a, kx, ky, kz) * e;
   }
+  s = block_sum64(s, sh);
+  if (threadIdx.x == 0) fint[blockIdx.x] = coef * s;
 }
 
-__global__ void p64_finish(const double* __restrict__ part, double* __restrict__ out) {
-  // one block: fixed-order sums of the block partials
-  __shared__ double s[PA_COUNT];
-  if (threadIdx.x < PA_COUNT) {
-    const int q = threadIdx.x;
-    double v = (q == PA_CMIN || q == PA_PHIMIN) ? 1.0 : ((q == PA_CMAX || q == PA_PHIPMAX) ? 0.0 : 0.0);
-    for (int b = 0; b < NB; ++b) {
-      const double x = part[q * NB + b];
-      if (q == PA_CMIN || q == PA_PHIMIN) v = fmin(v, x);
-      else if (q == PA_CMAX || q == PA_PHIPMAX) v = fmax(v, x);
-      else v += x;
-    }
-    s[q] = v;
+// The step's record: one block per quantity, sums in a fixed order.
+__global__ void p64_finish(const double* __restrict__ part, const double* __restrict__ fint, int nfint,
+                           double* __restrict__ out) {
+  __shared__ double sh[NT];
+  const int q = blockIdx.x;
+  const bool mn = q == PA_CMIN || q == PA_PHIMIN, mx = q == PA_CMAX || q == PA_PHIPMAX;
+  const double* src = q == PA_FINT ? fint : part + q * NB;
+  const int n = q == PA_FINT ? nfint : NB;
+  double v = mn ? 1.0 : 0.0;
+  for (int b = threadIdx.x; b < n; b += NT) {
+    const double x = src[b];
+    v = mn ? fmin(v, x) : (mx ? fmax(v, x) : v + x);
   }
+  sh[threadIdx.x] = v;
   __syncthreads();
-  if (threadIdx.x < PA_COUNT) out[threadIdx.x] = s[threadIdx.x];
+  for (int o = NT / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      const double x = sh[threadIdx.x + o], y = sh[threadIdx.x];
+      sh[threadIdx.x] = mn ? fmin(y, x) : (mx ? fmax(y, x) : y + x);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[q] = sh[0];
 }
 
 __global__ void p64_aos_to_soa(const double* __restrict__ aos, double* __restrict__ soa, int V, size_t n) {
@@ -299,12 +353,12 @@ int plain64_validate(const pf_config* c) {
 void plain64_destroy(Plain64* p) {
   if (!p) return;
   cudaSetDevice(p->device);
-  if (p->fwd) cufftDestroy(p->fwd);
-  if (p->inv) cufftDestroy(p->inv);
+  for (cufftHandle h : {p->fwd, p->inv, p->fwdB, p->invB})
+    if (h) cufftDestroy(h);
   if (p->stream) cudaStreamDestroy(p->stream);
-  cudaFree(p->phi); cudaFree(p->con); cudaFree(p->dfdphi); cudaFree(p->dfdc); cudaFree(p->mob);
-  cudaFree(p->work); cudaFree(p->spec); cudaFree(p->gamma); cudaFree(p->axes); cudaFree(p->part);
-  cudaFree(p->dstage);
+  cudaFree(p->phi); cudaFree(p->con); cudaFree(p->psi); cudaFree(p->dfdc); cudaFree(p->mob);
+  cudaFree(p->work); cudaFree(p->spec); cudaFree(p->chunk); cudaFree(p->axes); cudaFree(p->part);
+  cudaFree(p->fint); cudaFree(p->rec); cudaFree(p->fftwork);
   delete p;
 }
 
@@ -321,49 +375,62 @@ int plain64_create(const pf_config* c, Plain64** out) {
 #define TRY(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) \
     return bail(fail64(PF_ENOMEM, "%s: %s", #call, cudaGetErrorString(e_))); } while (0)
   TRY(cudaSetDevice(p->device));
+  p->var_mob = c->mobility == PF_MOB_C1MC || c->D_gb != 0.0;
+  {
+    // chunks of (nearly) equal size
+    const size_t fit = std::max<size_t>(1, kChunkBytes / (p->nspec * sizeof(cufftDoubleComplex)));
+    const int chunks = (int)((p->V + fit - 1) / fit);
+    p->B = (p->V + chunks - 1) / chunks;
+  }
+  const size_t chunk_bytes = std::max(p->B * p->nspec * sizeof(cufftDoubleComplex), p->V * p->ncell * sizeof(double));
   TRY(cudaMalloc(&p->phi, p->V * p->ncell * sizeof(double)));
   TRY(cudaMalloc(&p->con, p->ncell * sizeof(double)));
-  TRY(cudaMalloc(&p->dfdphi, p->V * p->ncell * sizeof(double)));
+  TRY(cudaMalloc(&p->psi, p->V * p->ncell * sizeof(double)));
   TRY(cudaMalloc(&p->dfdc, p->ncell * sizeof(double)));
-  TRY(cudaMalloc(&p->mob, p->ncell * sizeof(double)));
-  TRY(cudaMalloc(&p->work, 3 * p->ncell * sizeof(double)));
-  TRY(cudaMalloc(&p->spec, 5 * p->nspec * sizeof(cufftDoubleComplex)));
-  TRY(cudaMalloc(&p->gamma, (size_t)p->V * p->V * sizeof(double)));
+  if (p->var_mob) TRY(cudaMalloc(&p->mob, p->ncell * sizeof(double)));
+  if (p->var_mob) TRY(cudaMalloc(&p->work, p->ncell * sizeof(double)));
+  TRY(cudaMalloc(&p->spec, 3 * p->nspec * sizeof(cufftDoubleComplex)));
+  TRY(cudaMalloc(&p->chunk, chunk_bytes));
+  p->dstage = reinterpret_cast<double*>(p->chunk);
   TRY(cudaMalloc(&p->axes, 2 * (size_t)(p->Kx + p->Ny + p->Nz) * sizeof(double)));
-  TRY(cudaMalloc(&p->part, (PA_COUNT * NB + PA_COUNT) * sizeof(double)));
-  TRY(cudaMalloc(&p->dstage, (p->V + 1) * p->ncell * sizeof(double)));
+  TRY(cudaMalloc(&p->part, PA_COUNT * NB * sizeof(double)));
+  TRY(cudaMalloc(&p->fint, 2 * (size_t)(p->V + 1) * NB * sizeof(double)));
+  TRY(cudaMemset(p->fint, 0, 2 * (size_t)(p->V + 1) * NB * sizeof(double)));
+  TRY(cudaMalloc(&p->rec, NREC * PA_COUNT * sizeof(double)));
   TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
 #undef TRY
-  // gamma (src/var_diff.f90:206-218)
-  std::vector<double> g((size_t)p->V * p->V, 0.0);
-  const int mat = p->V - 1;
-  for (int j = 1; j <= p->V; ++j)
-    for (int i = 1; i <= p->V; ++i) {
-      double v = 0.0;
-      if (i != j && i <= mat && j <= mat) v = c->sigma_1;
-      if (j == p->V && i < p->V) v = c->sigma_2;
-      if (i == p->V && j < p->V) v = c->sigma_2;
-      g[(size_t)(i - 1) * p->V + (j - 1)] = v;
-    }
   std::vector<double> ax(2 * (size_t)(p->Kx + p->Ny + p->Nz));
   double* hq = ax.data();
   double* hn = ax.data() + (p->Kx + p->Ny + p->Nz);
   host_axis(p->Nx, p->Kx, hq, hn);
   host_axis(p->Ny, p->Ny, hq + p->Kx, hn + p->Kx);
   host_axis(p->Nz, p->Nz, hq + p->Kx + p->Ny, hn + p->Kx + p->Ny);
-  cudaError_t e = cudaMemcpy(p->gamma, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p->axes, ax.data(), ax.size() * sizeof(double), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpy(p->axes, ax.data(), ax.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return bail(fail64(PF_ECUDA, "table upload: %s", cudaGetErrorString(e)));
   const double* dq = p->axes;
   const double* dn = p->axes + (p->Kx + p->Ny + p->Nz);
   p->ax.qx = dq; p->ax.qy = dq + p->Kx; p->ax.qz = dq + p->Kx + p->Ny;
   p->ax.nx = dn; p->ax.ny = dn + p->Kx; p->ax.nz = dn + p->Kx + p->Ny;
   p->ax.Nx = p->Nx; p->ax.Ny = p->Ny; p->ax.Nz = p->Nz; p->ax.Kx = p->Kx;
-  if (cufftPlan3d(&p->fwd, p->Nz, p->Ny, p->Nx, CUFFT_D2Z) != CUFFT_SUCCESS ||
-      cufftPlan3d(&p->inv, p->Nz, p->Ny, p->Nx, CUFFT_Z2D) != CUFFT_SUCCESS)
-    return bail(fail64(PF_ECUDA, "cufftPlan3d failed"));
-  cufftSetStream(p->fwd, p->stream);
-  cufftSetStream(p->inv, p->stream);
+  // plans of one field and of B fields, sharing one work area
+  size_t need = 0;
+  auto plan = [&](cufftHandle* h, cufftType type, int batch) {
+    int dims[3] = {p->Nz, p->Ny, p->Nx};
+    size_t ws = 0;
+    if (cufftCreate(h) != CUFFT_SUCCESS || cufftSetAutoAllocation(*h, 0) != CUFFT_SUCCESS ||
+        cufftMakePlanMany(*h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, type, batch, &ws) != CUFFT_SUCCESS)
+      return false;
+    need = std::max(need, ws);
+    return true;
+  };
+  if (!plan(&p->fwd, CUFFT_D2Z, 1) || !plan(&p->inv, CUFFT_Z2D, 1) ||
+      (p->B > 1 && (!plan(&p->fwdB, CUFFT_D2Z, p->B) || !plan(&p->invB, CUFFT_Z2D, p->B))))
+    return bail(fail64(PF_ECUDA, "cufftMakePlanMany failed"));
+  if (need && cudaMalloc(&p->fftwork, need) != cudaSuccess)
+    return bail(fail64(PF_ENOMEM, "cuFFT work area of %zu bytes", need));
+  for (cufftHandle h : {p->fwd, p->inv, p->fwdB, p->invB})
+    if (h && (cufftSetWorkArea(h, p->fftwork) != CUFFT_SUCCESS || cufftSetStream(h, p->stream) != CUFFT_SUCCESS))
+      return bail(fail64(PF_ECUDA, "cufftSetWorkArea failed"));
   *out = p;
   return PF_OK;
 }
@@ -376,6 +443,7 @@ int plain64_set_fields(Plain64* p, const double* phi, const double* con) {
   P64_CUDA(cudaMemcpyAsync(p->con, con, p->ncell * sizeof(double), cudaMemcpyHostToDevice, p->stream));
   P64_CUDA(cudaStreamSynchronize(p->stream));
   p->steps = 0;
+  p->have_fint = false;
   return PF_OK;
 }
 
@@ -402,50 +470,61 @@ int plain64_device_fields(Plain64* p, DeviceFields* out) {
   return PF_OK;
 }
 
-static int one_step(Plain64* p, double* acc_out) {
+// nb fields (B, or 1) forward into the chunk buffer, or back from it.
+static int fft_chunk(Plain64* p, bool forward, double* real, int nb) {
+  cufftHandle h = nb > 1 ? (forward ? p->fwdB : p->invB) : (forward ? p->fwd : p->inv);
+  if (forward) P64_FFT(cufftExecD2Z(h, real, p->chunk));
+  else P64_FFT(cufftExecZ2D(h, p->chunk, real));
+  return PF_OK;
+}
+
+static int one_step(Plain64* p, double* rec) {
   const size_t n = p->ncell, ns = p->nspec;
   const double scale = 1.0 / (double)n;  // f_trans normalisation (src/f_trans.f90:12)
   cudaStream_t s = p->stream;
-  cufftDoubleComplex* W0 = p->spec;
-  cufftDoubleComplex* W1 = p->spec + ns;
-  cufftDoubleComplex* W2 = p->spec + 2 * ns;
-  cufftDoubleComplex* W3 = p->spec + 3 * ns;
-  cufftDoubleComplex* W4 = p->spec + 4 * ns;
+  cufftDoubleComplex *W0 = p->spec, *W1 = p->spec + ns, *W2 = p->spec + 2 * ns;
   const pf_config& c = p->c;
-  P64_CUDA(cudaMemsetAsync(p->part, 0, PA_COUNT * NB * sizeof(double), s));
-  // phases 1-4: gradient energy through 3 inverse transforms per field
-  for (int f = 0; f <= p->V; ++f) {
-    double* u = (f < p->V) ? p->phi + (size_t)f * n : p->con;
-    P64_FFT(cufftExecD2Z(p->fwd, u, W0));
-    for (int d = 0; d < 3; ++d) {
-      p64_grad_spec<<<NB, NT, 0, s>>>(W0, W1, p->ax, d, scale, ns);
-      P64_FFT(cufftExecZ2D(p->inv, W1, p->work + d * n));
+  const double ecoef = 0.5 * (double)n;  // 0.5 kappa N^3 sum w |kf|^2 |u_hat|^2
+  const size_t nfint = (size_t)(p->V + 1) * NB;
+  double *now = p->fint + p->cur * nfint, *next = p->fint + (1 - p->cur) * nfint;
+  auto chunk_at = [&](int f) { return f + p->B <= p->V ? p->B : 1; };
+  int rc;
+  if (!p->have_fint) {  // the first step after set_fields: phases 1-4 from the fields' own spectra
+    for (int f = 0; f <= p->V; ++f) {
+      P64_FFT(cufftExecD2Z(p->fwd, f < p->V ? p->phi + (size_t)f * n : p->con, W0));
+      p64_fint<<<NB, NT, 0, s>>>(W0, p->ax, ecoef * (f < p->V ? c.grad_coeff_phi : c.grad_coeff_c) * scale * scale, ns,
+                                 now + (size_t)f * NB);
     }
-    p64_fint<<<NB, NT, 0, s>>>(p->work, n, f < p->V ? c.grad_coeff_phi : c.grad_coeff_c, p->part);
+    p->have_fint = true;
   }
   // phases 5-10 (bulk), statistics of the same fields
-  p64_bulk<<<NB, NT, 0, s>>>(p->phi, p->con, p->gamma, p->dfdphi, p->dfdc, p->mob, p->V, n, c,
-                             c.mobility == PF_MOB_C1MC, p->part);
+  p64_bulk<<<NB, NT, 0, s>>>(p->phi, p->con, p->psi, p->dfdc, p->mob, p->V, n, c, c.mobility == PF_MOB_C1MC, p->part);
   P64_FFT(cufftExecD2Z(p->fwd, p->con, W0));   // dft_con
   P64_FFT(cufftExecD2Z(p->fwd, p->dfdc, W1));  // dft_df_dc
-  // phase 11-12: variable-mobility flux
-  p64_flux<<<NB, NT, 0, s>>>(W0, W1, W2, p->ax, c.grad_coeff_c, scale, ns);
-  P64_FFT(cufftExecZ2D(p->inv, W2, p->work));
-  p64_jmob<<<NB, NT, 0, s>>>(p->work, p->mob, c.D_L, n);
-  P64_FFT(cufftExecD2Z(p->fwd, p->work, W3));
-  // phase 13
-  p64_ch<<<NB, NT, 0, s>>>(W0, W3, W1, p->ax, c.t_step, c.D_L, c.grad_coeff_c, scale, ns);
-  P64_FFT(cufftExecZ2D(p->inv, W0, p->con));
-  // phase 14
-  for (int f = 0; f < p->V; ++f) {
-    P64_FFT(cufftExecD2Z(p->fwd, p->phi + (size_t)f * n, W0));
-    P64_FFT(cufftExecD2Z(p->fwd, p->dfdphi + (size_t)f * n, W4));
-    p64_ac<<<NB, NT, 0, s>>>(W0, W4, p->ax, c.mob_phi, c.t_step, c.grad_coeff_phi, scale, ns);
-    P64_FFT(cufftExecZ2D(p->inv, W0, p->phi + (size_t)f * n));
+  if (p->var_mob) {  // phases 11-12: variable-mobility flux
+    p64_flux<<<NB, NT, 0, s>>>(W0, W1, W2, p->ax, c.grad_coeff_c, scale, ns);
+    P64_FFT(cufftExecZ2D(p->inv, W2, p->work));
+    p64_jmob<<<NB, NT, 0, s>>>(p->work, p->mob, c.D_L, n);
+    P64_FFT(cufftExecD2Z(p->fwd, p->work, W2));
   }
-  p64_finish<<<1, 32, 0, s>>>(p->part, p->part + PA_COUNT * NB);
+  // phase 13
+  p64_ch<<<NB, NT, 0, s>>>(W0, p->var_mob ? W2 : nullptr, W1, p->ax, c.t_step, c.D_L, c.grad_coeff_c, scale,
+                           ecoef * c.grad_coeff_c, ns, next + (size_t)p->V * NB);
+  P64_FFT(cufftExecZ2D(p->inv, W0, p->con));
+  // phase 14; a chunk's partials go to its first field's slot, the others stay zero
+  for (int f = 0; f < p->V;) {
+    const int nb = chunk_at(f);
+    if ((rc = fft_chunk(p, true, p->psi + (size_t)f * n, nb))) return rc;
+    p64_ac<<<NB, NT, 0, s>>>(p->chunk, p->ax, c.mob_phi * c.grad_coeff_phi * c.t_step, scale, ecoef * c.grad_coeff_phi,
+                             ns, nb, next + (size_t)f * NB);
+    if ((rc = fft_chunk(p, false, p->phi + (size_t)f * n, nb))) return rc;
+    f += nb;
+  }
+  p64_finish<<<PA_COUNT, NT, 0, s>>>(p->part, now, (int)nfint, rec);
+  if (p->B > 1)  // the start's per-field partials must not stay in the slots that chunks leave alone
+    P64_CUDA(cudaMemsetAsync(now, 0, nfint * sizeof(double), s));
+  p->cur = 1 - p->cur;
   P64_CUDA(cudaGetLastError());
-  P64_CUDA(cudaMemcpyAsync(acc_out, p->part + PA_COUNT * NB, PA_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
   return PF_OK;
 }
 
@@ -454,11 +533,16 @@ int plain64_step(Plain64* p, int nsteps, pf_diag* diag) {
   P64_CUDA(cudaSetDevice(p->device));
   int bad = 0;
   std::vector<double> acc((size_t)std::max(nsteps, 1) * PA_COUNT);
-  for (int st = 0; st < nsteps; ++st) {
-    int rc = one_step(p, acc.data() + (size_t)st * PA_COUNT);
-    if (rc) return rc;
+  for (int st = 0; st < nsteps; st += NREC) {
+    const int m = std::min(NREC, nsteps - st);
+    for (int k = 0; k < m; ++k) {
+      int rc = one_step(p, p->rec + (size_t)k * PA_COUNT);
+      if (rc) return rc;
+    }
+    P64_CUDA(cudaMemcpyAsync(acc.data() + (size_t)st * PA_COUNT, p->rec, (size_t)m * PA_COUNT * sizeof(double),
+                             cudaMemcpyDeviceToHost, p->stream));
+    P64_CUDA(cudaStreamSynchronize(p->stream));
   }
-  P64_CUDA(cudaStreamSynchronize(p->stream));
   for (int st = 0; st < nsteps; ++st) {
     const double* a = acc.data() + (size_t)st * PA_COUNT;
     if (a[PA_BAD] != 0) bad = 1;
