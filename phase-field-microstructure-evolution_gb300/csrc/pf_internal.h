@@ -10,9 +10,9 @@ namespace pf {
 
 typedef void (*KernelFn)(const RunParams*, const Shape);
 
-// One compiled variant of the x pass (all four modes) ...
+// One compiled variant of the x pass (all modes) ...
 struct XKernels {
-  KernelFn bulk, xj, imp, exp;
+  KernelFn bulk, xj, imp, exp, fields;
   int wy;           // y rows per CTA
   int threads;      // threads per CTA
   const char* tag;  // how the tile is loaded and walked and the CTAs per SM asked for, for reports
@@ -49,6 +49,7 @@ static int add_x(XKernels* out, int n, const char* tag = "") {
   k.xj = x_pass_kernel<NX, WY, T, MODE_XJ, PHYS, ASYNC>;
   k.imp = x_pass_kernel<NX, WY, T, MODE_IMPORT>;
   k.exp = x_pass_kernel<NX, WY, T, MODE_EXPORT, PHYS, ASYNC>;
+  k.fields = x_pass_kernel<NX, WY, T, MODE_FIELDS, PHYS, ASYNC>;
   k.wy = WY;
   k.threads = T;
   k.tag = tag;

@@ -66,7 +66,8 @@ struct RunParams {
   float* part_yz;  // [2][2][nblk_yz]: per step parity, hi and lo of each yz CTA's weighted f_int sum
   double* diag;    // [ring][DR_COUNT]
   int* counter;    // step counter (device)
-  float* fin;      // [nF][Nz][Ny][Nx] real fields for import/export
+  float* fin;      // [nF][Nz][Ny][Nx] float fields (MODE_FIELDS)
+  double* aos;     // fields in the caller's layout: phi(var, x, y, z), then con(x, y, z)
   float L, kappa_phi, kappa_c, dt, D_L, D_gb, sigma1, sigma2, am, ap, c0m, c0p;
   int mobility;
   int V;           // number of order parameters
@@ -683,10 +684,34 @@ __device__ __forceinline__ void bulk_tile(float2* smem, const RunParams& rp, con
 
 // ---------------------------------------------------------------------------
 // x pass.  MODE_BULK: S -> D (+ mob, diagnostics).  MODE_XJ: J~ -> J~' with the
-// variable-mobility multiply (:947-965).  MODE_IMPORT: real fields -> S.
-// MODE_EXPORT: S -> real fields.
+// variable-mobility multiply (:947-965).  MODE_IMPORT: the caller's fields
+// (phi(var, x, y, z) and con, REAL*8) -> S.  MODE_EXPORT: S -> the caller's
+// fields.  MODE_FIELDS: S -> float fields [f][z][y][x].
+// A tile's rows are one contiguous piece of the caller's layout, so import and
+// export read and write it in full lines straight from and to shared memory.
 // ---------------------------------------------------------------------------
-enum XMode { MODE_BULK = 0, MODE_XJ = 1, MODE_IMPORT = 2, MODE_EXPORT = 3 };
+enum XMode { MODE_BULK = 0, MODE_XJ = 1, MODE_IMPORT = 2, MODE_EXPORT = 3, MODE_FIELDS = 4 };
+
+// Walk over the cells of a tile in the caller's layout: op(value in memory,
+// its place in the tile's lines) for phi (field fastest), then con.
+template <int NX, int WY, int T, class Op>
+__device__ __forceinline__ void walk_tile(float2* smem, double* aos, int V, size_t ncell, size_t cell0, Op op) {
+  using LM = XLine<NX / 2>;
+  float* lines = reinterpret_cast<float*>(smem);
+  const auto place = [&](int f, int cell) {
+    const int yy = cell / NX, x = cell % NX;
+    return lines + 2 * ((f * WY + yy) * LM::PITCH + LM::phys(x >> 1)) + (x & 1);
+  };
+  const FastDiv by_v(V);
+  double* phi = aos + cell0 * V;
+#pragma unroll 4
+  for (int it = threadIdx.x; it < WY * NX * V; it += T) {
+    const int cell = by_v(it);
+    op(phi + it, place(it - cell * V, cell));
+  }
+  double* con = aos + ncell * V + cell0;
+  for (int it = threadIdx.x; it < WY * NX; it += T) op(con + it, place(V, it));
+}
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -735,12 +760,8 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
   const float2* __restrict__ src = (MODE == MODE_XJ) ? rp.J : rp.Sm;
 
   if (MODE == MODE_IMPORT) {
-    // real rows -> interleaved lines (natural order)
-    for (int it = threadIdx.x; it < nF * WY * M; it += T) {
-      const int m = it % M, r = it / M, yy = r % WY, f = r / WY;
-      const float2 v = *reinterpret_cast<const float2*>(rp.fin + (((size_t)f * sh.Nz + z) * sh.Ny + y0 + yy) * NX + 2 * m);
-      smem[(f * WY + yy) * PM + LM::phys(m)] = v;
-    }
+    walk_tile<NX, WY, T>(smem, rp.aos, rp.V, (size_t)sh.Nz * sh.Ny * NX, (size_t)(z * sh.Ny + y0) * NX,
+                         [](const double* v, float* at) { *at = (float)*v; });
   } else {
     // 1. inverse x transform: global half spectrum -> pre-processing -> pass B'
     // a warp covers consecutive (y row, field) lines at one run pair: the
@@ -773,6 +794,11 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
   __syncthreads();
 
   if (MODE == MODE_EXPORT) {
+    walk_tile<NX, WY, T>(smem, rp.aos, rp.V, (size_t)sh.Nz * sh.Ny * NX, (size_t)(z * sh.Ny + y0) * NX,
+                         [](double* v, const float* at) { *v = (double)*at; });
+    return;
+  }
+  if (MODE == MODE_FIELDS) {
     for (int it = threadIdx.x; it < nF * WY * M; it += T) {
       const int m = it % M, r = it / M, yy = r % WY, f = r / WY;
       *reinterpret_cast<float2*>(rp.fin + (((size_t)f * sh.Nz + z) * sh.Ny + y0 + yy) * NX + 2 * m) =
