@@ -4,7 +4,7 @@
 // concentration c):
 //   Sk[f][kx][ypos][zpos]  u_hat in k-space (normalised like f_trans,
 //                          src/f_trans.f90:12), y/z in digit-transposed order;
-//   Sm[f][kx][z][y]        the same field in "mixed" space: its x half
+//   Sm[f][kx][z][y]        (large runs: [f][z][kx][y]) the same field in "mixed" space: its x half
 //                          spectrum (1/Nx) sum_x u e^{-2 pi i kx x/Nx} with y, z
 //                          in real space (what the x pass needs).
 // The reference keeps phi/con in real space and takes a full 3-D R2C per
@@ -58,10 +58,10 @@ enum Mobility { MOB_CONST = 0, MOB_REF_VAR = 1, MOB_C1MC = 2 };
 struct RunParams {
   float2* Sk;      // [nF][Kx] planes of the k-space state (digit-transposed y, z positions; the
                    // order inside a plane belongs to the yz-pass variant that runs the batch)
-  float2* Sm;      // [nF][Kx][Nz][Ny] state in mixed space (x spectrum, real-space y, z)
-  float2* D;       // [nF][Kx][Nz][Ny] x-spectra of dF/dphi_i and dF/dc
+  float2* Sm;      // [nF] x Kx, Nz, Ny (strides ks, zs, 1): state in mixed space (x spectrum, real-space y, z)
+  float2* D;       // as Sm: x-spectra of dF/dphi_i and dF/dc
   float* mob;      // [Nz][Ny][Nx] mobility minus D_mean (variable mobility only)
-  float2* J;       // [Kx][Nz][Ny] CH flux scratch (variable mobility only)
+  float2* J;       // one field as Sm: CH flux scratch (variable mobility only)
   float* part_x;   // [2][XQ_COUNT][nblk_x]: per step parity
   float* part_yz;  // [2][2][nblk_yz]: per step parity, hi and lo of each yz CTA's weighted f_int sum
   double* diag;    // [ring][DR_COUNT]
