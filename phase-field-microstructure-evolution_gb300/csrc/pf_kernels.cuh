@@ -1126,7 +1126,7 @@ __device__ __forceinline__ void cluster_barrier() { cg::this_cluster().sync(); }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
   uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
   return r;
 }
 __device__ __forceinline__ float2 ld_peer(uint32_t a) {
@@ -1140,50 +1140,66 @@ __device__ __forceinline__ float2 ld_peer(uint32_t a) {
 // cluster waits until every CTA has read everything it needs, and then each
 // CTA overwrites its own buffer with the new layout.  One buffer per CTA
 // instead of two, so a quarter of a 256 x 256 plane (140 KB) fits one CTA.
-template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_AB(float2* __restrict__ buf, uint32_t A_base, int r) {
-  using G = YZ<NY, NZ, C>;
-  constexpr int TOTAL = G::LB * NZ;
-  static_assert(T % G::LB == 0 && TOTAL % T == 0, "threads must cover whole rows");
-  constexpr int S = T / G::LB;
-  constexpr int ITER = TOTAL / T;
-  const int yl = threadIdx.x % G::LB;
-  const int z0 = threadIdx.x / G::LB;
-  const uint32_t src_off = (uint32_t)(Line<NY>::phys(r * G::LB + yl)) * 8u;
+//
+// One side of an exchange: CTA r gets, for its own position of the old lines
+// (at src, pitch PS), the elements of lines x0 + k S of the cluster, LS lines
+// per CTA, and stores them as one line of the new layout (at dst, runs of N1).
+// Every CTA starts with its own lines and goes round, so that no CTA's shared
+// memory serves all the others at once.
+template <int C, int LS, int PS, int N1, int S, int ITER>
+__device__ __forceinline__ void exchange(float2* __restrict__ dst, uint32_t src, int x0, int r) {
   float2 v[ITER];
+  if constexpr (LS % S == 0 && LS % N1 == 0) {
+    constexpr int J = LS / S;
 #pragma unroll
-  for (int k = 0; k < ITER; ++k) {
-    const int z = z0 + k * S;
-    const int owner = z / G::LA, zl = z - owner * G::LA;
-    v[k] = ld_peer(map_rank(A_base + (uint32_t)(zl * G::PY) * 8u + src_off, owner));
+    for (int i = 0; i < C; ++i) {
+      const int o = r + i < C ? r + i : r + i - C;
+      const uint32_t a = map_rank(src + (uint32_t)(x0 * PS) * 8u, o);
+#pragma unroll
+      for (int j = 0; j < J; ++j) v[i * J + j] = ld_peer(a + (uint32_t)(j * S * PS * 8));
+    }
+    cluster_barrier();  // every CTA holds its new layout in registers
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const int o = r + i < C ? r + i : r + i - C;
+      float2* d = dst + o * (LS + LS / N1) + x0;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        if constexpr (N1 % S == 0) d[j * S + (j * S) / N1] = v[i * J + j];  // x0 < S
+        else d[j * S + (x0 + j * S) / N1] = v[i * J + j];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < ITER; ++k) {
+      const int x = x0 + k * S, owner = x / LS;
+      v[k] = ld_peer(map_rank(src + (uint32_t)((x - owner * LS) * PS) * 8u, owner));
+    }
+    cluster_barrier();
+#pragma unroll
+    for (int k = 0; k < ITER; ++k) dst[x0 + k * S + (x0 + k * S) / N1] = v[k];
   }
-  cluster_barrier();  // every CTA holds its new layout in registers
-#pragma unroll
-  for (int k = 0; k < ITER; ++k) buf[yl * G::PZ + Line<NZ>::phys(z0 + k * S)] = v[k];
   __syncthreads();
 }
 
+// A (z rows of LA, pitch PY) -> B (y positions of LB, pitch PZ)
 template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_BA(float2* __restrict__ buf, uint32_t B_base, int r) {
+__device__ __forceinline__ void exch_AB(float2* __restrict__ buf, uint32_t base, int r) {
   using G = YZ<NY, NZ, C>;
-  constexpr int TOTAL = G::LA * NY;
-  static_assert(T % G::LA == 0 && TOTAL % T == 0, "threads must cover whole lines");
-  constexpr int S = T / G::LA;
-  constexpr int ITER = TOTAL / T;
+  static_assert(T % G::LB == 0 && (G::LB * NZ) % T == 0, "threads must cover whole rows");
+  const int yl = threadIdx.x % G::LB;
+  exchange<C, G::LA, G::PY, Line<NZ>::N1, T / G::LB, G::LB * NZ / T>(
+      buf + yl * G::PZ, base + (uint32_t)(Line<NY>::phys(r * G::LB + yl)) * 8u, threadIdx.x / G::LB, r);
+}
+
+// B -> A
+template <int NY, int NZ, int C, int T>
+__device__ __forceinline__ void exch_BA(float2* __restrict__ buf, uint32_t base, int r) {
+  using G = YZ<NY, NZ, C>;
+  static_assert(T % G::LA == 0 && (G::LA * NY) % T == 0, "threads must cover whole lines");
   const int zl = threadIdx.x % G::LA;
-  const int y0 = threadIdx.x / G::LA;
-  const uint32_t src_off = (uint32_t)(Line<NZ>::phys(r * G::LA + zl)) * 8u;
-  float2 v[ITER];
-#pragma unroll
-  for (int k = 0; k < ITER; ++k) {
-    const int y = y0 + k * S;
-    const int owner = y / G::LB, yl = y - owner * G::LB;
-    v[k] = ld_peer(map_rank(B_base + (uint32_t)(yl * G::PZ) * 8u + src_off, owner));
-  }
-  cluster_barrier();  // no CTA reads a peer's buffer after this point
-#pragma unroll
-  for (int k = 0; k < ITER; ++k) buf[zl * G::PY + Line<NY>::phys(y0 + k * S)] = v[k];
-  __syncthreads();
+  exchange<C, G::LB, G::PZ, Line<NY>::N1, T / G::LA, G::LA * NY / T>(
+      buf + zl * G::PY, base + (uint32_t)(Line<NZ>::phys(r * G::LA + zl)) * 8u, threadIdx.x / G::LA, r);
 }
 
 // pass A (forward or inverse) over NL lines of length L, pitch P, T threads

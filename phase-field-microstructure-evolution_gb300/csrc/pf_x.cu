@@ -11,7 +11,7 @@ int x_variants_a(int nx, XKernels* out, int n) {
     case 16: n = add_x<16, 16, 256>(out, n); break;
     case 32: n = add_x<32, 4, 128>(out, n); n = add_x<32, 8, 256>(out, n); break;
     case 64:
-      n = add_x<64, 16, 256, 3>(out, n, ",3/SM");
+      n = add_x<64, 16, 256, 3, false>(out, n, ",logical,3/SM");
       n = add_x<64, 8, 256>(out, n);
       n = add_x<64, 4, 128>(out, n);
       break;

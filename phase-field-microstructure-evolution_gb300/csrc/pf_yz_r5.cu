@@ -16,9 +16,10 @@ int yz_variants_r5(int ny, int nz, YZKernels* out, int n) {
     n = add_yz1<102, 102, 448, false, 2>(out, n);
     n = add_yz1<102, 102, 256, false>(out, n);
   }
-  // two clusters' CTAs per SM, one buffer each and k-space values five at a time: yz pass of 7 fields
-  // 614 -> 461 us against separate A and B buffers (135 KB, one CTA per SM)
-  if (ny == 200 && nz == 200) n = add_yz<200, 200, 5, 320, 2, 5>(out, n);
+  // two clusters' CTAs per SM, one buffer each and k-space values ten at a time: yz pass of 7 fields
+  // 614 -> 432 us against separate A and B buffers (135 KB, one CTA per SM); clusters of 2 x 800
+  // threads and of 10 x 160 were 2 to 5 % slower
+  if (ny == 200 && nz == 200) n = add_yz<200, 200, 5, 320, 2, 10>(out, n);
   return n;
 }
 
