@@ -132,19 +132,26 @@ static int build_tables(int Nx, int Ny, int Nz, int nF, DevTables& t) {
   return PF_OK;
 }
 
-static size_t x_smem(int nx, int nF, int wy) {
+// Shared memory of the x pass's lines; with `limit`, what the public limit on
+// var is counted with (lines with a pad slot after every run, as they once
+// were: what fits has grown since, the limit has not).
+template <int M>
+static constexpr int x_pitch(bool limit) {
+  return limit ? Line<M, XLine<M>::N1, XLine<M>::N2>::PITCH : XLine<M>::PITCH;
+}
+static size_t x_smem(int nx, int nF, int wy, bool limit = false) {
   int pitch;
   switch (nx) {
-    case 16: pitch = XLine<8>::PITCH; break;
-    case 32: pitch = XLine<16>::PITCH; break;
-    case 64: pitch = XLine<32>::PITCH; break;
-    case 96: pitch = XLine<48>::PITCH; break;
-    case 128: pitch = XLine<64>::PITCH; break;
-    case 256: pitch = XLine<128>::PITCH; break;
-    case 80: pitch = XLine<40>::PITCH; break;
-    case 160: pitch = XLine<80>::PITCH; break;
-    case 200: pitch = XLine<100>::PITCH; break;
-    case 102: pitch = XLine<51>::PITCH; break;
+    case 16: pitch = x_pitch<8>(limit); break;
+    case 32: pitch = x_pitch<16>(limit); break;
+    case 64: pitch = x_pitch<32>(limit); break;
+    case 96: pitch = x_pitch<48>(limit); break;
+    case 128: pitch = x_pitch<64>(limit); break;
+    case 256: pitch = x_pitch<128>(limit); break;
+    case 80: pitch = x_pitch<40>(limit); break;
+    case 160: pitch = x_pitch<80>(limit); break;
+    case 200: pitch = x_pitch<100>(limit); break;
+    case 102: pitch = x_pitch<51>(limit); break;
     default: return 0;
   }
   return (size_t)nF * wy * pitch * sizeof(float2);
@@ -174,7 +181,7 @@ static int validate(const pf_config* c) {
   for (int i = 0; i < nxv; ++i) {
     // at Nx = 32 the 8-row tiles set the limit on var: the 4-row ones are there for latency
     const int wy = c->nx == 32 ? std::max(xv[i].wy, 8) : xv[i].wy;
-    fits = fits || (c->ny % wy == 0 && x_smem(c->nx, c->var + 1, wy) + x_static_smem(c->nx) <= kMaxSmem);
+    fits = fits || (c->ny % wy == 0 && x_smem(c->nx, c->var + 1, wy, true) + x_static_smem(c->nx) <= kMaxSmem);
   }
   if (!fits) return fail(PF_EINVAL, "var=%d with Nx=%d, Ny=%d does not fit the x pass", c->var, c->nx, c->ny);
   if (c->mobility != PF_MOB_REFERENCE && c->mobility != PF_MOB_C1MC)

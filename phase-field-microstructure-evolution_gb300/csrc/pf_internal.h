@@ -38,18 +38,17 @@ int yz_variants_256(int ny, int nz, YZKernels* out, int n);
 int yz_variants_r5(int ny, int nz, YZKernels* out, int n);
 
 // An x-pass variant: WY rows and T threads per CTA, at least MINB CTAs per SM
-// (0: as many registers as the compiler likes).  PHYS: the bulk walk over
-// physical slots; ASYNC: the tile's spectra copied in by cp.async and
-// transformed in place.
-template <int NX, int WY, int T, int MINB = 0, bool PHYS = true, bool ASYNC = false>
+// (0: as many registers as the compiler likes).  ASYNC: the tile's spectra
+// copied in by cp.async and transformed in place.
+template <int NX, int WY, int T, int MINB = 0, bool ASYNC = false>
 static int add_x(XKernels* out, int n, const char* tag = "") {
   if (n >= kMaxVariants) return n;
   XKernels& k = out[n];
-  k.bulk = x_pass_kernel<NX, WY, T, MODE_BULK, PHYS, ASYNC, MINB>;
-  k.xj = x_pass_kernel<NX, WY, T, MODE_XJ, PHYS, ASYNC>;
+  k.bulk = x_pass_kernel<NX, WY, T, MODE_BULK, ASYNC, MINB>;
+  k.xj = x_pass_kernel<NX, WY, T, MODE_XJ, ASYNC>;
   k.imp = x_pass_kernel<NX, WY, T, MODE_IMPORT>;
-  k.exp = x_pass_kernel<NX, WY, T, MODE_EXPORT, PHYS, ASYNC>;
-  k.fields = x_pass_kernel<NX, WY, T, MODE_FIELDS, PHYS, ASYNC>;
+  k.exp = x_pass_kernel<NX, WY, T, MODE_EXPORT, ASYNC>;
+  k.fields = x_pass_kernel<NX, WY, T, MODE_FIELDS, ASYNC>;
   k.wy = WY;
   k.threads = T;
   k.tag = tag;

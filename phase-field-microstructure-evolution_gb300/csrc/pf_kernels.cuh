@@ -206,8 +206,17 @@ template <>
 struct XPlan<128> {
   static constexpr int N1 = 8, N2 = 16;
 };
+// A line of the x pass in shared memory: the runs follow one another without
+// pad slots, and an odd pitch of at least M + 1 (slot M takes kx = M while the
+// spectrum is in place).  The transforms' lanes go from line to line, so the
+// odd pitch alone keeps them free of bank conflicts; the bulk terms' lanes go
+// along a line, where a pad after each run put two of 16 slots in one bank
+// pair (a quarter of the pass's shared wavefronts at Nx = 128).
 template <int M>
-using XLine = Line<M, XPlan<M>::N1, XPlan<M>::N2>;
+struct XLine {
+  static constexpr int N1 = XPlan<M>::N1, N2 = XPlan<M>::N2;
+  static constexpr int PITCH = M % 2 == 0 ? M + 1 : M + 2;
+};
 
 // A twiddle of the x pass: from a copy of the table in shared memory (TWS),
 // else from the global table through the read-only path.
@@ -254,11 +263,11 @@ __device__ __forceinline__ void passA_rt(float2* buf, int NL, const float2* __re
     for (int k2 = 1; k2 < N2; ++k2) wt[k2] = ldtw<TWS>(tw + n1 * k2);
     const int full = NL & ~31;
     for (int l = (w / N1) * 32 + lane; l < full; l += 32 * (NW / N1))
-      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + n1, [&](int k2) { return wt[k2]; });
+      passA_item<N1, N2, N1, INV>(buf + l * P + n1, [&](int k2) { return wt[k2]; });
     const int rem = NL - full;
     if ((int)threadIdx.x < rem * N1) {
       const int m1 = threadIdx.x / rem, l = full + (int)threadIdx.x - m1 * rem;
-      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + m1, [&](int k2) { return ldtw<TWS>(tw + m1 * k2); });
+      passA_item<N1, N2, N1, INV>(buf + l * P + m1, [&](int k2) { return ldtw<TWS>(tw + m1 * k2); });
     }
   } else {
     const int nlb = (NL + 31) >> 5;  // groups of 32 lines
@@ -267,7 +276,7 @@ __device__ __forceinline__ void passA_rt(float2* buf, int NL, const float2* __re
       const int lo = it & 31, rest = it >> 5;
       const int n1 = rest % N1, l = (rest / N1) * 32 + lo;
       if (l >= NL) continue;
-      passA_item<N1, N2, N1 + 1, INV>(buf + l * P + n1, [&](int k2) { return ldtw<TWS>(tw + n1 * k2); });
+      passA_item<N1, N2, N1, INV>(buf + l * P + n1, [&](int k2) { return ldtw<TWS>(tw + n1 * k2); });
     }
   }
 }
@@ -283,7 +292,7 @@ struct FastDiv {
 // Where element kx of a line's half spectrum is read from:
 //   SPEC_GLOBAL  src + kx * stride in read-only global memory;
 //   SPEC_INPLACE the line itself, kx at run kx % N2, element kx / N2 of the
-//                run (x_spec_slot), and kx = M in the pad slot after run 0.
+//                run (x_spec_slot), and kx = M in slot M.
 // In place, the inputs of a run pair are exactly the slots its outputs go
 // to, so every item reads its inputs into registers and overwrites them.
 enum SpecSrc { SPEC_GLOBAL = 0, SPEC_INPLACE = 1 };
@@ -291,13 +300,13 @@ enum SpecSrc { SPEC_GLOBAL = 0, SPEC_INPLACE = 1 };
 template <int M>
 __device__ __forceinline__ int x_spec_slot(int kx) {
   constexpr int N1 = XLine<M>::N1, N2 = XLine<M>::N2;
-  return kx == M ? N1 : (N1 + 1) * (kx % N2) + kx / N2;
+  return kx == M ? M : N1 * (kx % N2) + kx / N2;
 }
 
 // Element k1 of run r: kx = r + N2 k1, step = N2 strides of kx.
 template <int SRC, int M>
 __device__ __forceinline__ float2 ld_spec(const float2* src, int step, int r, int k1) {
-  if constexpr (SRC == SPEC_INPLACE) return src[(XLine<M>::N1 + 1) * r + k1];
+  if constexpr (SRC == SPEC_INPLACE) return src[XLine<M>::N1 * r + k1];
   else return __ldg(src + (ptrdiff_t)k1 * step);
 }
 
@@ -340,14 +349,14 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, int ks, float2* li
     dft_inv<N1>(zb);
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
-      line[n1 + (N1 + 1) * ra] = za[n1];
-      line[n1 + (N1 + 1) * rb] = zb[n1];
+      line[n1 + N1 * ra] = za[n1];
+      line[n1 + N1 * rb] = zb[n1];
     }
   } else if (pr == 0) {
     float2 a[N1];
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) a[k1] = ld_spec<SRC, M>(src, step, 0, k1);
-    const float2 xM = ld_spec<SRC, M>(src, step, 0, N1);  // kx = M
+    const float2 xM = SRC == SPEC_INPLACE ? src[M] : ld_spec<SRC, M>(src, step, 0, N1);
     float2 z[N1];
     z[0] = make_float2(a[0].x + xM.x, a[0].x - xM.x);
 #pragma unroll
@@ -375,7 +384,7 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, int ks, float2* li
     }
     dft_inv<N1>(z);
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) line[n1 + (N1 + 1) * ra] = z[n1];
+    for (int n1 = 0; n1 < N1; ++n1) line[n1 + N1 * ra] = z[n1];
   }
 }
 
@@ -392,8 +401,8 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, con
     float2 za[N1], zb[N1];
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
-      za[n1] = line[n1 + (N1 + 1) * ra];
-      zb[n1] = line[n1 + (N1 + 1) * rb];
+      za[n1] = line[n1 + N1 * ra];
+      zb[n1] = line[n1 + N1 * rb];
     }
     Dft<N1>::fwd(za);
     Dft<N1>::fwd(zb);
@@ -426,7 +435,7 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, con
     float2* da = dst + ra * ks;
     float2 z[N1];
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) z[n1] = line[n1 + (N1 + 1) * ra];
+    for (int n1 = 0; n1 < N1; ++n1) z[n1] = line[n1 + N1 * ra];
     Dft<N1>::fwd(z);
 #pragma unroll
     for (int k1 = 0; k1 < N1 / 2; ++k1) {
@@ -647,38 +656,18 @@ __device__ __forceinline__ void store_block_diag(const BulkAcc& acc, const RunPa
 }
 
 // Bulk terms of one tile (WY rows of every field in shared memory), one
-// float2 slot (two cells) per item.  Consecutive lanes take consecutive
-// physical slots of the padded lines and the pad slots stay idle, so that the
-// 16 slots of a half warp always fall in distinct bank pairs (a walk over the
-// logical cells would span 17 slots and put its first and last in one pair).
-template <int NX, int WY, int T, bool PHYS = true>
+// float2 slot (two cells) per item.
+template <int NX, int WY, int T>
 __device__ __forceinline__ void bulk_tile(float2* smem, const RunParams& rp, const Shape& sh, int z, int y0,
                                           BulkAcc& acc) {
-  constexpr int M = NX / 2;
-  using LM = XLine<M>;
-  constexpr int PM = LM::PITCH, N1 = LM::N1;
-  if constexpr (!PHYS) {  // walk over the logical cells (a half warp spans N1 + 1 slots per N1 cells)
-    for (int it = threadIdx.x; it < WY * M; it += T) {
-      const int m = it % M, yy = it / M;
-      const int slot = LM::phys(m);
-      float2 dfdc, mob;
-      bulk_slot<PM, WY>(smem, yy, slot, rp, dfdc, mob, acc);
-      smem[(rp.V * WY + yy) * PM + slot] = dfdc;
-      if (rp.mobility != MOB_CONST)
-        *reinterpret_cast<float2*>(rp.mob + ((size_t)z * sh.Ny + y0 + yy) * NX + 2 * m) = mob;
-    }
-  } else {
-    for (int it = threadIdx.x; it < WY * PM; it += T) {
-      const int yy = it / PM, ps = it - yy * PM;
-      const int q = ps / (N1 + 1), r = ps - q * (N1 + 1);
-      if (r == N1 || ps >= LM::RAW) continue;  // pad slot
-      const int m = q * N1 + r;
-      float2 dfdc, mob;
-      bulk_slot<PM, WY>(smem, yy, ps, rp, dfdc, mob, acc);
-      smem[(rp.V * WY + yy) * PM + ps] = dfdc;
-      if (rp.mobility != MOB_CONST)
-        *reinterpret_cast<float2*>(rp.mob + ((size_t)z * sh.Ny + y0 + yy) * NX + 2 * m) = mob;
-    }
+  constexpr int M = NX / 2, PM = XLine<M>::PITCH;
+  for (int it = threadIdx.x; it < WY * M; it += T) {
+    const int m = it % M, yy = it / M;
+    float2 dfdc, mob;
+    bulk_slot<PM, WY>(smem, yy, m, rp, dfdc, mob, acc);
+    smem[(rp.V * WY + yy) * PM + m] = dfdc;
+    if (rp.mobility != MOB_CONST)
+      *reinterpret_cast<float2*>(rp.mob + ((size_t)z * sh.Ny + y0 + yy) * NX + 2 * m) = mob;
   }
 }
 
@@ -700,7 +689,7 @@ __device__ __forceinline__ void walk_tile(float2* smem, double* aos, int V, size
   float* lines = reinterpret_cast<float*>(smem);
   const auto place = [&](int f, int cell) {
     const int yy = cell / NX, x = cell % NX;
-    return lines + 2 * ((f * WY + yy) * LM::PITCH + LM::phys(x >> 1)) + (x & 1);
+    return lines + 2 * ((f * WY + yy) * LM::PITCH + (x >> 1)) + (x & 1);
   };
   const FastDiv by_v(V);
   double* phi = aos + cell0 * V;
@@ -724,7 +713,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // (all of them in flight at once, no registers held) in the in-place slot
 // order, and the inverse transform then runs in place; otherwise each item
 // loads its own inputs from global memory.
-template <int NX, int WY, int T, int MODE, bool PHYS = true, bool ASYNC = false, int MINB = 0>
+template <int NX, int WY, int T, int MODE, bool ASYNC = false, int MINB = 0>
 __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __restrict__ runs, const Shape sh) {
   constexpr int M = NX / 2;
   using LM = XLine<M>;
@@ -802,7 +791,7 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
     for (int it = threadIdx.x; it < nF * WY * M; it += T) {
       const int m = it % M, r = it / M, yy = r % WY, f = r / WY;
       *reinterpret_cast<float2*>(rp.fin + (((size_t)f * sh.Nz + z) * sh.Ny + y0 + yy) * NX + 2 * m) =
-          smem[(f * WY + yy) * PM + LM::phys(m)];
+          smem[(f * WY + yy) * PM + m];
     }
     return;
   }
@@ -812,12 +801,12 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
 
   if (MODE == MODE_BULK) {
     // 2. bulk terms, two cells per slot
-    bulk_tile<NX, WY, T, PHYS>(smem, rp, sh, z, y0, acc);
+    bulk_tile<NX, WY, T>(smem, rp, sh, z, y0, acc);
     __syncthreads();
   } else if (MODE == MODE_XJ) {
     for (int it = threadIdx.x; it < WY * M; it += T) {
       const int m = it % M, yy = it / M;
-      const int slot = LM::phys(m);
+      const int slot = m;
       const float2 mb = *reinterpret_cast<const float2*>(rp.mob + ((size_t)z * sh.Ny + y0 + yy) * NX + 2 * m);
       float2 v = smem[yy * PM + slot];
       v.x *= mb.x;

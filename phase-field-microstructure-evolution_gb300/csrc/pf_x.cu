@@ -11,8 +11,9 @@ int x_variants_a(int nx, XKernels* out, int n) {
     case 16: n = add_x<16, 16, 256>(out, n); break;
     case 32: n = add_x<32, 4, 128>(out, n); n = add_x<32, 8, 256>(out, n); break;
     case 64:
-      n = add_x<64, 16, 256, 3, false>(out, n, ",logical,3/SM");
+      n = add_x<64, 16, 256, 3>(out, n, ",3/SM");
       n = add_x<64, 8, 256>(out, n);
+      n = add_x<64, 16, 256, 4>(out, n, ",4/SM");
       n = add_x<64, 4, 128>(out, n);
       break;
     case 96:
@@ -22,10 +23,10 @@ int x_variants_a(int nx, XKernels* out, int n) {
       n = add_x<96, 4, 256>(out, n);
       break;
     case 128:
-      n = add_x<128, 8, 256, 0, false>(out, n, ",logical");
-      n = add_x<128, 8, 256, 3, false>(out, n, ",logical,3/SM");
+      n = add_x<128, 8, 256, 0>(out, n);
+      n = add_x<128, 8, 256, 3>(out, n, ",3/SM");
       n = add_x<128, 32, 256>(out, n);
-      n = add_x<128, 4, 256, 0, false, true>(out, n, ",async,logical");
+      n = add_x<128, 4, 256, 0, true>(out, n, ",async");
       break;
     case 256:
       // as many rows as fit: a warp's access covers WY x 8 bytes of each field and kx (256^3, x pass,
@@ -33,8 +34,8 @@ int x_variants_a(int nx, XKernels* out, int n) {
       n = add_x<256, 8, 256>(out, n);
       n = add_x<256, 16, 512>(out, n);
       n = add_x<256, 8, 512>(out, n);
-      n = add_x<256, 4, 512, 0, false, true>(out, n, ",async,logical");
-      n = add_x<256, 2, 256, 0, false, true>(out, n, ",async,logical");
+      n = add_x<256, 4, 512, 0, true>(out, n, ",async");
+      n = add_x<256, 2, 256, 0, true>(out, n, ",async");
       n = add_x<256, 1, 256>(out, n);  // one row per tile: up to 196 fields
       break;
     default: break;

@@ -21,13 +21,14 @@ int x_variants_r5(int nx, XKernels* out, int n) {
       n = add_x<160, 4, 256>(out, n);
       break;
     case 200:
-      n = add_x<200, 8, 256, 3, false>(out, n, ",logical,3/SM");
+      n = add_x<200, 8, 256, 3>(out, n, ",3/SM");
       n = add_x<200, 8, 512>(out, n);
       n = add_x<200, 4, 256>(out, n);
       n = add_x<200, 2, 256>(out, n);
       break;
     case 102:
-      n = add_x<102, 6, 256, 3, false>(out, n, ",logical,3/SM");
+      n = add_x<102, 17, 256, 2>(out, n, ",2/SM");
+      n = add_x<102, 6, 256, 3>(out, n, ",3/SM");
       n = add_x<102, 3, 256>(out, n);
       n = add_x<102, 2, 256>(out, n);
       break;
