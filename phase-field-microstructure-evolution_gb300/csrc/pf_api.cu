@@ -122,6 +122,8 @@ static int build_tables(int Nx, int Ny, int Nz, int nF, DevTables& t) {
   s.plane0 = 0;
   mixed_strides(Nx, Ny, Nz, nF, s.ks, s.zs);
   s.par = 0;
+  s.io_phi = s.io_con = nullptr;
+  s.fin = nullptr;
   s.twM = (const float2*)(b + off_tw[0]);
   s.twN = (const float2*)(b + off_tw[1]);
   s.twY = (const float2*)(b + off_tw[2]);
@@ -215,8 +217,9 @@ struct pf_batch {
   std::vector<RunParams> hrp;
   RunParams* drp = nullptr;
   void* mem = nullptr;         // all per-run buffers
-  float* fin = nullptr;        // float staging [nF][Nz][Ny][Nx]
-  double* dstage = nullptr;    // one run's fields in the caller's layout
+  float* fin = nullptr;        // float fields [nF][Nz][Ny][Nx] for the analysis (made on first use)
+  double* dstage = nullptr;    // one run's fields in the caller's layout, for memory the GPU does not reach (made on first use)
+  bool coherent = false;       // the GPU reads and writes the host's pages through their own page tables
   int ring = 0;
   cudaStream_t stream = nullptr;
   cudaGraphExec_t gexec = nullptr;   // one step
@@ -227,7 +230,8 @@ struct pf_batch {
   cudaStream_t rec = nullptr;         // the step records of the multi-step graph
   cudaEvent_t ev_yz = nullptr, ev_rec[2] = {nullptr, nullptr};
   int prio_hi = 0;                    // greatest stream priority of the device
-  std::vector<double> hdiag;
+  std::vector<double> hdiag;   // records of one chunk of steps
+  size_t diag_bytes = 0;       // of one run's ring; the rings follow one another
   std::vector<int> steps_done;
   std::string variant;  // chosen kernel variants, for reports
 };
@@ -520,6 +524,40 @@ static int env_int(const char* name, int dflt) {
   return v ? atoi(v) : dflt;
 }
 
+// The launch shape `sh` with the fields in the batch's staging buffer.
+static int stage(pf_batch* b, const Shape& sh, Shape& out) {
+  const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
+  if (!b->dstage) {
+    const cudaError_t e = cudaMalloc(&b->dstage, b->nF * ncell * sizeof(double));
+    if (e != cudaSuccess) {
+      b->dstage = nullptr;
+      cudaGetLastError();
+      return fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e));
+    }
+  }
+  out = sh;
+  out.io_phi = b->dstage;
+  out.io_con = b->dstage + (size_t)b->V * ncell;
+  return PF_OK;
+}
+
+// Whether kernels may read (write) `bytes` of the caller's memory themselves.
+// Reading: any host memory, on a machine whose GPU walks the host's page
+// tables.  Writing: only pinned memory, since pages that have never been
+// touched would fault one by one.  Device memory keeps the copies' answer.
+static bool direct(const pf_batch* b, const void* p, size_t bytes, bool write) {
+  if (!b->coherent || (uintptr_t)p % sizeof(double) != 0) return false;
+  for (const char* q : {(const char*)p, (const char*)p + bytes - 1}) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type != cudaMemoryTypeHost && (write || a.type != cudaMemoryTypeUnregistered)) return false;
+  }
+  return true;
+}
+
 static int tune_batch(pf_batch* b) {
   XKernels xv[kMaxVariants];
   YZKernels yv[kMaxVariants];
@@ -547,10 +585,13 @@ static int tune_batch(pf_batch* b) {
     } else if (env_int("PFGPU_AUTOTUNE", 1) != 0 && (xs.size() > 1 || ys.size() > 1)) {
       // synthetic non-zero state so that the bulk terms take their usual branches
       const size_t nfin = (size_t)b->nF * b->Nx * b->Ny * b->Nz;
+      Shape staged = {};
+      const int rs = stage(b, b->tab.sh, staged);
+      if (rs) return rs;
       fill_kernel<<<(unsigned)((nfin + 255) / 256), 256, 0, b->stream>>>(b->dstage, nfin, 0.3, 0.7);
       apply_variants(b, xv[xs[0]], yv[ys[0]]);
       const dim3 g1(b->Nz * (b->Ny / b->xk.wy), 1);
-      b->xk.imp<<<g1, b->xk.threads, b->smem_x, b->stream>>>(b->drp, b->tab.sh);
+      b->xk.imp<<<g1, b->xk.threads, b->smem_x, b->stream>>>(b->drp, staged);
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
@@ -755,16 +796,17 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
   const size_t szPyz = align((size_t)32 * b->nF * b->Kx * sizeof(double));  // 2 parities x 2 x clusters <= 16
   const size_t szDiag = align((size_t)b->ring * DR_COUNT * sizeof(double));
   const size_t szCnt = 256;  // step counter
-  const size_t per_run = 3 * szS + szMob + szJ + szPx + szPyz + szDiag + szCnt;
-  e = cudaMalloc(&b->mem, per_run * nruns);
+  const size_t per_run = 3 * szS + szMob + szJ + szPx + szPyz + szCnt;
+  const size_t total = (per_run + szDiag) * nruns;  // the record rings follow the runs
+  b->diag_bytes = szDiag;
+  e = cudaMalloc(&b->mem, total);
   if (e != cudaSuccess)
-    return bail(fail(PF_ENOMEM, "cudaMalloc(%zu bytes) for %d runs: %s", per_run * nruns, nruns, cudaGetErrorString(e)));
-  e = cudaMemset(b->mem, 0, per_run * nruns);
+    return bail(fail(PF_ENOMEM, "cudaMalloc(%zu bytes) for %d runs: %s", total, nruns, cudaGetErrorString(e)));
+  e = cudaMemset(b->mem, 0, total);
   if (e != cudaSuccess) return bail(fail(PF_ECUDA, "cudaMemset: %s", cudaGetErrorString(e)));
-  e = cudaMalloc(&b->fin, b->nF * ncell * sizeof(float));
-  if (e != cudaSuccess) return bail(fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e)));
-  e = cudaMalloc(&b->dstage, b->nF * ncell * sizeof(double));
-  if (e != cudaSuccess) return bail(fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e)));
+  int coherent = 0;
+  cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, b->device);
+  b->coherent = coherent != 0;
   b->hrp.resize(nruns);
   b->steps_done.assign(nruns, 0);
   for (int i = 0; i < nruns; ++i) {
@@ -779,10 +821,8 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     r.J = var ? (float2*)p : nullptr; p += szJ;
     r.part_x = (float*)p; p += szPx;
     r.part_yz = (float*)p; p += szPyz;
-    r.diag = (double*)p; p += szDiag;
+    r.diag = (double*)((char*)b->mem + per_run * nruns + szDiag * i);
     r.counter = (int*)p;
-    r.fin = b->fin;
-    r.aos = b->dstage;
     r.L = (float)c.mob_phi;
     r.kappa_phi = (float)c.grad_coeff_phi;
     r.kappa_c = (float)c.grad_coeff_c;
@@ -831,12 +871,19 @@ static int batch_set_fields(pf_batch* b, int run, const double* phi, const doubl
   if (!b || run < 0 || run >= b->nruns || !phi || !con) return fail(PF_EINVAL, "bad arguments to set_fields");
   PF_CUDA(cudaSetDevice(b->device));
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
-  double* dphi = b->dstage;
-  double* dcon = b->dstage + (size_t)b->V * ncell;
-  PF_CUDA(cudaMemcpyAsync(dphi, phi, (size_t)b->V * ncell * sizeof(double), cudaMemcpyHostToDevice, b->stream));
-  PF_CUDA(cudaMemcpyAsync(dcon, con, ncell * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+  const size_t bphi = (size_t)b->V * ncell * sizeof(double), bcon = ncell * sizeof(double);
+  Shape sh = b->tab.sh;
+  if (direct(b, phi, bphi, false) && direct(b, con, bcon, false)) {
+    sh.io_phi = const_cast<double*>(phi);
+    sh.io_con = const_cast<double*>(con);
+  } else {
+    const int rs = stage(b, b->tab.sh, sh);
+    if (rs) return rs;
+    PF_CUDA(cudaMemcpyAsync(sh.io_phi, phi, bphi, cudaMemcpyHostToDevice, b->stream));
+    PF_CUDA(cudaMemcpyAsync(sh.io_con, con, bcon, cudaMemcpyHostToDevice, b->stream));
+  }
   const dim3 gx(b->Nz * (b->Ny / b->xk.wy), 1);
-  b->xk.imp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, b->tab.sh);
+  b->xk.imp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, sh);
   int rc = launch_yz(b, b->yk.imp, b->nF * b->Kx, b->drp + run, 1, b->stream);
   if (rc) return rc;
   PF_CUDA(cudaMemsetAsync(b->hrp[run].counter, 0, 256, b->stream));  // step counter
@@ -850,13 +897,23 @@ static int batch_get_fields(pf_batch* b, int run, double* phi, double* con) {
   if (!b || run < 0 || run >= b->nruns || !phi || !con) return fail(PF_EINVAL, "bad arguments to get_fields");
   PF_CUDA(cudaSetDevice(b->device));
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
-  double* dphi = b->dstage;
-  double* dcon = b->dstage + (size_t)b->V * ncell;
+  const size_t bphi = (size_t)b->V * ncell * sizeof(double), bcon = ncell * sizeof(double);
+  Shape sh = b->tab.sh;
+  const bool own = direct(b, phi, bphi, true) && direct(b, con, bcon, true);
+  if (own) {
+    sh.io_phi = phi;
+    sh.io_con = con;
+  } else {
+    const int rs = stage(b, b->tab.sh, sh);
+    if (rs) return rs;
+  }
   const dim3 gx(b->Nz * (b->Ny / b->xk.wy), 1);
-  b->xk.exp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, b->tab.sh);
+  b->xk.exp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, sh);
   PF_CUDA(cudaGetLastError());
-  PF_CUDA(cudaMemcpyAsync(phi, dphi, (size_t)b->V * ncell * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-  PF_CUDA(cudaMemcpyAsync(con, dcon, ncell * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
+  if (!own) {
+    PF_CUDA(cudaMemcpyAsync(phi, sh.io_phi, bphi, cudaMemcpyDeviceToHost, b->stream));
+    PF_CUDA(cudaMemcpyAsync(con, sh.io_con, bcon, cudaMemcpyDeviceToHost, b->stream));
+  }
   PF_CUDA(cudaStreamSynchronize(b->stream));
   return PF_OK;
 }
@@ -866,7 +923,17 @@ static int batch_device_fields(pf_batch* b, DeviceFields* out) {
   PF_CUDA(cudaSetDevice(b->device));
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
   const dim3 gx(b->Nz * (b->Ny / b->xk.wy), 1);
-  b->xk.fields<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp, b->tab.sh);
+  if (!b->fin) {
+    const cudaError_t e = cudaMalloc(&b->fin, b->nF * ncell * sizeof(float));
+    if (e != cudaSuccess) {
+      b->fin = nullptr;
+      cudaGetLastError();
+      return fail(PF_ENOMEM, "float fields: %s", cudaGetErrorString(e));
+    }
+  }
+  Shape sh = b->tab.sh;
+  sh.fin = b->fin;
+  b->xk.fields<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp, sh);
   PF_CUDA(cudaGetLastError());
   out->phi = b->fin;
   out->con = b->fin + (size_t)b->V * ncell;
@@ -901,20 +968,29 @@ static int batch_step(pf_batch* b, int nsteps, pf_diag* diag) {
     const int chunk = std::min(nsteps - done, b->ring);
     const int rl = launch_steps(b, chunk);
     if (rl) return rl;
+    // This chunk's records, [run][step]: at most two pieces of a ring (when
+    // they wrap around), of all runs at once where they stand alike -- one copy
+    // of 64 runs' records instead of 64 (a lone run's copy is quicker alone)
     PF_CUDA(cudaStreamSynchronize(b->stream));
-    b->hdiag.resize((size_t)b->ring * DR_COUNT);
-    for (int r = 0; r < b->nruns; ++r) {
-      // copy only this chunk's records (two pieces when they wrap around the ring)
+    b->hdiag.resize((size_t)b->nruns * chunk * DR_COUNT);
+    const size_t rec = DR_COUNT * sizeof(double);
+    bool together = b->nruns > 1 && b->diag_bytes < ((size_t)1 << 31);
+    for (int r = 1; r < b->nruns; ++r) together = together && b->steps_done[r] % b->ring == b->steps_done[0] % b->ring;
+    for (int r = 0; r < (together ? 1 : b->nruns); ++r) {
       const int first = b->steps_done[r] % b->ring;
       const int n1 = std::min(chunk, b->ring - first);
-      PF_CUDA(cudaMemcpy(b->hdiag.data() + (size_t)first * DR_COUNT, b->hrp[r].diag + (size_t)first * DR_COUNT,
-                         (size_t)n1 * DR_COUNT * sizeof(double), cudaMemcpyDeviceToHost));
-      if (chunk > n1)
-        PF_CUDA(cudaMemcpy(b->hdiag.data(), b->hrp[r].diag, (size_t)(chunk - n1) * DR_COUNT * sizeof(double),
-                           cudaMemcpyDeviceToHost));
+      double* h = b->hdiag.data() + (size_t)r * chunk * DR_COUNT;
+      const char* d = (const char*)b->hrp[r].diag;
+      const auto copy = [&](double* to, const char* from, size_t bytes) {
+        return together ? cudaMemcpy2D(to, chunk * rec, from, b->diag_bytes, bytes, b->nruns, cudaMemcpyDeviceToHost)
+                        : cudaMemcpy(to, from, bytes, cudaMemcpyDeviceToHost);
+      };
+      PF_CUDA(copy(h, d + first * rec, n1 * rec));
+      if (chunk > n1) PF_CUDA(copy(h + (size_t)n1 * DR_COUNT, d, (chunk - n1) * rec));
+    }
+    for (int r = 0; r < b->nruns; ++r) {
       for (int s = 0; s < chunk; ++s) {
-        const int step = b->steps_done[r] + s;  // 0-based
-        const double* d = b->hdiag.data() + (size_t)(step % b->ring) * DR_COUNT;
+        const double* d = b->hdiag.data() + ((size_t)r * chunk + s) * DR_COUNT;
         if (d[DR_NONFINITE] != 0) bad = 1;
         if (diag) fill_diag(d, &diag[(size_t)r * nsteps + done + s]);
       }

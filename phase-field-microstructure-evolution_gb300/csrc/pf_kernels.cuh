@@ -66,8 +66,6 @@ struct RunParams {
   float* part_yz;  // [2][2][nblk_yz]: per step parity, hi and lo of each yz CTA's weighted f_int sum
   double* diag;    // [ring][DR_COUNT]
   int* counter;    // step counter (device)
-  float* fin;      // [nF][Nz][Ny][Nx] float fields (MODE_FIELDS)
-  double* aos;     // fields in the caller's layout: phi(var, x, y, z), then con(x, y, z)
   float L, kappa_phi, kappa_c, dt, D_L, D_gb, sigma1, sigma2, am, ap, c0m, c0p;
   int mobility;
   int V;           // number of order parameters
@@ -89,6 +87,10 @@ struct Shape {
   int nblk_yz;  // blocks of the yz pass per run
   int plane0;   // first (field, kx) plane of a yz-pass launch (a launch may cover a subset)
   int ks, zs;   // strides of kx and z in Sm, D and J (y contiguous; see mixed_strides)
+  // fields of one run for the import and export modes: the caller's layout,
+  // phi(var, x, y, z) and con(x, y, z), and float [nF][Nz][Ny][Nx] (MODE_FIELDS)
+  double *io_phi, *io_con;
+  float* fin;
   int par;  // parity of the step: which set of diagnostic partials its passes write and its record reads
 };
 
@@ -677,14 +679,16 @@ __device__ __forceinline__ void bulk_tile(float2* smem, const RunParams& rp, con
 // (phi(var, x, y, z) and con, REAL*8) -> S.  MODE_EXPORT: S -> the caller's
 // fields.  MODE_FIELDS: S -> float fields [f][z][y][x].
 // A tile's rows are one contiguous piece of the caller's layout, so import and
-// export read and write it in full lines straight from and to shared memory.
+// export read and write it in full lines straight from and to shared memory --
+// in the host's own memory where the GPU reaches that at the link's full rate
+// (NVLink-C2C: kernels move 210 GB/s in and 193 out, as copies do).
 // ---------------------------------------------------------------------------
 enum XMode { MODE_BULK = 0, MODE_XJ = 1, MODE_IMPORT = 2, MODE_EXPORT = 3, MODE_FIELDS = 4 };
 
 // Walk over the cells of a tile in the caller's layout: op(value in memory,
 // its place in the tile's lines) for phi (field fastest), then con.
 template <int NX, int WY, int T, class Op>
-__device__ __forceinline__ void walk_tile(float2* smem, double* aos, int V, size_t ncell, size_t cell0, Op op) {
+__device__ __forceinline__ void walk_tile(float2* smem, const Shape& sh, int V, size_t cell0, Op op) {
   using LM = XLine<NX / 2>;
   float* lines = reinterpret_cast<float*>(smem);
   const auto place = [&](int f, int cell) {
@@ -692,13 +696,13 @@ __device__ __forceinline__ void walk_tile(float2* smem, double* aos, int V, size
     return lines + 2 * ((f * WY + yy) * LM::PITCH + (x >> 1)) + (x & 1);
   };
   const FastDiv by_v(V);
-  double* phi = aos + cell0 * V;
+  double* phi = sh.io_phi + cell0 * V;
 #pragma unroll 4
   for (int it = threadIdx.x; it < WY * NX * V; it += T) {
     const int cell = by_v(it);
     op(phi + it, place(it - cell * V, cell));
   }
-  double* con = aos + ncell * V + cell0;
+  double* con = sh.io_con + cell0;
   for (int it = threadIdx.x; it < WY * NX; it += T) op(con + it, place(V, it));
 }
 
@@ -749,7 +753,7 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
   const float2* __restrict__ src = (MODE == MODE_XJ) ? rp.J : rp.Sm;
 
   if (MODE == MODE_IMPORT) {
-    walk_tile<NX, WY, T>(smem, rp.aos, rp.V, (size_t)sh.Nz * sh.Ny * NX, (size_t)(z * sh.Ny + y0) * NX,
+    walk_tile<NX, WY, T>(smem, sh, rp.V, (size_t)(z * sh.Ny + y0) * NX,
                          [](const double* v, float* at) { *at = (float)*v; });
   } else {
     // 1. inverse x transform: global half spectrum -> pre-processing -> pass B'
@@ -783,14 +787,14 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
   __syncthreads();
 
   if (MODE == MODE_EXPORT) {
-    walk_tile<NX, WY, T>(smem, rp.aos, rp.V, (size_t)sh.Nz * sh.Ny * NX, (size_t)(z * sh.Ny + y0) * NX,
+    walk_tile<NX, WY, T>(smem, sh, rp.V, (size_t)(z * sh.Ny + y0) * NX,
                          [](double* v, const float* at) { *v = (double)*at; });
     return;
   }
   if (MODE == MODE_FIELDS) {
     for (int it = threadIdx.x; it < nF * WY * M; it += T) {
       const int m = it % M, r = it / M, yy = r % WY, f = r / WY;
-      *reinterpret_cast<float2*>(rp.fin + (((size_t)f * sh.Nz + z) * sh.Ny + y0 + yy) * NX + 2 * m) =
+      *reinterpret_cast<float2*>(sh.fin + (((size_t)f * sh.Nz + z) * sh.Ny + y0 + yy) * NX + 2 * m) =
           smem[(f * WY + yy) * PM + m];
     }
     return;
