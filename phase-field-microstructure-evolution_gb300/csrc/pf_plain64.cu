@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -569,27 +570,51 @@ int plain64_step(Plain64* p, int nsteps, pf_diag* diag) {
 // ---------------------------------------------------------------------------
 // Fortran shims
 // ---------------------------------------------------------------------------
-__global__ void p64_zyx_to_xyz(const cufftDoubleComplex* __restrict__ in, cufftDoubleComplex* __restrict__ out, int Kx,
-                               int Ny, int Nz, double scale) {
-  // in [z][y][kx] -> out [kx][y][z] (P3DFFT transposed order), scaled
-  const size_t n = (size_t)Kx * Ny * Nz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(i % Kx);
-    const size_t r = i / Kx;
-    const int y = (int)(r % Ny), z = (int)(r / Ny);
-    const cufftDoubleComplex v = in[i];
-    out[((size_t)kx * Ny + y) * Nz + z] = make_cuDoubleComplex(v.x * scale, v.y * scale);
+// out[b][y][a] = scale in[a][y][b]: between cuFFT's [z][y][kx] and P3DFFT's
+// transposed order [kx][y][z], 32 x 32 tiles through shared memory so that both
+// sides move in 512-byte pieces; `in` may be the caller's own memory.
+constexpr int kTile = 32, kTileRows = 8;
+__global__ void __launch_bounds__(kTile* kTileRows) p64_transpose(const cufftDoubleComplex* __restrict__ in,
+                                                                  cufftDoubleComplex* __restrict__ out, int nA, int Ny,
+                                                                  int nB, double scale) {
+  __shared__ cufftDoubleComplex tile[kTile][kTile + 1];
+  const int y = blockIdx.z, b0 = blockIdx.x * kTile, a0 = blockIdx.y * kTile;
+  for (int r = threadIdx.y; r < kTile; r += kTileRows) {
+    const int a = a0 + r, b = b0 + threadIdx.x;
+    if (a < nA && b < nB) tile[r][threadIdx.x] = in[((size_t)a * Ny + y) * nB + b];
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < kTile; r += kTileRows) {
+    const int b = b0 + r, a = a0 + threadIdx.x;
+    if (a < nA && b < nB) {
+      const cufftDoubleComplex v = tile[threadIdx.x][r];
+      out[((size_t)b * Ny + y) * nA + a] = make_cuDoubleComplex(v.x * scale, v.y * scale);
+    }
   }
 }
-__global__ void p64_xyz_to_zyx(const cufftDoubleComplex* __restrict__ in, cufftDoubleComplex* __restrict__ out, int Kx,
-                               int Ny, int Nz) {
-  const size_t n = (size_t)Kx * Ny * Nz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(i % Kx);
-    const size_t r = i / Kx;
-    const int y = (int)(r % Ny), z = (int)(r / Ny);
-    out[i] = in[((size_t)kx * Ny + y) * Nz + z];
+static int transpose(const cufftDoubleComplex* in, cufftDoubleComplex* out, int nA, int Ny, int nB, double scale) {
+  for (int y0 = 0; y0 < Ny; y0 += 65535) {  // the grid's z extent
+    const dim3 grid((nB + kTile - 1) / kTile, (nA + kTile - 1) / kTile, std::min(Ny - y0, 65535));
+    p64_transpose<<<grid, dim3(kTile, kTileRows)>>>(in + (size_t)y0 * nB, out + (size_t)y0 * nA, nA, Ny, nB, scale);
   }
+  P64_CUDA(cudaGetLastError());
+  return PF_OK;
+}
+
+// Whether the shims' kernels may read the caller's array where it is: host
+// memory, aligned as the transforms want it, on a GPU that walks the host's
+// page tables.  The first kernel then takes the place of a copy and runs while
+// the data arrives.
+static bool reads_host(const void* p, int device) {
+  int coherent = 0;
+  cudaPointerAttributes a;
+  if ((uintptr_t)p % 16 != 0 ||
+      cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) != cudaSuccess ||
+      !coherent || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
 }
 
 struct ShimCtx {
@@ -661,10 +686,13 @@ static int f_trans_impl(const double* in, double* out, int Nx, int Ny, int Nz, c
   int rc = shim_plans(Nx, Ny, Nz, &pl);
   if (rc) return rc;
   const size_t n = (size_t)Nx * Ny * Nz, ns = (size_t)(Nx / 2 + 1) * Ny * Nz;
-  P64_CUDA(cudaMemcpy(pl->real, in, n * sizeof(double), cudaMemcpyHostToDevice));
-  P64_FFT(cufftExecD2Z(pl->f, pl->real, pl->a));
-  p64_zyx_to_xyz<<<NB, NT>>>(pl->a, pl->b, Nx / 2 + 1, Ny, Nz, 1.0 / (double)n);
-  P64_CUDA(cudaGetLastError());
+  double* real = const_cast<double*>(in);  // a real-to-complex transform out of place leaves its input alone
+  if (!reads_host(in, S.device)) {
+    real = pl->real;
+    P64_CUDA(cudaMemcpy(real, in, n * sizeof(double), cudaMemcpyHostToDevice));
+  }
+  P64_FFT(cufftExecD2Z(pl->f, real, pl->a));
+  if ((rc = transpose(pl->a, pl->b, Nz, Ny, Nx / 2 + 1, 1.0 / (double)n))) return rc;
   P64_CUDA(cudaMemcpy(out, pl->b, ns * sizeof(cufftDoubleComplex), cudaMemcpyDeviceToHost));
   return PF_OK;
 }
@@ -686,9 +714,12 @@ static int inv_trans_impl(const double* in, double* out, const int* ist, const i
   int rc = shim_plans(Nx, Ny, Nz, &pl);
   if (rc) return rc;
   const size_t n = (size_t)Nx * Ny * Nz, ns = (size_t)(Nx / 2 + 1) * Ny * Nz;
-  P64_CUDA(cudaMemcpy(pl->b, in, ns * sizeof(cufftDoubleComplex), cudaMemcpyHostToDevice));
-  p64_xyz_to_zyx<<<NB, NT>>>(pl->b, pl->a, Nx / 2 + 1, Ny, Nz);
-  P64_CUDA(cudaGetLastError());
+  const cufftDoubleComplex* spec = reinterpret_cast<const cufftDoubleComplex*>(in);
+  if (!reads_host(in, S.device)) {
+    spec = pl->b;
+    P64_CUDA(cudaMemcpy(pl->b, in, ns * sizeof(cufftDoubleComplex), cudaMemcpyHostToDevice));
+  }
+  if ((rc = transpose(spec, pl->a, Nx / 2 + 1, Ny, Nz, 1.0))) return rc;
   P64_FFT(cufftExecZ2D(pl->i, pl->a, pl->real));
   P64_CUDA(cudaMemcpy(out, pl->real, n * sizeof(double), cudaMemcpyDeviceToHost));
   return PF_OK;
