@@ -160,6 +160,7 @@ static size_t x_smem(int nx, int nF, int wy, bool limit = false) {
 }
 
 static const size_t kMaxSmem = 227 * 1024;
+static const size_t kHostRings = (size_t)8 << 20;  // pinned memory a batch may keep for its records (102 runs)
 
 // Static shared memory of the one-CTA x-pass kernels beside the dynamic line
 // buffer: the twiddle tables (Nx + Nx/2 float2, from Nx = 96 up) and the
@@ -230,8 +231,9 @@ struct pf_batch {
   cudaStream_t rec = nullptr;         // the step records of the multi-step graph
   cudaEvent_t ev_yz = nullptr, ev_rec[2] = {nullptr, nullptr};
   int prio_hi = 0;                    // greatest stream priority of the device
-  std::vector<double> hdiag;   // records of one chunk of steps
+  std::vector<double> hdiag;   // records of one chunk of steps, copied (more runs)
   size_t diag_bytes = 0;       // of one run's ring; the rings follow one another
+  double* hring = nullptr;     // the rings in pinned host memory, written by the record kernel (up to kHostRings bytes)
   std::vector<int> steps_done;
   std::string variant;  // chosen kernel variants, for reports
 };
@@ -705,6 +707,7 @@ static void destroy_batch(pf_batch* b) {
   if (b->ev_c) cudaEventDestroy(b->ev_c);
   cudaFree(b->drp);
   cudaFree(b->mem);
+  cudaFreeHost(b->hring);
   cudaFree(b->fin);
   cudaFree(b->dstage);
   cudaFree(b->tab.base);
@@ -804,6 +807,10 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     return bail(fail(PF_ENOMEM, "cudaMalloc(%zu bytes) for %d runs: %s", total, nruns, cudaGetErrorString(e)));
   e = cudaMemset(b->mem, 0, total);
   if (e != cudaSuccess) return bail(fail(PF_ECUDA, "cudaMemset: %s", cudaGetErrorString(e)));
+  if (szDiag * nruns <= kHostRings && cudaMallocHost(&b->hring, szDiag * nruns) != cudaSuccess) {
+    b->hring = nullptr;
+    cudaGetLastError();
+  }
   int coherent = 0;
   cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, b->device);
   b->coherent = coherent != 0;
@@ -822,6 +829,7 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     r.part_x = (float*)p; p += szPx;
     r.part_yz = (float*)p; p += szPyz;
     r.diag = (double*)((char*)b->mem + per_run * nruns + szDiag * i);
+    r.hdiag = b->hring ? (double*)((char*)b->hring + szDiag * i) : nullptr;
     r.counter = (int*)p;
     r.L = (float)c.mob_phi;
     r.kappa_phi = (float)c.grad_coeff_phi;
@@ -959,6 +967,28 @@ static void fill_diag(const double* d, pf_diag* o) {
   o->mass = d[DR_MASS];
 }
 
+// The records of the last `chunk` steps into b->hdiag, [run][step]: at most two
+// pieces of a ring (when they wrap around), of all runs at once where they
+// stand alike.
+static int copy_records(pf_batch* b, int chunk) {
+  b->hdiag.resize((size_t)b->nruns * chunk * DR_COUNT);
+  const size_t rec = DR_COUNT * sizeof(double);
+  bool together = b->diag_bytes < ((size_t)1 << 31);
+  for (int r = 1; r < b->nruns; ++r) together = together && b->steps_done[r] % b->ring == b->steps_done[0] % b->ring;
+  for (int r = 0; r < (together ? 1 : b->nruns); ++r) {
+    const int rows = together ? b->nruns : 1;
+    const int first = b->steps_done[r] % b->ring;
+    const int n1 = std::min(chunk, b->ring - first);
+    double* h = b->hdiag.data() + (size_t)r * chunk * DR_COUNT;
+    const char* d = (const char*)b->hrp[r].diag;
+    PF_CUDA(cudaMemcpy2D(h, chunk * rec, d + first * rec, b->diag_bytes, n1 * rec, rows, cudaMemcpyDeviceToHost));
+    if (chunk > n1)
+      PF_CUDA(cudaMemcpy2D(h + (size_t)n1 * DR_COUNT, chunk * rec, d, b->diag_bytes, (chunk - n1) * rec, rows,
+                           cudaMemcpyDeviceToHost));
+  }
+  return PF_OK;
+}
+
 static int batch_step(pf_batch* b, int nsteps, pf_diag* diag) {
   if (!b || nsteps < 0) return fail(PF_EINVAL, "bad arguments to step");
   PF_CUDA(cudaSetDevice(b->device));
@@ -968,29 +998,16 @@ static int batch_step(pf_batch* b, int nsteps, pf_diag* diag) {
     const int chunk = std::min(nsteps - done, b->ring);
     const int rl = launch_steps(b, chunk);
     if (rl) return rl;
-    // This chunk's records, [run][step]: at most two pieces of a ring (when
-    // they wrap around), of all runs at once where they stand alike -- one copy
-    // of 64 runs' records instead of 64 (a lone run's copy is quicker alone)
     PF_CUDA(cudaStreamSynchronize(b->stream));
-    b->hdiag.resize((size_t)b->nruns * chunk * DR_COUNT);
-    const size_t rec = DR_COUNT * sizeof(double);
-    bool together = b->nruns > 1 && b->diag_bytes < ((size_t)1 << 31);
-    for (int r = 1; r < b->nruns; ++r) together = together && b->steps_done[r] % b->ring == b->steps_done[0] % b->ring;
-    for (int r = 0; r < (together ? 1 : b->nruns); ++r) {
-      const int first = b->steps_done[r] % b->ring;
-      const int n1 = std::min(chunk, b->ring - first);
-      double* h = b->hdiag.data() + (size_t)r * chunk * DR_COUNT;
-      const char* d = (const char*)b->hrp[r].diag;
-      const auto copy = [&](double* to, const char* from, size_t bytes) {
-        return together ? cudaMemcpy2D(to, chunk * rec, from, b->diag_bytes, bytes, b->nruns, cudaMemcpyDeviceToHost)
-                        : cudaMemcpy(to, from, bytes, cudaMemcpyDeviceToHost);
-      };
-      PF_CUDA(copy(h, d + first * rec, n1 * rec));
-      if (chunk > n1) PF_CUDA(copy(h + (size_t)n1 * DR_COUNT, d, (chunk - n1) * rec));
+    if (!b->hring) {
+      const int rc = copy_records(b, chunk);
+      if (rc) return rc;
     }
     for (int r = 0; r < b->nruns; ++r) {
+      const double* ring = b->hring ? (const double*)((const char*)b->hring + b->diag_bytes * r) : nullptr;
       for (int s = 0; s < chunk; ++s) {
-        const double* d = b->hdiag.data() + ((size_t)r * chunk + s) * DR_COUNT;
+        const double* d = ring ? ring + (size_t)((b->steps_done[r] + s) % b->ring) * DR_COUNT
+                               : b->hdiag.data() + ((size_t)r * chunk + s) * DR_COUNT;
         if (d[DR_NONFINITE] != 0) bad = 1;
         if (diag) fill_diag(d, &diag[(size_t)r * nsteps + done + s]);
       }

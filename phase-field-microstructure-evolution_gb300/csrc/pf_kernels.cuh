@@ -65,6 +65,7 @@ struct RunParams {
   float* part_x;   // [2][XQ_COUNT][nblk_x]: per step parity
   float* part_yz;  // [2][2][nblk_yz]: per step parity, hi and lo of each yz CTA's weighted f_int sum
   double* diag;    // [ring][DR_COUNT]
+  double* hdiag;   // the same in pinned host memory (few runs), else null
   int* counter;    // step counter (device)
   float L, kappa_phi, kappa_c, dt, D_L, D_gb, sigma1, sigma2, am, ap, c0m, c0p;
   int mobility;
@@ -1073,18 +1074,24 @@ __global__ void __launch_bounds__(T) record_kernel(const RunParams* __restrict__
     const int nbad = __reduce_add_sync(0xffffffffu, in ? si[lane] : 0);
     if (lane == 0) {
       const int step = *rp.counter;
-      double* d = rp.diag + (size_t)(step % rp.ring) * DR_COUNT;
       const double n3 = (double)sh.Nx * sh.Ny * sh.Nz;
-      d[DR_STEP] = step + 1;
-      d[DR_FINT] = 0.5 * n3 * ((double)rp.kappa_phi * a.value() + (double)rp.kappa_c * b.value());
-      d[DR_FETA] = e.value();
-      d[DR_FCH] = c.value();
-      d[DR_CMIN] = m0;
-      d[DR_CMAX] = m1;
-      d[DR_PHIMIN] = m2;
-      d[DR_PHIPMAX] = m3;
-      d[DR_MASS] = m.value();
-      d[DR_NONFINITE] = nbad;
+      const double fint = 0.5 * n3 * ((double)rp.kappa_phi * a.value() + (double)rp.kappa_c * b.value());
+      const double mass = m.value();
+      // to the host as well where it keeps a ring: pf_step then needs no copy
+      for (double* ring : {rp.diag, rp.hdiag}) {
+        if (!ring) break;
+        double* d = ring + (size_t)(step % rp.ring) * DR_COUNT;
+        d[DR_STEP] = step + 1;
+        d[DR_FINT] = fint;
+        d[DR_FETA] = e.value();
+        d[DR_FCH] = c.value();
+        d[DR_CMIN] = m0;
+        d[DR_CMAX] = m1;
+        d[DR_PHIMIN] = m2;
+        d[DR_PHIPMAX] = m3;
+        d[DR_MASS] = mass;
+        d[DR_NONFINITE] = nbad;
+      }
       *rp.counter = step + 1;
     }
   }
