@@ -252,24 +252,26 @@ __device__ __forceinline__ void passA_item(float2* p, const Tw& w) {
 
 // pass A over a runtime number of lines (pitch P, T threads).  A warp takes 32
 // consecutive lines at one column n1: with an odd pitch those 32 accesses hit
-// distinct bank pairs.  Where the CTA's warps are a multiple of N1, a warp
-// keeps one column and loads its twiddles once; the lines beyond the last
+// distinct bank pairs.  Where the CTA's warps are a multiple of N1 or divide
+// it, a warp loads a column's twiddles once for all its lines; the lines beyond the last
 // whole 32 are spread over (line, column), so that they cost rem N1 / 32
 // warp items instead of N1 (17 fields x 8 rows: 136 lines, 34 items, not 40).
 template <int L, int P, int T, bool INV, bool TWS = false>
 __device__ __forceinline__ void passA_rt(float2* buf, int NL, const float2* __restrict__ tw) {
   constexpr int N1 = XLine<L>::N1, N2 = XLine<L>::N2, NW = T / 32;
-  if constexpr (NW % N1 == 0) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n1 = w % N1;
-    float2 wt[N2];
-#pragma unroll
-    for (int k2 = 1; k2 < N2; ++k2) wt[k2] = ldtw<TWS>(tw + n1 * k2);
+  if constexpr (NW % N1 == 0 || N1 % NW == 0) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int full = NL & ~31;
-    for (int l = (w / N1) * 32 + lane; l < full; l += 32 * (NW / N1))
-      passA_item<N1, N2, N1, INV>(buf + l * P + n1, [&](int k2) { return wt[k2]; });
+    for (int n1 = w % N1; n1 < N1; n1 += NW) {
+      float2 wt[N2];
+#pragma unroll
+      for (int k2 = 1; k2 < N2; ++k2) wt[k2] = ldtw<TWS>(tw + n1 * k2);
+      for (int l = (w / N1) * 32 + lane; l < full; l += 32 * (NW > N1 ? NW / N1 : 1))
+        passA_item<N1, N2, N1, INV>(buf + l * P + n1, [&](int k2) { return wt[k2]; });
+    }
     const int rem = NL - full;
-    if ((int)threadIdx.x < rem * N1) {
-      const int m1 = threadIdx.x / rem, l = full + (int)threadIdx.x - m1 * rem;
+    for (int it = threadIdx.x; it < rem * N1; it += T) {
+      const int m1 = it / rem, l = full + it - m1 * rem;
       passA_item<N1, N2, N1, INV>(buf + l * P + m1, [&](int k2) { return ldtw<TWS>(tw + m1 * k2); });
     }
   } else {

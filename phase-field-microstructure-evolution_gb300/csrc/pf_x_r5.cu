@@ -20,15 +20,15 @@ int x_variants_r5(int nx, XKernels* out, int n) {
       n = add_x<160, 8, 512>(out, n);
       n = add_x<160, 4, 256>(out, n);
       break;
-    case 200:
+    case 200:  // 10 warps: one to each column of the 10 x 10 lines (x pass of 17 fields 495 us with 8 or 16 warps, 429)
+      n = add_x<200, 8, 320, 2>(out, n, ",2/SM");
       n = add_x<200, 8, 256, 3>(out, n, ",3/SM");
-      n = add_x<200, 8, 512>(out, n);
-      n = add_x<200, 4, 256>(out, n);
+      n = add_x<200, 4, 320>(out, n);
       n = add_x<200, 2, 256>(out, n);
       break;
-    case 102:
-      n = add_x<102, 17, 256, 2>(out, n, ",2/SM");
-      n = add_x<102, 6, 256, 3>(out, n, ",3/SM");
+    case 102:  // 6 warps: two to each column of the 3 x 17 lines (5 fields 30.8 -> 26.7 us)
+      n = add_x<102, 6, 192, 3>(out, n, ",3/SM");
+      n = add_x<102, 17, 192, 3>(out, n, ",3/SM");
       n = add_x<102, 3, 256>(out, n);
       n = add_x<102, 2, 256>(out, n);
       break;
