@@ -186,15 +186,15 @@ __device__ __forceinline__ void pre_pair(float2 xk, float2 xm, float2 wk, float2
   zk = __fadd2_rn(s, e);
   zm = make_float2(s.x - e.x, e.y - s.y);
 }
-// forward post-processing of the pair (k, M-k), 0 < k < M, scaled by h = scale/2:
+// forward post-processing of the pair (k, M-k), 0 < k < M: twice the spectrum,
 // with s = z_k + conj(z_m), d = z_k - conj(z_m), e = -i d w_k:
-//   x_k = h (s + e),   x_m = h conj(s - e).
-__device__ __forceinline__ void post_pair(float2 zk, float2 zm, float2 wk, float h, float2& xk, float2& xm) {
+//   2 x_k = s + e,   2 x_m = conj(s - e).
+__device__ __forceinline__ void post_pair(float2 zk, float2 zm, float2 wk, float2& xk, float2& xm) {
   const float2 s = __ffma2_rn(zm, make_float2(1.f, -1.f), zk);
   const float2 d = __ffma2_rn(zm, make_float2(-1.f, 1.f), zk);
   const float2 e = make_float2(fmaf(d.x, wk.y, d.y * wk.x), fmaf(-d.x, wk.x, d.y * wk.y));  // -i d wk
-  xk = __fmul2_rn(__fadd2_rn(s, e), make_float2(h, h));
-  xm = __fmul2_rn(make_float2(s.x - e.x, e.y - s.y), make_float2(h, h));
+  xk = __fadd2_rn(s, e);
+  xm = make_float2(s.x - e.x, e.y - s.y);
 }
 
 // Factorization of the x pass's lines (M = Nx/2 complex points): the plan's,
@@ -394,13 +394,18 @@ __device__ __forceinline__ void x_inv_runs(const float2* src, int ks, float2* li
 }
 
 // Forward x transform, last half: forward DFT_N1 of the run pair `pr` (pass
-// B), post-process, store the half spectrum (scaled) to global.
-template <int M, bool TWS = false>
+// B), post-process, store the half spectrum to global: as it comes, 2 Nx times
+// the normalised one, which the yz pass takes into its coefficients, or
+// (SCALED) normalised.
+template <int M, bool SCALED, bool TWS = false>
 __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, const float2* line, int pr,
-                                           float scale, const float2* __restrict__ twN) {
+                                           const float2* __restrict__ twN) {
   constexpr int N1 = XLine<M>::N1, N2 = XLine<M>::N2;
   const int step = N2 * ks;
-  const float h = 0.5f * scale;
+  const auto out = [](float2 x) {
+    constexpr float h = 0.25f / (float)M;  // 1 / (2 Nx)
+    return SCALED ? __fmul2_rn(x, make_float2(h, h)) : x;
+  };
   if (pr > 0 && 2 * pr < N2) {
     const int ra = pr, rb = N2 - pr;
     float2 za[N1], zb[N1];
@@ -416,24 +421,24 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, con
     for (int k1 = 0; k1 < N1; ++k1) {
       const int k = ra + N2 * k1;
       float2 xk, xm;
-      post_pair(za[k1], zb[N1 - 1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
-      da[(ptrdiff_t)k1 * step] = xk;
-      db[(ptrdiff_t)(N1 - 1 - k1) * step] = xm;  // kx = M - k
+      post_pair(za[k1], zb[N1 - 1 - k1], ldtw<TWS>(twN + k), xk, xm);
+      da[(ptrdiff_t)k1 * step] = out(xk);
+      db[(ptrdiff_t)(N1 - 1 - k1) * step] = out(xm);  // kx = M - k
     }
   } else if (pr == 0) {
     float2 z[N1];
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) z[n1] = line[n1];
     Dft<N1>::fwd(z);
-    dst[0] = make_float2((z[0].x + z[0].y) * scale, 0.f);
-    dst[(ptrdiff_t)N1 * step] = make_float2((z[0].x - z[0].y) * scale, 0.f);  // kx = M
+    dst[0] = out(make_float2(2.f * (z[0].x + z[0].y), 0.f));
+    dst[(ptrdiff_t)N1 * step] = out(make_float2(2.f * (z[0].x - z[0].y), 0.f));  // kx = M
 #pragma unroll
     for (int k1 = 1; k1 <= N1 / 2; ++k1) {
       const int k = N2 * k1;
       float2 xk, xm;
-      post_pair(z[k1], z[N1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
-      dst[(ptrdiff_t)k1 * step] = xk;
-      if (k1 != N1 - k1) dst[(ptrdiff_t)(N1 - k1) * step] = xm;
+      post_pair(z[k1], z[N1 - k1], ldtw<TWS>(twN + k), xk, xm);
+      dst[(ptrdiff_t)k1 * step] = out(xk);
+      if (k1 != N1 - k1) dst[(ptrdiff_t)(N1 - k1) * step] = out(xm);
     }
   } else {
     const int ra = N2 / 2;
@@ -446,9 +451,9 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, con
     for (int k1 = 0; k1 < N1 / 2; ++k1) {
       const int k = ra + N2 * k1;
       float2 xk, xm;
-      post_pair(z[k1], z[N1 - 1 - k1], ldtw<TWS>(twN + k), h, xk, xm);
-      da[(ptrdiff_t)k1 * step] = xk;
-      da[(ptrdiff_t)(N1 - 1 - k1) * step] = xm;
+      post_pair(z[k1], z[N1 - 1 - k1], ldtw<TWS>(twN + k), xk, xm);
+      da[(ptrdiff_t)k1 * step] = out(xk);
+      da[(ptrdiff_t)(N1 - 1 - k1) * step] = out(xm);
     }
   }
 }
@@ -458,42 +463,41 @@ __device__ __forceinline__ void x_fwd_runs(float2* __restrict__ dst, int ks, con
 // fields.
 // ---------------------------------------------------------------------------
 struct BulkAcc {
-  float feta, fch;  // per-thread partial sums over a few cells (FP64 from the warp level up)
-  FF mass;          // compensated (exact) per-thread sum of c
+  // per-thread partial sums over a few cells, one for each cell of a slot
+  // (compensated from the warp level up; the mass, hi + lo, throughout)
+  float2 feta, fch, mass_hi, mass_lo;
   float cmin, cmax, phimin, phipmax;
   int nonfinite;
   __device__ __forceinline__ void init() {
-    feta = 0.f; fch = 0.f; mass.hi = 0.f; mass.lo = 0.f;
+    feta = fch = mass_hi = mass_lo = make_float2(0.f, 0.f);
     cmin = 1.0f; cmax = 0.0f; phimin = 1.0f; phipmax = 0.0f;  // reference start values (:1076-1079)
     nonfinite = 0;
   }
+  __device__ __forceinline__ void add_mass(float2 c) {  // two_sum of both cells at once
+    const float2 t = cadd(mass_hi, c), bb = csub(t, mass_hi);
+    mass_lo = cadd(mass_lo, cadd(csub(mass_hi, csub(t, bb)), csub(c, bb)));
+    mass_hi = t;
+  }
+  __device__ __forceinline__ FF mass() const {
+    FF a = ff(mass_hi.x, mass_lo.x);
+    a.add(ff(mass_hi.y, mass_lo.y));
+    return a;
+  }
 };
 
-// Bulk terms of the two cells x = 2m, 2m+1 held in one float2 slot of every
-// field line.  Pass 1 forms the per-cell aggregates, pass 2 overwrites each
-// phi slot with dF/dphi_i; dF/dc and the mobility are returned.
+// Bulk terms of a slot cell by cell, phi rescaled by 1/max|phi| where FP32
+// would lose phi^4 (bulk_slot).
 template <int PM, int WY>
-__device__ __forceinline__ void bulk_slot(float2* smem, int yy, int slot, const RunParams& rp, float2& dfdc,
-                                          float2& mob, BulkAcc& acc) {
+__device__ __forceinline__ void bulk_slot_tiny(float2* base, const RunParams& rp, float2 pre2, float2 n4v, float2 prs,
+                                               float2& dfdc, float2& mob, BulkAcc& acc) {
   const int V = rp.V;
   const float sg1 = rp.sigma1, sg2 = rp.sigma2;
-  float2* base = smem + yy * PM + slot;
-  constexpr int FS = WY * PM;  // stride between fields
-  // pass 1: S2 = sum phi^2, Smat = sum_{i<V-1} phi^2, S4, N4, f_eta pair
-  // sum, both cells of the slot at once in packed FP32 pairs
-  float2 pre = make_float2(0.f, 0.f), n4v = make_float2(0.f, 0.f), prs = make_float2(0.f, 0.f);
-#pragma unroll 4
-  for (int f = 0; f < V - 1; ++f) {
-    const float2 p = base[f * FS];
-    const float2 a = __fmul2_rn(p, p);
-    prs = __ffma2_rn(a, pre, prs);
-    pre = __fadd2_rn(pre, a);
-    n4v = __ffma2_rn(a, a, n4v);
-  }
-  const float pre0 = pre.x, pre1 = pre.y, n40 = n4v.x, n41 = n4v.y, pr0 = prs.x, pr1 = prs.y;
+  constexpr int FS = WY * PM;
+  const float pre0 = pre2.x, pre1 = pre2.y, n40 = n4v.x, n41 = n4v.y, pr0 = prs.x, pr1 = prs.y;
   const float2 pP = base[(V - 1) * FS];
   const float2 cc = base[V * FS];
   float2 out_df[2];
+  float fch[2], feta[2];
   float t4a[2], t4p[2], invm[2], rP4[2];
   float Smat[2], gP[2];
   // per-cell scalar work (two cells)
@@ -545,10 +549,9 @@ __device__ __forceinline__ void bulk_slot(float2* smem, int yy, int slot, const 
     const float dcm = c - rp.c0m, dcp = c - rp.c0p;
     const float fm = rp.am * dcm * dcm, fp = rp.ap * dcp * dcp;
     const float dfm = fm - fp;
-    acc.fch += h * fm + (1.f - h) * fp;
+    fch[q] = h * fm + (1.f - h) * fp;
     const float dc = 2.f * h * rp.am * dcm + 2.f * (1.f - h) * rp.ap * dcp;
-    acc.feta += -0.5f * S2 + 0.25f * S4 + sg1 * pairs + sg2 * pp2 * pre;
-    acc.mass.add(c);
+    feta[q] = -0.5f * S2 + 0.25f * S4 + sg1 * pairs + sg2 * pp2 * pre;
     acc.cmin = fminf(acc.cmin, c);
     acc.cmax = fmaxf(acc.cmax, c);
     acc.phimin = fminf(acc.phimin, S2);
@@ -569,30 +572,11 @@ __device__ __forceinline__ void bulk_slot(float2* smem, int yy, int slot, const 
   }
   dfdc = make_float2(out_df[0].x, out_df[1].x);
   mob = make_float2(out_df[0].y, out_df[1].y);
-  // pass 2: dF/dphi_i = phi^3 - phi + 2 phi Gamma_i + term4_i   (:782-857)
-  // with Gamma_i = sigma1 (Smat - phi_i^2) + sigma2 phiP^2 and term4_i =
-  // t4a q_i^3, q_i = phi_i / max|phi| (the rescaled branch) or phi_i.
+  acc.fch = cadd(acc.fch, make_float2(fch[0], fch[1]));
+  acc.feta = cadd(acc.feta, make_float2(feta[0], feta[1]));
+  acc.add_mass(cc);
   float dsum = dfdc.x + dfdc.y;
-  if (invm[0] == 1.f && invm[1] == 1.f) {
-    // packed over the slot's two cells:
-    //   dF = phi (2 sigma1 (Smat - phi^2) + phi^2 (1 + t4a) + 2 gP - 1)
-    const float2 two_s1 = make_float2(2.f * sg1, 2.f * sg1), m1 = make_float2(-1.f, -1.f);
-    const float2 opt4 = make_float2(1.f + t4a[0], 1.f + t4a[1]);
-    const float2 cterm = make_float2(fmaf(2.f, gP[0], -1.f), fmaf(2.f, gP[1], -1.f));
-    const float2 sm = make_float2(Smat[0], Smat[1]);
-    float2 ds = make_float2(0.f, 0.f);
-#pragma unroll 4
-    for (int f = 0; f < V - 1; ++f) {
-      const float2 p = base[f * FS];
-      const float2 p2 = __fmul2_rn(p, p);
-      const float2 sd = __ffma2_rn(p2, m1, sm);                              // Smat - phi^2
-      const float2 h = __ffma2_rn(sd, two_s1, __ffma2_rn(p2, opt4, cterm));
-      const float2 d = __fmul2_rn(p, h);
-      ds = __fadd2_rn(ds, d);
-      base[f * FS] = d;
-    }
-    dsum += ds.x + ds.y;
-  } else {
+  {
     for (int f = 0; f < V - 1; ++f) {
       float2 p = base[f * FS];
       const float g0 = fmaf(sg1, Smat[0] - p.x * p.x, gP[0]);
@@ -614,6 +598,83 @@ __device__ __forceinline__ void bulk_slot(float2* smem, int yy, int slot, const 
   acc.nonfinite += !isfinite(dsum);  // any NaN/Inf term makes the sum non-finite
 }
 
+// Bulk terms of the two cells x = 2m, 2m+1 held in one float2 slot of every
+// field line, both at once in packed FP32 pairs.  Pass 1 forms the per-cell
+// aggregates, pass 2 overwrites each phi slot with dF/dphi_i; dF/dc and the
+// mobility are returned.  Cells with S4 = sum phi^4 below 1e-30 (or a NaN) take
+// bulk_slot_tiny instead.
+template <int PM, int WY>
+__device__ __forceinline__ void bulk_slot(float2* smem, int yy, int slot, const RunParams& rp, float2& dfdc,
+                                          float2& mob, BulkAcc& acc) {
+  const int V = rp.V;
+  const float sg1 = rp.sigma1, sg2 = rp.sigma2;
+  float2* base = smem + yy * PM + slot;
+  constexpr int FS = WY * PM;  // stride between fields
+  const auto both = [](float x) { return make_float2(x, x); };
+  // pass 1: pre = sum_{i<V-1} phi^2, n4 = sum_{i<V-1} phi^4, prs = the f_eta pair sum
+  float2 pre = both(0.f), n4 = both(0.f), prs = both(0.f);
+#pragma unroll 4
+  for (int f = 0; f < V - 1; ++f) {
+    const float2 p = base[f * FS];
+    const float2 a = __fmul2_rn(p, p);
+    prs = __ffma2_rn(a, pre, prs);
+    pre = __fadd2_rn(pre, a);
+    n4 = __ffma2_rn(a, a, n4);
+  }
+  const float2 pP = base[(V - 1) * FS], c = base[V * FS];
+  const float2 pp2 = __fmul2_rn(pP, pP), pp4 = __fmul2_rn(pp2, pp2);
+  const float2 S2 = __fadd2_rn(pre, pp2), S4 = __fadd2_rn(n4, pp4);
+  if (!(S4.x >= 1e-30f && S4.y >= 1e-30f)) {
+    bulk_slot_tiny<PM, WY>(base, rp, pre, n4, prs, dfdc, mob, acc);
+    return;
+  }
+  const float2 invS4 = make_float2(1.f / S4.x, 1.f / S4.y);
+  const float2 h = __fmul2_rn(n4, invS4), g = csub(both(1.f), h);  // phi_mat (:741) and phi_ppt
+  const float2 dcm = __fadd2_rn(c, both(-rp.c0m)), dcp = __fadd2_rn(c, both(-rp.c0p));
+  const float2 adm = __fmul2_rn(both(rp.am), dcm), adp = __fmul2_rn(both(rp.ap), dcp);
+  const float2 fm = __fmul2_rn(adm, dcm), fp = __fmul2_rn(adp, dcp), dfm = csub(fm, fp);
+  acc.fch = __fadd2_rn(acc.fch, __ffma2_rn(h, fm, __fmul2_rn(g, fp)));
+  dfdc = __fmul2_rn(both(2.f), __ffma2_rn(h, adm, __fmul2_rn(g, adp)));
+  // -0.5 S2 + 0.25 S4 + sigma_1 pairs + sigma_2 phi_P^2 pre
+  const float2 eta = __ffma2_rn(both(0.25f), S4, __fmul2_rn(both(-0.5f), S2));
+  acc.feta = __fadd2_rn(acc.feta, __ffma2_rn(both(sg2), __fmul2_rn(pp2, pre), __ffma2_rn(both(sg1), prs, eta)));
+  acc.add_mass(c);
+  acc.cmin = fminf(acc.cmin, fminf(c.x, c.y));
+  acc.cmax = fmaxf(acc.cmax, fmaxf(c.x, c.y));
+  acc.phimin = fminf(acc.phimin, fminf(S2.x, S2.y));
+  acc.phipmax = fmaxf(acc.phipmax, fmaxf(pP.x, pP.y));
+  if (rp.mobility == MOB_REF_VAR) mob = __fmul2_rn(both(2.f * rp.D_gb), csub(both(1.f), S2));
+  else if (rp.mobility == MOB_C1MC) mob = __fmul2_rn(__fmul2_rn(both(rp.D_L), c), csub(both(1.f), c));
+  else mob = both(0.f);
+  // term4_i = t4a phi_i^3 (i < V-1), t4p for the precipitate (:829-835), in
+  // the ratios phi_P^4 / S4, phi_P^3 / S4 and N4 / S4
+  const float2 d4 = __fmul2_rn(both(4.f), dfm);
+  const float2 t4a = __fmul2_rn(__fmul2_rn(invS4, __fmul2_rn(pp4, invS4)), d4);
+  const float2 t4p = __fmul2_rn(__fmul2_rn(__fmul2_rn(__fmul2_rn(pP, pp2), invS4), h), d4);  // its negative
+  // pass 2: dF/dphi_i = phi^3 - phi + 2 phi Gamma_i + term4_i   (:782-857)
+  // with Gamma_i = sigma1 (Smat - phi_i^2) + sigma2 phiP^2:
+  //   dF = phi (2 sigma1 (Smat - phi^2) + phi^2 (1 + t4a) + 2 sigma2 phiP^2 - 1)
+  const float2 two_s1 = both(2.f * sg1), m1 = both(-1.f);
+  const float2 opt4 = __fadd2_rn(both(1.f), t4a);
+  const float2 cterm = __ffma2_rn(both(2.f * sg2), pp2, m1);
+  float2 ds = dfdc;
+#pragma unroll 4
+  for (int f = 0; f < V - 1; ++f) {
+    const float2 p = base[f * FS];
+    const float2 p2 = __fmul2_rn(p, p);
+    const float2 sd = __ffma2_rn(p2, m1, pre);  // Smat - phi^2
+    const float2 q = __ffma2_rn(sd, two_s1, __ffma2_rn(p2, opt4, cterm));
+    const float2 d = __fmul2_rn(p, q);
+    ds = __fadd2_rn(ds, d);
+    base[f * FS] = d;
+  }
+  // precipitate: phi^3 - phi + 2 sigma2 Smat phi + t4p
+  const float2 dP = csub(__fmul2_rn(pP, __ffma2_rn(both(2.f * sg2), pre, __fadd2_rn(pp2, m1))), t4p);
+  ds = __fadd2_rn(ds, dP);
+  base[(V - 1) * FS] = dP;
+  acc.nonfinite += !isfinite(ds.x + ds.y);  // any NaN/Inf term makes the sum non-finite
+}
+
 // Block reduction of the x pass's diagnostics into the block's partials
 // part_x[(par * XQ_COUNT + q) * nblk_x + blk] (all threads of the block call it).  Sums travel as
 // compensated FP32 pairs: FP64 arithmetic is scarce on this part, and a
@@ -627,7 +688,8 @@ __device__ __forceinline__ void store_block_diag(const BulkAcc& acc, const RunPa
   __shared__ float red_m[4][NW];
   __shared__ int red_i[NW];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const FF s0 = warp_sum_ff(ff(acc.feta)), s1 = warp_sum_ff(ff(acc.fch)), s2 = warp_sum_ff(acc.mass);
+  const FF s0 = warp_sum_ff(ff(acc.feta.x + acc.feta.y)), s1 = warp_sum_ff(ff(acc.fch.x + acc.fch.y)),
+           s2 = warp_sum_ff(acc.mass());
   const float m0 = warp_min(acc.cmin), m1 = warp_max(acc.cmax), m2 = warp_min(acc.phimin), m3 = warp_max(acc.phipmax);
   const int nb = __reduce_add_sync(0xffffffffu, acc.nonfinite);
   if (lane == 0) {
@@ -827,11 +889,10 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
   passA_rt<M, PM, T, false, TWS>(smem, nF * WY, twM);
   __syncthreads();
   float2* __restrict__ dst = (MODE == MODE_BULK) ? rp.D : (MODE == MODE_XJ ? rp.J : rp.Sm);
-  const float scale = 1.0f / (float)NX;
   for (int it = threadIdx.x; it < nF * WY * NP; it += T) {
     const int q = by_line(it), l = it - q * (nF * WY), pr = x_run_pair<M>(q);
     const int f = l / WY, yy = l - f * WY;
-    x_fwd_runs<M, TWS>(dst + f * fstride + row_off + yy, ks, smem + l * PM, pr, scale, twN);
+    x_fwd_runs<M, MODE == MODE_IMPORT, TWS>(dst + f * fstride + row_off + yy, ks, smem + l * PM, pr, twN);
   }
 
   if (MODE != MODE_BULK) return;
@@ -892,11 +953,18 @@ __device__ __forceinline__ void stage_kz(float4* qt, const Shape& sh) {
   }
 }
 
+// Normalisation of what a yz pass transforms: over y and z, and over x where
+// the x pass has left that to it (x_fwd_runs).
+template <int MODE>
+__device__ __forceinline__ float yz_norm(int nyz, int nx) {
+  return 1.0f / ((float)nyz * (MODE == YZ_IMPORT ? 1.0f : 2.0f * (float)nx));
+}
+
 struct KPlane {
   float qx2, qx4, qnx;
   float a;    // t = a Q
   float b;    // coefficient of the driving term, normalisation included
-  float nrm;  // 1 / (NY NZ)
+  float nrm;  // normalisation of the transforms
   float kc;   // kappa_c
   __device__ __forceinline__ KPlane(const RunParams& rp, const Shape& sh, int kx, int mode, bool is_c, float nrm_) {
     qx2 = sh.qx2[kx];
@@ -1317,7 +1385,7 @@ __global__ void __launch_bounds__(T, MINB) yz_kernel(const RunParams* __restrict
 
   // 2. last forward z pass, pointwise k-space update, first inverse z pass,
   //    fused per run of N1z positions
-  const KPlane P(rp, sh, kx, MODE, is_c, 1.0f / (float)(NY * NZ));
+  const KPlane P(rp, sh, kx, MODE, is_c, yz_norm<MODE>(NY * NZ, sh.Nx));
   const float wkx = (kx == 0 || 2 * kx == sh.Nx) ? 1.0f : 2.0f;
   float fint = 0.f;
   {
@@ -1499,7 +1567,7 @@ __global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restric
   colA<NY, NZ, T, false, RAWP, TWS>(U, twZ);
   __syncthreads();
   // 2. last forward z pass, pointwise k-space update, first inverse z pass
-  const KPlane P(rp, sh, kx, MODE, is_c, 1.0f / (float)(NY * NZ));
+  const KPlane P(rp, sh, kx, MODE, is_c, yz_norm<MODE>(NY * NZ, sh.Nx));
   const float wkx = (kx == 0 || 2 * kx == sh.Nx) ? 1.0f : 2.0f;
   float fint = 0.f;
   {
