@@ -70,17 +70,17 @@ static int add_yz1(YZKernels* out, int n) {
   return n + 1;
 }
 
-// ... and with clusters of C CTAs per plane.
-template <int NY, int NZ, int C, int T, int MINB = 0, int UC = Line<NZ>::N1>
+// ... and with C CTAs per plane, ZA, ZB and ZP points of z in the first three passes.
+template <int NY, int NZ, int C, int T, bool RAWP, int ZA, int ZB, int ZP = 1, int MINB = 0, int UC = 0>
 static int add_yz(YZKernels* out, int n) {
   if (n >= kMaxVariants) return n;
   YZKernels& k = out[n];
-  k.main = yz_kernel<NY, NZ, C, T, YZ_MAIN, MINB, UC>;
-  k.c2 = yz_kernel<NY, NZ, C, T, YZ_C2, MINB, UC>;
-  k.imp = yz_kernel<NY, NZ, C, T, YZ_IMPORT, MINB, UC>;
+  k.main = yz_kernel<NY, NZ, C, T, YZ_MAIN, RAWP, ZA, ZB, ZP, MINB, UC>;
+  k.c2 = yz_kernel<NY, NZ, C, T, YZ_C2, RAWP, ZA, ZB, ZP, MINB, UC>;
+  k.imp = yz_kernel<NY, NZ, C, T, YZ_IMPORT, RAWP, ZA, ZB, ZP, MINB, UC>;
   k.cluster = C;
   k.threads = T;
-  k.smem = YZ<NY, NZ, C>::SMEM;
+  k.smem = YZ<NY, NZ, C, RAWP, ZA, ZB, ZP>::SMEM;
   return n + 1;
 }
 

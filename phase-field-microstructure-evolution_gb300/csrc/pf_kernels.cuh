@@ -912,24 +912,10 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
 //   * forms u_hat_new = u_hat + m1 u_hat + m2 D_hat (semi-implicit update),
 //   * transforms u_hat_new back over z and y to the mixed-space field the next
 //     x pass reads (Sm).
-// A cluster of C CTAs shares a plane: CTA r holds z rows [r*NZ/C, ...) for
-// the y transforms ("A layout") and y positions [r*NY/C, ...) for the z
-// transforms ("B layout"); the layouts are exchanged through distributed
-// shared memory.  All loops have compile-time trip counts.
+// Two kernels do it: yz1_kernel, one CTA per plane, one transform stage per
+// pass over shared memory; and yz_kernel, stages of y and z in one pass and a
+// cluster of CTAs where a plane is shared.  All loops have compile-time trip counts.
 // ---------------------------------------------------------------------------
-template <int NY, int NZ, int C>
-struct YZ {
-  static constexpr int LA = NZ / C;  // z rows per CTA (A layout)
-  static constexpr int LB = NY / C;  // y positions per CTA (B layout)
-  static constexpr int PY = Line<NY>::PITCH;
-  static constexpr int PZ = Line<NZ>::PITCH;
-  static constexpr int UA = LA * PY;
-  static constexpr int UB = LB * PZ;
-  // the A and B layouts share one buffer
-  static constexpr size_t SMEM = (size_t)(UA > UB ? UA : UB) * sizeof(float2);
-  static_assert(NZ % C == 0 && NY % C == 0, "cluster must divide the plane");
-};
-
 enum YZMode { YZ_MAIN = 0, YZ_C2 = 1, YZ_IMPORT = 2 };
 
 // ---------------------------------------------------------------------------
@@ -1205,105 +1191,8 @@ __device__ __forceinline__ float2 ld_peer(uint32_t a) {
   return v;
 }
 
-// In-place exchanges: every thread first reads all the elements it will own
-// in the new layout from the cluster's old layouts (into registers), the
-// cluster waits until every CTA has read everything it needs, and then each
-// CTA overwrites its own buffer with the new layout.  One buffer per CTA
-// instead of two, so a quarter of a 256 x 256 plane (140 KB) fits one CTA.
-//
-// One side of an exchange: CTA r gets, for its own position of the old lines
-// (at src, pitch PS), the elements of lines x0 + k S of the cluster, LS lines
-// per CTA, and stores them as one line of the new layout (at dst, runs of N1).
-// Every CTA starts with its own lines and goes round, so that no CTA's shared
-// memory serves all the others at once.
-template <int C, int LS, int PS, int N1, int S, int ITER>
-__device__ __forceinline__ void exchange(float2* __restrict__ dst, uint32_t src, int x0, int r) {
-  float2 v[ITER];
-  if constexpr (LS % S == 0 && LS % N1 == 0) {
-    constexpr int J = LS / S;
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const int o = r + i < C ? r + i : r + i - C;
-      const uint32_t a = map_rank(src + (uint32_t)(x0 * PS) * 8u, o);
-#pragma unroll
-      for (int j = 0; j < J; ++j) v[i * J + j] = ld_peer(a + (uint32_t)(j * S * PS * 8));
-    }
-    cluster_barrier();  // every CTA holds its new layout in registers
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const int o = r + i < C ? r + i : r + i - C;
-      float2* d = dst + o * (LS + LS / N1) + x0;
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        if constexpr (N1 % S == 0) d[j * S + (j * S) / N1] = v[i * J + j];  // x0 < S
-        else d[j * S + (x0 + j * S) / N1] = v[i * J + j];
-      }
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < ITER; ++k) {
-      const int x = x0 + k * S, owner = x / LS;
-      v[k] = ld_peer(map_rank(src + (uint32_t)((x - owner * LS) * PS) * 8u, owner));
-    }
-    cluster_barrier();
-#pragma unroll
-    for (int k = 0; k < ITER; ++k) dst[x0 + k * S + (x0 + k * S) / N1] = v[k];
-  }
-  __syncthreads();
-}
-
-// A (z rows of LA, pitch PY) -> B (y positions of LB, pitch PZ)
-template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_AB(float2* __restrict__ buf, uint32_t base, int r) {
-  using G = YZ<NY, NZ, C>;
-  static_assert(T % G::LB == 0 && (G::LB * NZ) % T == 0, "threads must cover whole rows");
-  const int yl = threadIdx.x % G::LB;
-  exchange<C, G::LA, G::PY, Line<NZ>::N1, T / G::LB, G::LB * NZ / T>(
-      buf + yl * G::PZ, base + (uint32_t)(Line<NY>::phys(r * G::LB + yl)) * 8u, threadIdx.x / G::LB, r);
-}
-
-// B -> A
-template <int NY, int NZ, int C, int T>
-__device__ __forceinline__ void exch_BA(float2* __restrict__ buf, uint32_t base, int r) {
-  using G = YZ<NY, NZ, C>;
-  static_assert(T % G::LA == 0 && (G::LA * NY) % T == 0, "threads must cover whole lines");
-  const int zl = threadIdx.x % G::LA;
-  exchange<C, G::LB, G::PZ, Line<NY>::N1, T / G::LA, G::LA * NY / T>(
-      buf + zl * G::PY, base + (uint32_t)(Line<NZ>::phys(r * G::LA + zl)) * 8u, threadIdx.x / G::LA, r);
-}
-
-// pass A (forward or inverse) over NL lines of length L, pitch P, T threads
-template <int L, int NL, int P, int T, bool INV>
-__device__ __forceinline__ void passA(float2* buf, const float2* __restrict__ tw) {
-  constexpr int N1 = Line<L>::N1, N2 = Line<L>::N2;
-  static_assert(T % N1 == 0, "threads must be a multiple of N1");
-  const int n1 = threadIdx.x % N1;
-  float2 w[N2];
-#pragma unroll
-  for (int k2 = 1; k2 < N2; ++k2) w[k2] = __ldg(tw + n1 * k2);
-  constexpr int ITEMS = NL * N1, ITER = (ITEMS + T - 1) / T;
-#pragma unroll
-  for (int j = 0; j < ITER; ++j) {
-    const int it = threadIdx.x + j * T;
-    if (ITEMS % T != 0 && it >= ITEMS) break;
-    const int l = it / N1;
-    float2* p = buf + l * P + n1;
-    float2 v[N2];
-    if (!INV) {
-#pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) v[n2] = p[n2 * (N1 + 1)];
-      Dft<N2>::fwd(v);
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmul(v[k2], w[k2]);
-    } else {
-      v[0] = p[0];
-#pragma unroll
-      for (int k2 = 1; k2 < N2; ++k2) v[k2] = cmulc(p[k2 * (N1 + 1)], w[k2]);
-      dft_inv<N2>(v);
-    }
-#pragma unroll
-    for (int k = 0; k < N2; ++k) p[k * (N1 + 1)] = v[k];
-  }
+__device__ __forceinline__ void st_peer(uint32_t a, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
 }
 
 template <int L, int NL, int P, int T, bool INV>
@@ -1325,148 +1214,12 @@ __device__ __forceinline__ void passB(float2* buf) {
   }
 }
 
-template <int NY, int NZ, int C, int T, int MODE, int MINB = 0, int UC = Line<NZ>::N1>
-__global__ void __launch_bounds__(T, MINB) yz_kernel(const RunParams* __restrict__ runs, const Shape sh) {
-  using G = YZ<NY, NZ, C>;
-  using LY = Line<NY>;
-  using LZ = Line<NZ>;
-  constexpr int N1y = LY::N1, N2y = LY::N2, N1z = LZ::N1, N2z = LZ::N2;
-  static_assert(T % N1y == 0 && T % N2z == 0, "thread count");
-  extern __shared__ float2 smem[];
-  __shared__ float4 qzt[NZ];  // kz factors of the k-space update
-  stage_kz<NZ, T>(qzt, sh);   // read after the barriers of the forward passes
-  float2 *UA = smem, *UB = smem;  // both layouts share one buffer
-  const RunParams& rp = runs[blockIdx.y];
-  const int r = (int)(blockIdx.x % C);
-  const int p = sh.plane0 + (int)(blockIdx.x / C);
-  const int Kx = sh.Kx;
-  const int f = (MODE == YZ_C2) ? rp.V : p / Kx;
-  const int kx = p - (p / Kx) * Kx;
-  const size_t plane_elems = (size_t)NZ * NY;
-  const size_t fstride = (size_t)Kx * plane_elems;
-  const size_t poff = f * fstride + kx * plane_elems;  // k-space state
-  const size_t moff = f * fstride + kx * sh.ks;        // mixed space
-  const bool is_c = (f == rp.V);
-  const bool var_c = (MODE == YZ_MAIN) && is_c && rp.mobility != MOB_CONST;
-  const int z0 = r * G::LA;
-
-  // 1. forward y transform of the mixed-space input rows z0..z0+LA
-  //    (MAIN/IMPORT: D~ or S~; C2: J~'), first pass straight from global
-  {
-    const float2* src = (MODE == YZ_MAIN) ? rp.D + moff : (MODE == YZ_C2 ? rp.J + kx * sh.ks : rp.Sm + moff);
-    const int n1 = threadIdx.x % N1y;
-    float2 w[N2y];
-#pragma unroll
-    for (int k2 = 1; k2 < N2y; ++k2) w[k2] = __ldg(sh.twY + n1 * k2);
-    constexpr int ITEMS = G::LA * N1y, ITER = (ITEMS + T - 1) / T;
-#pragma unroll
-    for (int j = 0; j < ITER; ++j) {
-      const int it = threadIdx.x + j * T;
-      if (ITEMS % T != 0 && it >= ITEMS) break;
-      const int zl = it / N1y;
-      const float2* s = src + (z0 + zl) * sh.zs + n1;
-      float2 v[N2y];
-#pragma unroll
-      for (int n2 = 0; n2 < N2y; ++n2) v[n2] = __ldg(s + n2 * N1y);
-      Dft<N2y>::fwd(v);
-      float2* d = UA + zl * G::PY + n1;
-      d[0] = v[0];
-#pragma unroll
-      for (int k2 = 1; k2 < N2y; ++k2) d[k2 * (N1y + 1)] = cmul(v[k2], w[k2]);
-    }
-  }
-  __syncthreads();
-  passB<NY, G::LA, G::PY, T, false>(UA);
-  cluster_barrier();
-  exch_AB<NY, NZ, C, T>(UB, smem_addr(UA), r);
-  __syncthreads();
-  passA<NZ, G::LB, G::PZ, T, false>(UB, sh.twZ);
-  __syncthreads();
-
-  // 2. last forward z pass, pointwise k-space update, first inverse z pass,
-  //    fused per run of N1z positions
-  const KPlane P(rp, sh, kx, MODE, is_c, yz_norm<MODE>(NY * NZ, sh.Nx));
-  const float wkx = (kx == 0 || 2 * kx == sh.Nx) ? 1.0f : 2.0f;
-  float fint = 0.f;
-  {
-    const int k2 = threadIdx.x % N2z;
-    constexpr int ITEMS = G::LB * N2z, ITER = (ITEMS + T - 1) / T;
-#pragma unroll 1
-    for (int j = 0; j < ITER; ++j) {
-      const int it = threadIdx.x + j * T;
-      if (ITEMS % T != 0 && it >= ITEMS) break;
-      const int yl = it / N2z;
-      const int ypos = r * G::LB + yl;
-      const KRow R(P, sh, LY::freq_of_pos(ypos));
-      float2* pb = UB + yl * G::PZ + k2 * (N1z + 1);
-      // k-space state of this plane in [k1][y position][k2] order: for every
-      // k1 a warp reads and writes consecutive (y position, k2) (coalesced)
-      float2* gk = rp.Sk + poff + (size_t)ypos * N2z + k2;
-      constexpr size_t SK1 = (size_t)NY * N2z;  // stride of k1
-      float2 d[N1z];
-#pragma unroll
-      for (int k1 = 0; k1 < N1z; ++k1) d[k1] = pb[k1];
-      update_run<N1z, N2z, MODE, UC>(d, gk, SK1, P, R, qzt + k2, is_c, var_c, fint);
-      if (MODE != YZ_IMPORT) {
-#pragma unroll
-        for (int k1 = 0; k1 < N1z; ++k1) pb[k1] = d[k1];
-      }
-    }
-  }
-  if (MODE == YZ_IMPORT) {
-    cluster_barrier();  // peers may still read this CTA's A buffer
-    return;
-  }
-  __syncthreads();
-  passA<NZ, G::LB, G::PZ, T, true>(UB, sh.twZ);
-  cluster_barrier();
-  exch_BA<NY, NZ, C, T>(UA, smem_addr(UB), r);  // ends after the last peer read
-  passB<NY, G::LA, G::PY, T, true>(UA);
-  __syncthreads();
-
-  // 3. last inverse y pass straight to the mixed-space output
-  //    (u~ for the next x pass, or J~ for the variable-mobility chain)
-  {
-    const bool real_plane = (kx == 0) || (2 * kx == sh.Nx);  // the x-DFT of real data is real there
-    float2* dst = var_c ? rp.J + kx * sh.ks : rp.Sm + moff;
-    const int n1 = threadIdx.x % N1y;
-    float2 w[N2y];
-#pragma unroll
-    for (int k2 = 1; k2 < N2y; ++k2) w[k2] = __ldg(sh.twY + n1 * k2);
-    constexpr int ITEMS = G::LA * N1y, ITER = (ITEMS + T - 1) / T;
-#pragma unroll
-    for (int j = 0; j < ITER; ++j) {
-      const int it = threadIdx.x + j * T;
-      if (ITEMS % T != 0 && it >= ITEMS) break;
-      const int zl = it / N1y;
-      const float2* s = UA + zl * G::PY + n1;
-      float2 v[N2y];
-      v[0] = s[0];
-#pragma unroll
-      for (int k2 = 1; k2 < N2y; ++k2) v[k2] = cmulc(s[k2 * (N1y + 1)], w[k2]);
-      dft_inv<N2y>(v);
-      float2* o = dst + (z0 + zl) * sh.zs + n1;
-#pragma unroll
-      for (int n2 = 0; n2 < N2y; ++n2) {
-        float2 x = v[n2];
-        if (real_plane && !var_c) x.y = 0.f;
-        o[n2 * N1y] = x;
-      }
-    }
-  }
-
-  if (MODE == YZ_MAIN) {
-    // f_int partial (:609-678 by Parseval): 0.5 kappa N^3 w |kf|^2 |u_hat|^2
-    yz_finish<T>(rp, sh, fint, wkx, (size_t)sh.plane0 * C + blockIdx.x);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Single-CTA yz pass for planes that fit one CTA's shared memory: the plane
 // stays in one buffer U[z][phys_y(y)] (row pitch PY, odd); y transforms run
 // along rows, z transforms down columns (consecutive threads take consecutive
 // y positions, so column accesses are conflict-free).  No re-layout, no
-// cluster.  Same k-space position order as the cluster kernel.
+// cluster.  Same k-space position order as yz_kernel.
 // ---------------------------------------------------------------------------
 // Row pitch: the odd line pitch, or (RAWP) the unpadded run layout
 // N2 (N1 + 1).  yz1 reads columns with lanes along y, so only its row passes
@@ -1634,6 +1387,284 @@ __global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restric
 
   if (MODE == YZ_MAIN) {
     yz_finish<T>(rp, sh, fint, wkx, (size_t)p);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Yz pass whose register passes take stages of both axes, with C CTAs (a
+// cluster) per plane.  z = t + N1 s: a run is the N1 points t of one frequency
+// of s, the s transform has Q = ZA ZB ZP points.  CTA r holds the z rows
+// z = r (mod C), whole rows of y, so every stage but the last is its own:
+//   P1  N2y points of y (stride N1y) x ZA of z, straight from global memory,
+//   P2  a run of N1y points of y x ZB of z,
+//   P3  ZP points of z (left out where ZP = 1),
+//   P4  a run: last forward stage, update, first inverse.
+// and P3, P2, P1 again for the inverse.  A run's points t lie t mod C over the
+// cluster, ZL = N1/C in each CTA: P4 reads them from there, and puts them back
+// there.  Every stage works in place: s frequency kb + ZA ka + ZA ZB kp is found
+// at rows ZL (kp + ZP (ka + ZB kb)) on.  The k-space order is yz1_kernel's.
+//
+// Against re-laying the plane out over the cluster before and after the z
+// transform (each way a pass and two cluster barriers of its own): two cluster
+// barriers instead of five, 12 crossings of shared memory instead of 16, and a
+// P4 that hides the peers' latency behind the state's loads.  Yz pass of 33
+// fields of 256^3 3340 -> 2584 us, of 7 of 200^3 433 -> 302 us, and 160^2 planes
+// (200 KB: one CTA per SM) by clusters of four 385 -> 350 us for 21 fields.
+// C = 1: passes that join two axes save 2 of 6 crossings and barriers.  What
+// bounds several CTAs per SM is the shared-memory data pipe, so it gains at
+// 64^2 (64 runs of 64^3 x 8: 509 -> 446 us, 5.6 TB/s), 96^2 (96^3 x 55: 207 ->
+// 198 us) and 80^2 (80^3 x 50: 97 -> 90 us).
+// What bounds it: barriers and shared memory; DRAM at 50 to 80 % of its rate.
+// One item of P1 at a time: 32 values in flight (unroll 2 to 4) cost 1 to 2 %.
+// ---------------------------------------------------------------------------
+template <int NY, int NZ, int C, bool RAWP, int ZA, int ZB, int ZP>
+struct YZ {
+  static constexpr int Q = ZA * ZB * ZP, N1 = NZ / Q, R = NZ / C, ZL = N1 / C;  // z points a CTA holds: R, ZL of each run
+  static constexpr int PY = RAWP ? Line<NY>::RAW : Line<NY>::PITCH;
+  static constexpr size_t SMEM = (size_t)R * PY * sizeof(float2);
+  static_assert(Q * N1 == NZ && ZL * C == N1 && Q % C == 0, "whole factors");
+};
+
+// P3 (forward or inverse): ZP points (stride S rows) of the H S columns of every y position
+template <int NY, int H, int ZP, int S, int PY, int C, int T, bool INV>
+__device__ __forceinline__ void colP(float2* U, const float2* twZ, int r) {
+#pragma unroll 2
+  for (int it = threadIdx.x; it < NY * S * H; it += T) {
+    const int g = it / NY, yp = it - g * NY, h = g / S, j = g - h * S;
+    const int t = (r + C * j) * H;
+    passA_item<S, ZP, S * PY, INV>(U + (j + S * ZP * h) * PY + Line<NY>::phys(yp), [&](int k) { return twZ[t * k]; });
+  }
+}
+
+template <int NY, int NZ, int C, int T, int MODE, bool RAWP, int ZA, int ZB, int ZP, int MINB, int UCT>
+__global__ void __launch_bounds__(T, MINB) yz_kernel(const RunParams* __restrict__ runs, const Shape sh) {
+  using LY = Line<NY>;
+  using G = YZ<NY, NZ, C, RAWP, ZA, ZB, ZP>;
+  constexpr int N1y = LY::N1, N2y = LY::N2, N1z = G::N1, Q = G::Q, ZL = G::ZL, PY = G::PY;
+  constexpr int S3 = ZL, S2 = S3 * ZP, S1 = S2 * ZB;  // row strides of the stages ZP, ZB, ZA
+  constexpr int UC = UCT ? UCT : N1z;
+  static_assert(T % 32 == 0, "whole warps");
+  extern __shared__ float2 U[];
+  constexpr int QC = Q / C;           // runs a CTA updates
+  __shared__ float4 qzt[QC * N1z];    // their kz factors, in the runs' order
+  __shared__ float2 twZ[NZ];
+  const int r = C == 1 ? 0 : (int)(blockIdx.x % C);
+  const auto freq = [](int rr) { return rr / (ZP * ZB) + ZA * (rr / ZP % ZB) + ZA * ZB * (rr % ZP); };
+  for (int j = threadIdx.x; j < QC * N1z; j += T) {
+    const int k = freq(r * QC + j / N1z) + Q * (j % N1z);
+    const float n = __ldg(sh.qnz + k);
+    qzt[j] = make_float4(__ldg(sh.qz2 + k), __ldg(sh.qz4 + k), n, n * n);
+  }
+  for (int j = threadIdx.x; j < NZ; j += T) twZ[j] = __ldg(sh.twZ + j);
+  const RunParams& rp = runs[blockIdx.y];
+  const int p = sh.plane0 + (int)(blockIdx.x / C);
+  const int Kx = sh.Kx;
+  const int f = (MODE == YZ_C2) ? rp.V : p / Kx;
+  const int kx = p - (p / Kx) * Kx;
+  const size_t plane_elems = (size_t)NZ * NY;
+  const size_t poff = ((size_t)f * Kx + kx) * plane_elems;        // k-space state
+  const size_t moff = (size_t)f * Kx * plane_elems + kx * sh.ks;  // mixed space
+  const bool is_c = (f == rp.V);
+  const bool var_c = (MODE == YZ_MAIN) && is_c && rp.mobility != MOB_CONST;
+
+  // y twiddles of a column n1y: preloaded when every item of a thread has the same one
+  constexpr bool FIXED = T % N1y == 0;
+  const auto load_wy = [&](float2* wy, int n1y) {
+#pragma unroll
+    for (int k2 = 1; k2 < N2y; ++k2) wy[k2] = __ldg(sh.twY + n1y * k2);
+  };
+  constexpr int I1 = N1y * S1, I2 = N2y * S2 * ZA;  // items of P1 and P2
+  __syncthreads();  // the tables
+
+  // P1 forward
+  {
+    const float2* src = (MODE == YZ_MAIN) ? rp.D + moff : (MODE == YZ_C2 ? rp.J + kx * sh.ks : rp.Sm + moff);
+    float2 wy[N2y];
+    if constexpr (FIXED) load_wy(wy, threadIdx.x % N1y);
+#pragma unroll 1
+    for (int it = threadIdx.x; it < I1; it += T) {
+      const int m = it / N1y, n1y = it - m * N1y;
+      float2 v[ZA][N2y];
+#pragma unroll
+      for (int b = 0; b < ZA; ++b) {
+        const float2* s = src + (r + C * (m + S1 * b)) * sh.zs + n1y;
+#pragma unroll
+        for (int n2 = 0; n2 < N2y; ++n2) v[b][n2] = __ldg(s + n2 * N1y);
+      }
+      if constexpr (!FIXED) load_wy(wy, n1y);
+      float2* d = U + m * PY + n1y;
+#pragma unroll
+      for (int b = 0; b < ZA; ++b) {
+        Dft<N2y>::fwd(v[b]);
+#pragma unroll
+        for (int k2 = 1; k2 < N2y; ++k2) v[b][k2] = cmul(v[b][k2], wy[k2]);
+      }
+      float2 wz[ZA];
+#pragma unroll
+      for (int kb = 1; kb < ZA; ++kb) wz[kb] = twZ[(r + C * m) * kb];
+#pragma unroll
+      for (int k2 = 0; k2 < N2y; ++k2) {
+        float2 c[ZA];
+#pragma unroll
+        for (int b = 0; b < ZA; ++b) c[b] = v[b][k2];
+        Dft<ZA>::fwd(c);
+#pragma unroll
+        for (int kb = 0; kb < ZA; ++kb)
+          d[S1 * kb * PY + k2 * (N1y + 1)] = kb == 0 ? c[0] : cmul(c[kb], wz[kb]);
+      }
+    }
+  }
+  __syncthreads();
+  // P2 forward
+#pragma unroll 1
+  for (int it = threadIdx.x; it < I2; it += T) {
+    const int g = it / N2y, k2y = it - g * N2y, kb = g / S2, m = g - kb * S2;
+    float2* q = U + (m + S1 * kb) * PY + k2y * (N1y + 1);
+    float2 v[ZB][N1y];
+#pragma unroll
+    for (int a = 0; a < ZB; ++a) {
+#pragma unroll
+      for (int j = 0; j < N1y; ++j) v[a][j] = q[S2 * a * PY + j];
+    }
+#pragma unroll
+    for (int a = 0; a < ZB; ++a) Dft<N1y>::fwd(v[a]);
+    float2 wz[ZB];
+#pragma unroll
+    for (int ka = 1; ka < ZB; ++ka) wz[ka] = twZ[(r + C * m) * ZA * ka];
+#pragma unroll
+    for (int j = 0; j < N1y; ++j) {
+      float2 c[ZB];
+#pragma unroll
+      for (int a = 0; a < ZB; ++a) c[a] = v[a][j];
+      Dft<ZB>::fwd(c);
+#pragma unroll
+      for (int ka = 0; ka < ZB; ++ka) q[S2 * ka * PY + j] = ka == 0 ? c[0] : cmul(c[ka], wz[ka]);
+    }
+  }
+  if (C == 1 || ZP > 1) __syncthreads();
+  // P3 forward: z points ZP of a column
+  if constexpr (ZP > 1) {
+    colP<NY, ZA * ZB, ZP, S3, PY, C, T, false>(U, twZ, r);
+    if (C == 1) __syncthreads();
+  }
+  if (C > 1) cluster_barrier();
+  // P4: last forward z stage, pointwise k-space update, first inverse z stage
+  const KPlane P(rp, sh, kx, MODE, is_c, yz_norm<MODE>(NY * NZ, sh.Nx));
+  const float wkx = (kx == 0 || 2 * kx == sh.Nx) ? 1.0f : 2.0f;
+  float fint = 0.f;
+#pragma unroll 1
+  for (int it = threadIdx.x; it < NY * QC; it += T) {
+    const int yp = it % NY, rl = it / NY, rr = r * QC + rl;
+    const KRow R(P, sh, LY::freq_of_pos(yp));
+    float2* pc = U + rr * ZL * PY + LY::phys(yp);
+    // k-space state of this plane in [k1][k2][y position] order: for every
+    // k1 a warp reads and writes 32 consecutive y positions (coalesced)
+    float2* gk = rp.Sk + poff + freq(rr) * NY + yp;
+    constexpr size_t SK1 = (size_t)Q * NY;  // stride of k1
+    const uint32_t a = smem_addr(pc);
+    float2 d[N1z];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const uint32_t ac = C > 1 ? map_rank(a, c) : 0;
+#pragma unroll
+      for (int j = 0; j < ZL; ++j) d[c + C * j] = C > 1 ? ld_peer(ac + (uint32_t)(j * PY * 8)) : pc[j * PY];
+    }
+    update_run<N1z, 1, MODE, UC>(d, gk, SK1, P, R, qzt + rl * N1z, is_c, var_c, fint);
+    if (MODE != YZ_IMPORT) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const uint32_t ac = C > 1 ? map_rank(a, c) : 0;
+#pragma unroll
+        for (int j = 0; j < ZL; ++j) {
+          if (C > 1) st_peer(ac + (uint32_t)(j * PY * 8), d[c + C * j]);
+          else pc[j * PY] = d[j];
+        }
+      }
+    }
+  }
+  if (C > 1) cluster_barrier();  // also: nothing reads a CTA that has left
+  if (MODE == YZ_IMPORT) return;
+  if (C == 1) __syncthreads();
+  // P3 inverse: z points ZP of a column
+  if constexpr (ZP > 1) {
+    colP<NY, ZA * ZB, ZP, S3, PY, C, T, true>(U, twZ, r);
+    __syncthreads();
+  }
+  // P2 inverse
+#pragma unroll 1
+  for (int it = threadIdx.x; it < I2; it += T) {
+    const int g = it / N2y, k2y = it - g * N2y, kb = g / S2, m = g - kb * S2;
+    float2* q = U + (m + S1 * kb) * PY + k2y * (N1y + 1);
+    float2 wz[ZB];
+#pragma unroll
+    for (int ka = 1; ka < ZB; ++ka) wz[ka] = twZ[(r + C * m) * ZA * ka];
+    float2 v[ZB][N1y];
+#pragma unroll
+    for (int j = 0; j < N1y; ++j) {
+      float2 c[ZB];
+#pragma unroll
+      for (int ka = 0; ka < ZB; ++ka) {
+        const float2 x = q[S2 * ka * PY + j];
+        c[ka] = ka == 0 ? x : cmulc(x, wz[ka]);
+      }
+      dft_inv<ZB>(c);
+#pragma unroll
+      for (int a = 0; a < ZB; ++a) v[a][j] = c[a];
+    }
+#pragma unroll
+    for (int a = 0; a < ZB; ++a) {
+      dft_inv<N1y>(v[a]);
+#pragma unroll
+      for (int j = 0; j < N1y; ++j) q[S2 * a * PY + j] = v[a][j];
+    }
+  }
+  __syncthreads();
+  // P1 inverse, straight to the mixed-space output
+  {
+    const bool real_plane = (kx == 0) || (2 * kx == sh.Nx);  // the x-DFT of real data is real there
+    const bool real_out = real_plane && !var_c;
+    float2* dst = var_c ? rp.J + kx * sh.ks : rp.Sm + moff;
+    float2 wy[N2y];
+    if constexpr (FIXED) load_wy(wy, threadIdx.x % N1y);
+#pragma unroll 1
+    for (int it = threadIdx.x; it < I1; it += T) {
+      const int m = it / N1y, n1y = it - m * N1y;
+      const float2* q = U + m * PY + n1y;
+      float2 wz[ZA];
+#pragma unroll
+      for (int kb = 1; kb < ZA; ++kb) wz[kb] = twZ[(r + C * m) * kb];
+      float2 v[ZA][N2y];
+#pragma unroll
+      for (int k2 = 0; k2 < N2y; ++k2) {
+        float2 c[ZA];
+#pragma unroll
+        for (int kb = 0; kb < ZA; ++kb) {
+          const float2 x = q[S1 * kb * PY + k2 * (N1y + 1)];
+          c[kb] = kb == 0 ? x : cmulc(x, wz[kb]);
+        }
+        dft_inv<ZA>(c);
+#pragma unroll
+        for (int b = 0; b < ZA; ++b) v[b][k2] = c[b];
+      }
+      if constexpr (!FIXED) load_wy(wy, n1y);
+#pragma unroll
+      for (int b = 0; b < ZA; ++b) {
+#pragma unroll
+        for (int k2 = 1; k2 < N2y; ++k2) v[b][k2] = cmulc(v[b][k2], wy[k2]);
+        dft_inv<N2y>(v[b]);
+        float2* o = dst + (r + C * (m + S1 * b)) * sh.zs + n1y;
+#pragma unroll
+        for (int n2 = 0; n2 < N2y; ++n2) {
+          float2 x = v[b][n2];
+          if (real_out) x.y = 0.f;
+          o[n2 * N1y] = x;
+        }
+      }
+    }
+  }
+
+  if (MODE == YZ_MAIN) {
+    yz_finish<T>(rp, sh, fint, wkx, (size_t)sh.plane0 * C + blockIdx.x);
   }
 }
 
