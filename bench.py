@@ -464,7 +464,7 @@ def run_ours(args):
             "kernel_variants": lib.pf_batch_variant(b).decode(),
         }
         if ws == 1 and not args.no_fp64:
-            # the plain FP64 GPU path (cuFFT, one kernel per reference phase) on
+            # the FP64 GPU path (cuFFT) on
             # the same workload: its throughput, and the error of this run's
             # fields against it after ERROR_STEPS steps from the same start
             r64 = pkg.Run(p, precision=pkg.PF_FP64_PLAIN, device=local)

@@ -41,7 +41,7 @@ extern "C" {
 
 /* arithmetic of the step */
 #define PF_FP32_FUSED 32 /* fused sm_103a kernels, FP32 fields and FFTs */
-#define PF_FP64_PLAIN 64 /* plain FP64 path: cuFFT + one kernel per reference phase */
+#define PF_FP64_PLAIN 64 /* FP64 path: cuFFT and plain kernels */
 
 /* Coefficients of one run; names and meaning follow input.txt
  * (src/var_diff.f90:104-121). dx, dy, dz are not used by the reference step. */
@@ -122,7 +122,7 @@ int pf_batch_destroy(pf_batch* b);
 
 /* ---- a run's error against the FP64 GPU path -------------------------------
  * The same start stepped nsteps times on the fused FP32 path and on the plain
- * FP64 path (cuFFT + one kernel per phase of src/var_diff.f90:556-1050, held
+ * FP64 path (the phases of src/var_diff.f90:556-1050 with cuFFT, held
  * to the FP64 CPU restatement at 1e-10 by the tests); the fields are compared
  * on the device: max-abs and L2 difference relative to the FP64 fields'
  * max-abs and L2 norm, for all order parameters together and for c.  Holds

@@ -1,7 +1,7 @@
 // pf_check_fp64: the error of the fused FP32 path against the plain FP64 GPU
 // path for one run -- the same start stepped nsteps times on both, the fields
-// compared on the device.  The FP64 path (cuFFT and one kernel per phase of
-// src/var_diff.f90:556-1050) is held to the FP64 CPU oracle at 1e-10 by the
+// compared on the device.  The FP64 path (the phases of
+// src/var_diff.f90:556-1050 with cuFFT) is held to the FP64 CPU oracle at 1e-10 by the
 // tests, so this is the run's error against an FP64 oracle of the reference's
 // algorithm, reported as max-abs and L2 differences relative to the FP64
 // fields' max-abs and L2 norms, for the order parameters together and for c.

@@ -2,8 +2,8 @@
 //
 // State of one run, for every field f (the var order parameters, then the
 // concentration c):
-//   Sk[f][kx][ypos][zpos]  u_hat in k-space (normalised like f_trans,
-//                          src/f_trans.f90:12), y/z in digit-transposed order;
+//   Sk[f][kx][kz][ypos]    u_hat in k-space (normalised like f_trans,
+//                          src/f_trans.f90:12), y in digit-transposed order;
 //   Sm[f][kx][z][y]        (large runs: [f][z][kx][y]) the same field in "mixed" space: its x half
 //                          spectrum (1/Nx) sum_x u e^{-2 pi i kx x/Nx} with y, z
 //                          in real space (what the x pass needs).
@@ -14,7 +14,7 @@
 //   x pass  (x_pass_kernel, one CTA per WY y-rows at one z, all fields):
 //       Sm --C2R_x--> phi, c --bulk terms (src/var_diff.f90:685-898)-->
 //       dF/dphi_i, dF/dc (, mobility) --R2C_x/Nx--> D
-//   yz pass (yz_kernel, one CTA cluster per (field, kx) plane):
+//   yz pass (yz1_kernel, yz_kernel: one CTA or cluster per (field, kx) plane):
 //       D --DFT_yz--> D_hat;  u_hat += m1 u_hat + m2 D_hat  (pointwise);
 //       u_hat --IDFT_yz--> Sm
 //
@@ -23,7 +23,7 @@
 //   c_hat_new = (c_hat + D_mean K2 dt mu_hat) / (1 + D_mean dt kappa_c K4)  (CH, :976-983)
 // written as an increment so that the state never takes an FP32 round trip
 // through an FFT.  The variable-mobility term dt G J'_hat / (...) of :976-983 is
-// added by a second x/yz pass pair (xj pass + yz_kernel in C2 mode).
+// added by a second x/yz pass pair (xj pass + the yz kernel in C2 mode).
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -56,8 +56,7 @@ enum Mobility { MOB_CONST = 0, MOB_REF_VAR = 1, MOB_C1MC = 2 };
 
 // Device-side description of one run (all runs of a launch share one shape)
 struct RunParams {
-  float2* Sk;      // [nF][Kx] planes of the k-space state (digit-transposed y, z positions; the
-                   // order inside a plane belongs to the yz-pass variant that runs the batch)
+  float2* Sk;      // [nF][Kx] planes [kz][y position] of the k-space state
   float2* Sm;      // [nF] x Kx, Nz, Ny (strides ks, zs, 1): state in mixed space (x spectrum, real-space y, z)
   float2* D;       // as Sm: x-spectra of dF/dphi_i and dF/dc
   float* mob;      // [Nz][Ny][Nx] mobility minus D_mean (variable mobility only)
@@ -904,8 +903,8 @@ __global__ void __launch_bounds__(T, MINB) x_pass_kernel(const RunParams* __rest
 
 // ---------------------------------------------------------------------------
 // yz pass.  The state of every field is kept in full k-space,
-//     Sk[f][kx][ypos][zpos] = u_hat (normalised like f_trans, src/f_trans.f90:12),
-// in the digit-transposed position order of the y and z transforms, and is
+//     Sk[f][kx][kz][ypos] = u_hat (normalised like f_trans, src/f_trans.f90:12),
+// y in the digit-transposed position order of its transform, and is
 // updated pointwise there (exact increment, no FFT round trip of the state).
 // Per (field, kx) plane the yz pass
 //   * transforms D~ (the x pass output, mixed space) forward over y and z,
@@ -1195,6 +1194,7 @@ __device__ __forceinline__ void st_peer(uint32_t a, float2 v) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
 }
 
+// run pass (forward or inverse) over NL lines of length L, pitch P, T threads
 template <int L, int NL, int P, int T, bool INV>
 __device__ __forceinline__ void passB(float2* buf) {
   constexpr int N1 = Line<L>::N1, N2 = Line<L>::N2;
@@ -1414,7 +1414,7 @@ __global__ void __launch_bounds__(T, MINB) yz1_kernel(const RunParams* __restric
 // bounds several CTAs per SM is the shared-memory data pipe, so it gains at
 // 64^2 (64 runs of 64^3 x 8: 509 -> 446 us, 5.6 TB/s), 96^2 (96^3 x 55: 207 ->
 // 198 us) and 80^2 (80^3 x 50: 97 -> 90 us).
-// What bounds it: barriers and shared memory; DRAM at 50 to 80 % of its rate.
+// What bounds it: the load/store pipe (53 to 60 %) and barriers; DRAM at 42 to 82 % of its rate.
 // One item of P1 at a time: 32 values in flight (unroll 2 to 4) cost 1 to 2 %.
 // ---------------------------------------------------------------------------
 template <int NY, int NZ, int C, bool RAWP, int ZA, int ZB, int ZP>

@@ -1,7 +1,7 @@
-// Plain FP64 GPU path: cuFFT D2Z/Z2D plus one simple kernel per phase of the
-// reference loop body, following its 7*var+9 transforms per step.  It is the
-// comparator for the fused FP32 path and an FP64 GPU cross-check of the CPU
-// oracle; it is not the performance path.
+// FP64 GPU path: cuFFT D2Z/Z2D and plain kernels for the phases of the
+// reference loop body, 2 var + 3 transforms per step (2 more with variable
+// mobility).  It is the comparator for the fused FP32 path, an FP64 GPU
+// cross-check of the CPU oracle, and what runs grids outside the fused list.
 #pragma once
 #include "../../include/pfgpu.h"
 
