@@ -457,9 +457,6 @@ static bool yz_ok(pf_batch* b, const YZKernels& k) {
   for (KernelFn f : {k.main, k.c2, k.imp}) {
     if (cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem) != cudaSuccess)
       return false;
-    if (k.cluster > 8 &&
-        cudaFuncSetAttribute((const void*)f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-      return false;
   }
   return yz_clusters(b, k) >= 1;
 }
