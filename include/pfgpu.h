@@ -81,7 +81,9 @@ typedef struct pf_run pf_run;
 /* ---- step-level API (replaces src/var_diff.f90:474-1118) ---------------- */
 
 /* Create a run on cfg->device: validates the sizes, allocates the resident
- * state and builds the FP64 wavenumber/twiddle tables.  Supported grids on
+ * state and the buffer that its fields go in and out through (no later call of
+ * this group allocates device memory) and builds the FP64 wavenumber/twiddle
+ * tables.  Supported grids on
  * the fused FP32 path: Nx, Ny, Nz in {16, 32, 64, 80, 96, 102, 128, 160,
  * 200, 256} (the reference's weak-scaling grids included; every
  * (Ny, Nz) pair with Ny == Nz plus the non-cubic pairs listed by

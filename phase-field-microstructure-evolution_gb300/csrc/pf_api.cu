@@ -218,8 +218,7 @@ struct pf_batch {
   std::vector<RunParams> hrp;
   RunParams* drp = nullptr;
   void* mem = nullptr;         // all per-run buffers
-  float* fin = nullptr;        // float fields [nF][Nz][Ny][Nx] for the analysis (made on first use)
-  double* dstage = nullptr;    // one run's fields in the caller's layout, for memory the GPU does not reach (made on first use)
+  double* dstage = nullptr;    // one run's fields: in the caller's layout, for memory the GPU does not reach, or float for the analysis
   bool coherent = false;       // the GPU reads and writes the host's pages through their own page tables
   int ring = 0;
   cudaStream_t stream = nullptr;
@@ -523,21 +522,12 @@ static int env_int(const char* name, int dflt) {
   return v ? atoi(v) : dflt;
 }
 
-// The launch shape `sh` with the fields in the batch's staging buffer.
-static int stage(pf_batch* b, const Shape& sh, Shape& out) {
-  const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
-  if (!b->dstage) {
-    const cudaError_t e = cudaMalloc(&b->dstage, b->nF * ncell * sizeof(double));
-    if (e != cudaSuccess) {
-      b->dstage = nullptr;
-      cudaGetLastError();
-      return fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e));
-    }
-  }
-  out = sh;
-  out.io_phi = b->dstage;
-  out.io_con = b->dstage + (size_t)b->V * ncell;
-  return PF_OK;
+// The batch's launch shape with the fields in its staging buffer.
+static Shape staged(const pf_batch* b) {
+  Shape sh = b->tab.sh;
+  sh.io_phi = b->dstage;
+  sh.io_con = b->dstage + (size_t)b->V * b->Nx * b->Ny * b->Nz;
+  return sh;
 }
 
 // Whether kernels may read (write) `bytes` of the caller's memory themselves.
@@ -584,13 +574,10 @@ static int tune_batch(pf_batch* b) {
     } else if (env_int("PFGPU_AUTOTUNE", 1) != 0 && (xs.size() > 1 || ys.size() > 1)) {
       // synthetic non-zero state so that the bulk terms take their usual branches
       const size_t nfin = (size_t)b->nF * b->Nx * b->Ny * b->Nz;
-      Shape staged = {};
-      const int rs = stage(b, b->tab.sh, staged);
-      if (rs) return rs;
       fill_kernel<<<(unsigned)((nfin + 255) / 256), 256, 0, b->stream>>>(b->dstage, nfin, 0.3, 0.7);
       apply_variants(b, xv[xs[0]], yv[ys[0]]);
       const dim3 g1(b->Nz * (b->Ny / b->xk.wy), 1);
-      b->xk.imp<<<g1, b->xk.threads, b->smem_x, b->stream>>>(b->drp, staged);
+      b->xk.imp<<<g1, b->xk.threads, b->smem_x, b->stream>>>(b->drp, staged(b));
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
@@ -705,7 +692,6 @@ static void destroy_batch(pf_batch* b) {
   cudaFree(b->drp);
   cudaFree(b->mem);
   cudaFreeHost(b->hring);
-  cudaFree(b->fin);
   cudaFree(b->dstage);
   cudaFree(b->tab.base);
   delete b;
@@ -808,6 +794,9 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     b->hring = nullptr;
     cudaGetLastError();
   }
+  // here, not in the call that first needs it: a run that has done its steps must be able to hand out its fields
+  e = cudaMalloc(&b->dstage, b->nF * ncell * sizeof(double));
+  if (e != cudaSuccess) return bail(fail(PF_ENOMEM, "staging allocation: %s", cudaGetErrorString(e)));
   int coherent = 0;
   cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, b->device);
   b->coherent = coherent != 0;
@@ -882,8 +871,7 @@ static int batch_set_fields(pf_batch* b, int run, const double* phi, const doubl
     sh.io_phi = const_cast<double*>(phi);
     sh.io_con = const_cast<double*>(con);
   } else {
-    const int rs = stage(b, b->tab.sh, sh);
-    if (rs) return rs;
+    sh = staged(b);
     PF_CUDA(cudaMemcpyAsync(sh.io_phi, phi, bphi, cudaMemcpyHostToDevice, b->stream));
     PF_CUDA(cudaMemcpyAsync(sh.io_con, con, bcon, cudaMemcpyHostToDevice, b->stream));
   }
@@ -909,8 +897,7 @@ static int batch_get_fields(pf_batch* b, int run, double* phi, double* con) {
     sh.io_phi = phi;
     sh.io_con = con;
   } else {
-    const int rs = stage(b, b->tab.sh, sh);
-    if (rs) return rs;
+    sh = staged(b);
   }
   const dim3 gx(b->Nz * (b->Ny / b->xk.wy), 1);
   b->xk.exp<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp + run, sh);
@@ -923,25 +910,17 @@ static int batch_get_fields(pf_batch* b, int run, double* phi, double* con) {
   return PF_OK;
 }
 
-// Real-space fields of run 0 of a batch in the float staging buffer fin.
+// Real-space fields of run 0 of a batch, as floats in its staging buffer.
 static int batch_device_fields(pf_batch* b, DeviceFields* out) {
   PF_CUDA(cudaSetDevice(b->device));
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
   const dim3 gx(b->Nz * (b->Ny / b->xk.wy), 1);
-  if (!b->fin) {
-    const cudaError_t e = cudaMalloc(&b->fin, b->nF * ncell * sizeof(float));
-    if (e != cudaSuccess) {
-      b->fin = nullptr;
-      cudaGetLastError();
-      return fail(PF_ENOMEM, "float fields: %s", cudaGetErrorString(e));
-    }
-  }
   Shape sh = b->tab.sh;
-  sh.fin = b->fin;
+  sh.fin = reinterpret_cast<float*>(b->dstage);
   b->xk.fields<<<gx, b->xk.threads, b->smem_x, b->stream>>>(b->drp, sh);
   PF_CUDA(cudaGetLastError());
-  out->phi = b->fin;
-  out->con = b->fin + (size_t)b->V * ncell;
+  out->phi = sh.fin;
+  out->con = sh.fin + (size_t)b->V * ncell;
   out->is_double = 0;
   out->fstride = ncell;
   out->cstride = 1;

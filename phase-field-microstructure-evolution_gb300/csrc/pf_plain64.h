@@ -8,7 +8,7 @@
 namespace pf {
 // A run's real-space fields on its device: field f of cell i is
 // phi[f * fstride + i * cstride] (float or double), c contiguous; valid on
-// `stream` until the run is stepped or destroyed.
+// `stream` until the run is stepped or destroyed or its fields are set or got.
 struct DeviceFields {
   const void* phi;
   const void* con;
@@ -18,7 +18,7 @@ struct DeviceFields {
   void* stream;
 };
 // for either precision path (the fused path first transforms its spectral
-// state into its float staging buffer)
+// state into its staging buffer)
 int run_device_fields(pf_run* run, DeviceFields* out);
 
 struct Plain64;

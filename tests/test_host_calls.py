@@ -1,0 +1,73 @@
+"""The library's host code against a CUDA runtime of the host (fake_cuda.cpp):
+what it allocates and when, and how it leaves a call that fails.  No GPU."""
+import ctypes
+import importlib.util
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+DP = ctypes.POINTER(ctypes.c_double)
+PF_ENOMEM = -3
+
+
+@pytest.fixture(scope="module")
+def fake(pkg, lib, tmp_path_factory):
+    out = Path(pkg.__file__).parent / "_build"
+    home = importlib.util.spec_from_file_location("recipe", Path(pkg.__file__).parent / "build.py")
+    recipe = importlib.util.module_from_spec(home)
+    home.loader.exec_module(recipe)
+    so = tmp_path_factory.mktemp("fake") / "libpfgpu_fake.so"
+    objs = [str(out / (p.stem + ".o")) for p in recipe._sources()]
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", str(recipe.cuda_home() / "include"),
+                    str(ROOT / "tests" / "fake_cuda.cpp"), *objs, "-Wl,-Bsymbolic", "-Wl,-z,defs", "-lpthread",
+                    "-o", str(so)], check=True)
+    f = ctypes.CDLL(str(so))
+    f.fake_order.restype = f.pf_last_error.restype = ctypes.c_char_p
+    f.fake_reset()
+    return f
+
+
+@pytest.fixture(autouse=True)
+def clean(fake):
+    fake.fake_reset()
+
+
+def _ptr(a):
+    return a.ctypes.data_as(DP)
+
+
+class Run:
+    """A run of 16^3 cells and two order parameters, with host fields."""
+
+    def __init__(self, fake, pkg, oracle, precision=32, **more):
+        self.f = fake
+        cfg = pkg.make_config(oracle.Params(16, 16, 16, 2, **more), precision)
+        self.h = ctypes.c_void_p()
+        assert fake.pf_create(ctypes.byref(cfg), ctypes.byref(self.h)) == 0, fake.pf_last_error()
+        self.phi, self.con = np.zeros(16 ** 3 * 2), np.zeros(16 ** 3)
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *_):
+        self.f.pf_destroy(self.h)
+
+
+@pytest.mark.parametrize("coherent", [0, 1])
+@pytest.mark.parametrize("precision", [32, 64])
+def test_memory_is_allocated_when_the_run_is_made(fake, pkg, oracle, coherent, precision):
+    """After pf_create a run needs no more device memory to take fields, step and hand them out."""
+    fake.fake_coherent(coherent)
+    with Run(fake, pkg, oracle, precision, mobility="c1mc") as r:
+        fake.fake_fail(b"cudaMalloc", 1, 2)
+        assert fake.pf_set_fields(r.h, _ptr(r.phi), _ptr(r.con)) == 0
+        assert fake.pf_step(r.h, 5, None) == 0
+        assert fake.pf_get_fields(r.h, _ptr(r.phi), _ptr(r.con)) == 0, fake.pf_last_error()
+    fake.fake_reset()
+    if precision == 32:  # and where there is none, it is pf_create that says so
+        fake.fake_fail(b"cudaMalloc", 3, 2)
+        cfg, h = pkg.make_config(oracle.Params(16, 16, 16, 2)), ctypes.c_void_p()
+        assert fake.pf_create(ctypes.byref(cfg), ctypes.byref(h)) == PF_ENOMEM
