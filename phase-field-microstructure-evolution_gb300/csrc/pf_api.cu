@@ -867,6 +867,7 @@ static int batch_set_fields(pf_batch* b, int run, const double* phi, const doubl
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
   const size_t bphi = (size_t)b->V * ncell * sizeof(double), bcon = ncell * sizeof(double);
   Shape sh = b->tab.sh;
+  Drain drain{b->stream};
   if (direct(b, phi, bphi, false) && direct(b, con, bcon, false)) {
     sh.io_phi = const_cast<double*>(phi);
     sh.io_con = const_cast<double*>(con);
@@ -882,6 +883,7 @@ static int batch_set_fields(pf_batch* b, int run, const double* phi, const doubl
   PF_CUDA(cudaMemsetAsync(b->hrp[run].counter, 0, 256, b->stream));  // step counter
   PF_CUDA(cudaGetLastError());
   PF_CUDA(cudaStreamSynchronize(b->stream));
+  drain.armed = false;
   b->steps_done[run] = 0;
   return PF_OK;
 }
@@ -892,6 +894,7 @@ static int batch_get_fields(pf_batch* b, int run, double* phi, double* con) {
   const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
   const size_t bphi = (size_t)b->V * ncell * sizeof(double), bcon = ncell * sizeof(double);
   Shape sh = b->tab.sh;
+  Drain drain{b->stream};
   const bool own = direct(b, phi, bphi, true) && direct(b, con, bcon, true);
   if (own) {
     sh.io_phi = phi;
@@ -907,6 +910,7 @@ static int batch_get_fields(pf_batch* b, int run, double* phi, double* con) {
     PF_CUDA(cudaMemcpyAsync(con, sh.io_con, bcon, cudaMemcpyDeviceToHost, b->stream));
   }
   PF_CUDA(cudaStreamSynchronize(b->stream));
+  drain.armed = false;
   return PF_OK;
 }
 

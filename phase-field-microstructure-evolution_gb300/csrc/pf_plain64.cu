@@ -439,10 +439,12 @@ int plain64_create(const pf_config* c, Plain64** out) {
 int plain64_set_fields(Plain64* p, const double* phi, const double* con) {
   if (!p || !phi || !con) return fail64(PF_EINVAL, "bad arguments to set_fields");
   P64_CUDA(cudaSetDevice(p->device));
+  Drain drain{p->stream};
   P64_CUDA(cudaMemcpyAsync(p->dstage, phi, p->V * p->ncell * sizeof(double), cudaMemcpyHostToDevice, p->stream));
   p64_aos_to_soa<<<NB, NT, 0, p->stream>>>(p->dstage, p->phi, p->V, p->ncell);
   P64_CUDA(cudaMemcpyAsync(p->con, con, p->ncell * sizeof(double), cudaMemcpyHostToDevice, p->stream));
   P64_CUDA(cudaStreamSynchronize(p->stream));
+  drain.armed = false;
   p->steps = 0;
   p->have_fint = false;
   return PF_OK;
@@ -451,10 +453,12 @@ int plain64_set_fields(Plain64* p, const double* phi, const double* con) {
 int plain64_get_fields(Plain64* p, double* phi, double* con) {
   if (!p || !phi || !con) return fail64(PF_EINVAL, "bad arguments to get_fields");
   P64_CUDA(cudaSetDevice(p->device));
+  Drain drain{p->stream};
   p64_soa_to_aos<<<NB, NT, 0, p->stream>>>(p->phi, p->dstage, p->V, p->ncell);
   P64_CUDA(cudaMemcpyAsync(phi, p->dstage, p->V * p->ncell * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
   P64_CUDA(cudaMemcpyAsync(con, p->con, p->ncell * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
   P64_CUDA(cudaStreamSynchronize(p->stream));
+  drain.armed = false;
   return PF_OK;
 }
 
@@ -686,6 +690,7 @@ static int f_trans_impl(const double* in, double* out, int Nx, int Ny, int Nz, c
   int rc = shim_plans(Nx, Ny, Nz, &pl);
   if (rc) return rc;
   const size_t n = (size_t)Nx * Ny * Nz, ns = (size_t)(Nx / 2 + 1) * Ny * Nz;
+  Drain drain{nullptr};
   double* real = const_cast<double*>(in);  // a real-to-complex transform out of place leaves its input alone
   if (!reads_host(in, S.device)) {
     real = pl->real;
@@ -694,6 +699,7 @@ static int f_trans_impl(const double* in, double* out, int Nx, int Ny, int Nz, c
   P64_FFT(cufftExecD2Z(pl->f, real, pl->a));
   if ((rc = transpose(pl->a, pl->b, Nz, Ny, Nx / 2 + 1, 1.0 / (double)n))) return rc;
   P64_CUDA(cudaMemcpy(out, pl->b, ns * sizeof(cufftDoubleComplex), cudaMemcpyDeviceToHost));
+  drain.armed = false;
   return PF_OK;
 }
 
@@ -714,6 +720,7 @@ static int inv_trans_impl(const double* in, double* out, const int* ist, const i
   int rc = shim_plans(Nx, Ny, Nz, &pl);
   if (rc) return rc;
   const size_t n = (size_t)Nx * Ny * Nz, ns = (size_t)(Nx / 2 + 1) * Ny * Nz;
+  Drain drain{nullptr};
   const cufftDoubleComplex* spec = reinterpret_cast<const cufftDoubleComplex*>(in);
   if (!reads_host(in, S.device)) {
     spec = pl->b;
@@ -722,6 +729,7 @@ static int inv_trans_impl(const double* in, double* out, const int* ist, const i
   if ((rc = transpose(spec, pl->a, Nx / 2 + 1, Ny, Nz, 1.0))) return rc;
   P64_FFT(cufftExecZ2D(pl->i, pl->a, pl->real));
   P64_CUDA(cudaMemcpy(out, pl->real, n * sizeof(double), cudaMemcpyDeviceToHost));
+  drain.armed = false;
   return PF_OK;
 }
 

@@ -3,6 +3,8 @@
 // mobility).  It is the comparator for the fused FP32 path, an FP64 GPU
 // cross-check of the CPU oracle, and what runs grids outside the fused list.
 #pragma once
+#include <cuda_runtime.h>
+
 #include "../../include/pfgpu.h"
 
 namespace pf {
@@ -20,6 +22,16 @@ struct DeviceFields {
 // for either precision path (the fused path first transforms its spectral
 // state into its staging buffer)
 int run_device_fields(pf_run* run, DeviceFields* out);
+
+// Waits for a stream when the scope ends, unless disarmed by then: a call that
+// fails halfway must not leave a kernel or a copy at work on the caller's arrays.
+struct Drain {
+  cudaStream_t stream;
+  bool armed = true;
+  ~Drain() {
+    if (armed) cudaStreamSynchronize(stream);
+  }
+};
 
 struct Plain64;
 int plain64_device_fields(Plain64* p, DeviceFields* out);

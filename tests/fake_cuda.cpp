@@ -18,7 +18,7 @@ std::map<void*, int> device_mem, host_mem;  // device the block belongs to
 std::map<const void*, int> smem;            // kernels' shared-memory attribute
 std::map<cufftHandle, int> plan_device;
 std::string fail_name, order;  // the call that fails, the calls so far
-int fail_in = 0, fail_code = 0, coherent = 1, lowered = 0, strays = 0, next_plan = 1;
+int last = 0, fail_in = 0, fail_code = 0, coherent = 1, lowered = 0, strays = 0, next_plan = 1;
 thread_local int dev = 0;
 
 int hit(const char* name) {
@@ -26,8 +26,9 @@ int hit(const char* name) {
   ++counts[name];
   order += name;
   order += ' ';
-  if (fail_name == name && fail_in > 0 && --fail_in == 0) return fail_code;
-  return 0;
+  if (fail_name != name || fail_in == 0 || --fail_in > 0) return 0;
+  order += "FAILED ";
+  return last = fail_code;
 }
 // a call of device `dev` given memory of another one
 void check(const void* p) {
@@ -65,7 +66,7 @@ void fake_reset() {
   counts.clear();
   order.clear();
   fail_name.clear();
-  fail_in = lowered = strays = 0;
+  last = fail_in = lowered = strays = 0;
   coherent = 1;
 }
 void fake_fail(const char* name, int nth, int code) { fail_name = name, fail_in = nth, fail_code = code; }
@@ -131,7 +132,11 @@ cudaError_t cudaDeviceGetStreamPriorityRange(int* lo, int* hi) {
   return cudaSuccess;
 }
 const char* cudaGetErrorString(cudaError_t) { return "made to fail"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const int e = last;
+  last = 0;
+  return (cudaError_t)e;
+}
 cudaError_t cudaDeviceSynchronize() { CALL("cudaDeviceSynchronize"); }
 
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {

@@ -71,3 +71,26 @@ def test_memory_is_allocated_when_the_run_is_made(fake, pkg, oracle, coherent, p
         fake.fake_fail(b"cudaMalloc", 3, 2)
         cfg, h = pkg.make_config(oracle.Params(16, 16, 16, 2)), ctypes.c_void_p()
         assert fake.pf_create(ctypes.byref(cfg), ctypes.byref(h)) == PF_ENOMEM
+
+
+@pytest.mark.parametrize("call,step,nth", [("set", b"cudaLaunchKernelExC", 1), ("set", b"cudaMemsetAsync", 1),
+                                           ("get", b"cudaMemcpyAsync", 2), ("set64", b"cudaMemcpyAsync", 2),
+                                           ("get64", b"cudaMemcpyAsync", 2), ("f_trans", b"launch", 1),
+                                           ("inv_trans", b"cufftExec", 1)])
+def test_a_failed_call_leaves_the_callers_memory_alone(fake, pkg, oracle, call, step, nth):
+    """Kernels and copies already under way on the caller's arrays have ended when the call reports its error."""
+    with Run(fake, pkg, oracle, 64 if call.endswith("64") else 32) as r:
+        three = ctypes.c_int * 3
+        n, one, ien, fen = ctypes.c_int(16), three(1, 1, 1), three(16, 16, 16), three(16, 16, 9)
+        spec = np.zeros(2 * 9 * 256)
+        fake.fake_reset()
+        fake.fake_fail(step, nth, 700)
+        if call == "f_trans":
+            fake.f_trans_(_ptr(r.con), _ptr(spec), ctypes.byref(n), ctypes.byref(n), ctypes.byref(n), one, ien, one, fen)
+        elif call == "inv_trans":
+            fake.inv_trans_(_ptr(spec), _ptr(r.con), one, ien, one, fen)
+        else:
+            fn = fake.pf_set_fields if call.startswith("set") else fake.pf_get_fields
+            assert fn(r.h, _ptr(r.phi), _ptr(r.con)) != 0
+        _, failed, after = fake.fake_order().decode().partition("FAILED")
+        assert failed and "cudaStreamSynchronize" in after, fake.fake_order()
