@@ -180,18 +180,15 @@ cudaError_t launch_classify(const Src<T>& s, int V, size_t n, double thr, cudaSt
                             unsigned long long* counts) {
   if constexpr (sizeof(T) == sizeof(double)) {
     if (s.cstride == (size_t)V && V > 1) {
-      // as many warps as share 48 KB, at least one (V <= 255: 65 KB; more go the general way)
+      // as many warps as share 48 KB, at least one (V = 255: 65 KB); beyond V = 799, 200 KB, the general way
       const size_t per_warp = (size_t)32 * (V | 1) * sizeof(double);
       const int warps = (int)std::max<size_t>(1, std::min<size_t>(kThreads / 32, (48u << 10) / per_warp));
       const size_t smem = warps * per_warp;
-      if (smem <= (200u << 10) &&
-          (smem <= (48u << 10) || cudaFuncSetAttribute(classify_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)smem) == cudaSuccess)) {
+      if (smem <= (200u << 10) && (smem <= (48u << 10) || raise_smem((const void*)classify_cells_kernel, smem))) {
         const size_t want = (n + 32 * warps - 1) / (32 * warps);
         classify_cells_kernel<<<(unsigned)std::min<size_t>(want, 152 * 4), warps * 32, smem, st>>>(s, V, n, thr, o, counts);
         return cudaGetLastError();
       }
-      cudaGetLastError();
     }
   }
   classify_kernel<T><<<grid_for(n), kThreads, 0, st>>>(s, V, n, thr, o, counts);

@@ -167,6 +167,25 @@ static const size_t kHostRings = (size_t)8 << 20;  // pinned memory a batch may 
 // diagnostics reduction's arrays (under 1 KB).  Both count against kMaxSmem.
 static size_t x_static_smem(int nx) { return (nx >= 96 ? (size_t)(nx + nx / 2) * sizeof(float2) : 0) + 1024; }
 
+// Dynamic shared memory a kernel may use is a per-function setting shared by
+// every batch in the process: only ever raise it, so that a batch of fewer
+// fields never lowers it under a live batch of the same grid with more fields.
+static std::mutex g_attr_mu;
+static std::map<std::pair<int, const void*>, int> g_attr_smem;
+bool raise_smem(const void* fn, size_t bytes) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_attr_mu);
+  int& cur = g_attr_smem[std::make_pair(dev, fn)];
+  if ((int)bytes <= cur) return true;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cur = (int)bytes;
+  return true;
+}
+
 // order parameters per run; the x pass must also fit (var+1) field lines of
 // its rows in shared memory (checked below)
 static const int kMaxVar = 255;
@@ -458,25 +477,6 @@ static bool yz_ok(pf_batch* b, const YZKernels& k) {
       return false;
   }
   return yz_clusters(b, k) >= 1;
-}
-
-// Dynamic shared memory a kernel may use is a per-function setting shared by
-// every batch in the process: only ever raise it, so that a batch of fewer
-// fields never lowers it under a live batch of the same grid with more fields.
-static std::mutex g_attr_mu;
-static std::map<std::pair<int, const void*>, int> g_attr_smem;
-static bool raise_smem(const void* fn, size_t bytes) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lk(g_attr_mu);
-  int& cur = g_attr_smem[std::make_pair(dev, fn)];
-  if ((int)bytes <= cur) return true;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  cur = (int)bytes;
-  return true;
 }
 
 static bool x_ok(pf_batch* b, const XKernels& k) {

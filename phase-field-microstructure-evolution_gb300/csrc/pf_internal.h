@@ -115,4 +115,8 @@ constexpr size_t x_smem_bytes(int nF, int wy) {
 
 void set_error(const std::string& msg);
 
+// Let kernel `fn` use `bytes` of dynamic shared memory on the current device;
+// false if it cannot.  The limit is the process's, so it is only ever raised.
+bool raise_smem(const void* fn, size_t bytes);
+
 }  // namespace pf

@@ -94,3 +94,14 @@ def test_a_failed_call_leaves_the_callers_memory_alone(fake, pkg, oracle, call, 
             assert fn(r.h, _ptr(r.phi), _ptr(r.con)) != 0
         _, failed, after = fake.fake_order().decode().partition("FAILED")
         assert failed and "cudaStreamSynchronize" in after, fake.fake_order()
+
+
+def test_analysis_never_lowers_a_kernels_shared_memory(fake, pkg, oracle):
+    """The limit is the process's: lowered for one call, it would fail another thread's larger one."""
+    fields = np.ones((256, 64))
+    counts = pkg.VoxelCounts()
+    for var in (255, 200, 230, 700, 193):
+        cfg = pkg.make_config(oracle.Params(4, 4, 4, var))
+        assert fake.pf_analyze_fields(ctypes.byref(cfg), _ptr(np.ones(64 * var)), _ptr(fields[0]), ctypes.c_double(0.3),
+                                      None, ctypes.byref(counts)) == 0
+    assert fake.fake_count(b"cudaFuncSetAttribute") > 0 and fake.fake_lowered() == 0
