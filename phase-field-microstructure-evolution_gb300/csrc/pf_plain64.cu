@@ -630,25 +630,39 @@ struct ShimCtx {
     cufftDoubleComplex* a = nullptr;
     cufftDoubleComplex* b = nullptr;
   };
-  std::map<std::tuple<int, int, int>, Plans> plans;
+  std::map<std::tuple<int, int, int, int>, Plans> plans;  // plans and memory belong to a device
 };
 static ShimCtx& shim() {
   static ShimCtx* s = new ShimCtx();
   return *s;
 }
 
-static int shim_plans(int Nx, int Ny, int Nz, ShimCtx::Plans** out) {
-  ShimCtx& S = shim();
-  auto key = std::make_tuple(Nx, Ny, Nz);
-  auto it = S.plans.find(key);
-  if (it != S.plans.end()) { *out = &it->second; return PF_OK; }
-  ShimCtx::Plans pl;
+static int make_shim_plans(int Nx, int Ny, int Nz, ShimCtx::Plans& pl) {
   const size_t n = (size_t)Nx * Ny * Nz, ns = (size_t)(Nx / 2 + 1) * Ny * Nz;
   P64_CUDA(cudaMalloc(&pl.real, n * sizeof(double)));
   P64_CUDA(cudaMalloc(&pl.a, ns * sizeof(cufftDoubleComplex)));
   P64_CUDA(cudaMalloc(&pl.b, ns * sizeof(cufftDoubleComplex)));
   P64_FFT(cufftPlan3d(&pl.f, Nz, Ny, Nx, CUFFT_D2Z));
   P64_FFT(cufftPlan3d(&pl.i, Nz, Ny, Nx, CUFFT_Z2D));
+  return PF_OK;
+}
+
+static int shim_plans(int Nx, int Ny, int Nz, ShimCtx::Plans** out) {
+  ShimCtx& S = shim();
+  auto key = std::make_tuple(S.device, Nx, Ny, Nz);
+  auto it = S.plans.find(key);
+  if (it != S.plans.end()) { *out = &it->second; return PF_OK; }
+  ShimCtx::Plans pl;
+  const int rc = make_shim_plans(Nx, Ny, Nz, pl);
+  if (rc) {
+    for (cufftHandle h : {pl.f, pl.i})
+      if (h) cufftDestroy(h);
+    cudaFree(pl.real);
+    cudaFree(pl.a);
+    cudaFree(pl.b);
+    cudaGetLastError();  // reported: not to be taken for the next call's
+    return rc;
+  }
   S.plans[key] = pl;
   *out = &S.plans[key];
   return PF_OK;

@@ -105,3 +105,40 @@ def test_analysis_never_lowers_a_kernels_shared_memory(fake, pkg, oracle):
         assert fake.pf_analyze_fields(ctypes.byref(cfg), _ptr(np.ones(64 * var)), _ptr(fields[0]), ctypes.c_double(0.3),
                                       None, ctypes.byref(counts)) == 0
     assert fake.fake_count(b"cudaFuncSetAttribute") > 0 and fake.fake_lowered() == 0
+
+
+class Shim:
+    """f_trans_ of a grid no other test uses."""
+
+    def __init__(self, fake, nx, ny, nz):
+        three = ctypes.c_int * 3
+        self.f, self.n = fake, [ctypes.c_int(v) for v in (nx, ny, nz)]
+        self.one, self.ien, self.fen = three(1, 1, 1), three(nx, ny, nz), three(nz, ny, nx // 2 + 1)
+        self.real, self.spec = np.zeros(nx * ny * nz), np.zeros(2 * (nx // 2 + 1) * ny * nz)
+
+    def __call__(self):
+        self.f.f_trans_(_ptr(self.real), _ptr(self.spec), *map(ctypes.byref, self.n), self.one, self.ien, self.one, self.fen)
+
+
+def test_shims_use_what_belongs_to_their_device(fake):
+    shim = Shim(fake, 6, 4, 2)
+    try:
+        for device in (0, 1, 0, 1):
+            assert fake.pf_shim_device(device) == 0
+            shim()
+    finally:
+        fake.pf_shim_device(0)
+    assert fake.fake_strays() == 0
+    assert fake.fake_count(b"cufftPlan") == 4  # two a device, kept
+
+
+@pytest.mark.parametrize("step,nth", [(b"cudaMalloc", 1), (b"cudaMalloc", 3), (b"cufftPlan", 1), (b"cufftPlan", 2)])
+def test_shims_give_back_what_they_could_not_finish(fake, capfd, step, nth):
+    shim = Shim(fake, 6, 4, 10 + 2 * nth + len(step))
+    before = fake.fake_live()
+    fake.fake_fail(step, nth, 2)
+    shim()
+    assert b"FAILED" in fake.fake_order() and fake.fake_live() == before
+    assert "f_trans_" in capfd.readouterr().err
+    shim()  # and the next call makes them
+    assert fake.fake_count(b"cufftExec") == 1 and capfd.readouterr().err == ""
