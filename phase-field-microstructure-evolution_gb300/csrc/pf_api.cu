@@ -759,7 +759,11 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     if (mob_mode(&cfgs[i]) != MOB_CONST) b->mob = mob_mode(&cfgs[i]);
   get_x_kernels(b->Nx, &b->xk);
   get_yz_kernels(b->Ny, b->Nz, &b->yk);
-  auto bail = [&](int rc) { destroy_batch(b); return rc; };
+  auto bail = [&](int rc) {
+    destroy_batch(b);
+    cudaGetLastError();  // reported by rc: not to be taken for another call's
+    return rc;
+  };
   cudaError_t e = cudaSetDevice(b->device);
   if (e != cudaSuccess) return bail(fail(PF_ECUDA, "cudaSetDevice(%d): %s", b->device, cudaGetErrorString(e)));
   int rc = build_tables(b->Nx, b->Ny, b->Nz, b->nF, b->tab);

@@ -372,7 +372,11 @@ int plain64_create(const pf_config* c, Plain64** out) {
   p->Nx = c->nx; p->Ny = c->ny; p->Nz = c->nz; p->Kx = c->nx / 2 + 1; p->V = c->var;
   p->ncell = (size_t)p->Nx * p->Ny * p->Nz;
   p->nspec = (size_t)p->Kx * p->Ny * p->Nz;
-  auto bail = [&](int r) { plain64_destroy(p); return r; };
+  auto bail = [&](int r) {
+    plain64_destroy(p);
+    cudaGetLastError();  // reported by r: not to be taken for another call's
+    return r;
+  };
 #define TRY(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) \
     return bail(fail64(PF_ENOMEM, "%s: %s", #call, cudaGetErrorString(e_))); } while (0)
   TRY(cudaSetDevice(p->device));

@@ -142,3 +142,14 @@ def test_shims_give_back_what_they_could_not_finish(fake, capfd, step, nth):
     assert "f_trans_" in capfd.readouterr().err
     shim()  # and the next call makes them
     assert fake.fake_count(b"cufftExec") == 1 and capfd.readouterr().err == ""
+
+
+@pytest.mark.parametrize("precision,nth", [(32, 1), (32, 2), (32, 3), (64, 1), (64, 5)])
+def test_a_run_that_does_not_fit_is_no_error_of_the_others(fake, pkg, oracle, precision, nth):
+    cfg, h = pkg.make_config(oracle.Params(16, 16, 16, 2), precision), ctypes.c_void_p()
+    with Run(fake, pkg, oracle) as r:
+        before = fake.fake_live()
+        fake.fake_fail(b"cudaMalloc", nth, 2)
+        assert fake.pf_create(ctypes.byref(cfg), ctypes.byref(h)) < 0
+        assert fake.fake_live() == before
+        assert fake.pf_set_fields(r.h, _ptr(r.phi), _ptr(r.con)) == 0, fake.pf_last_error()
