@@ -168,14 +168,15 @@ __global__ void p64_bulk(const double* __restrict__ phi, const double* __restric
     // phase 5
     feta += -0.5 * ssq + 0.25 * den + c.sigma_1 * pairs + c.sigma_2 * S * aP;
     // phase 6
-    const double rden = 1.0 / den, r2 = rden * rden;
+    const double rden = 1.0 / den;
     const double pm = num * rden, pp = 1.0 - pm;
     const double dm = cc - c.con_0_mat, dp = cc - c.con_0_ppt;
     const double fmat = c.am * dm * dm, fppt = c.ap * dp * dp;
     fch += pm * fmat + pp * fppt;
     dfdc[i] = 2.0 * (pm * c.am * dm + pp * c.ap * dp);
-    // phases 7-9: dF = phi (phi^2 - 1 + 2 Gamma) + term4
-    const double t4 = 4.0 * (aP * aP) * r2 * (fmat - fppt);
+    // phases 7-9: dF = phi (phi^2 - 1 + 2 Gamma) + term4, its factors as ratios to
+    // sum phi^4, whose square leaves the range of a double at |phi| = 1e-39
+    const double t4 = 4.0 * (aP * aP * rden) * rden * (fmat - fppt);
     const double g0 = 2.0 * c.sigma_2 * aP - 1.0;
     for (int iv = 0; iv < P; ++iv) {
       const double f = phi[iv * n + i], a = f * f;
@@ -184,7 +185,7 @@ __global__ void p64_bulk(const double* __restrict__ phi, const double* __restric
       psi[iv * n + i] = f - Ldt * d;
     }
     {
-      const double d = fP * (aP - 1.0 + 2.0 * c.sigma_2 * S + 4.0 * aP * num * r2 * (fppt - fmat));
+      const double d = fP * (aP - 1.0 + 2.0 * c.sigma_2 * S + 4.0 * (aP * rden) * pm * (fppt - fmat));
       if (!isfinite(d)) bad += 1;
       psi[P * n + i] = fP - Ldt * d;
     }
