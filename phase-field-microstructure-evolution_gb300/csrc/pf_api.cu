@@ -442,9 +442,16 @@ static int launch_steps(pf_batch* b, int n) {
 // kernels.  PFGPU_AUTOTUNE=0 keeps the default variants; PFGPU_X_VARIANT /
 // PFGPU_YZ_VARIANT force one.
 // ---------------------------------------------------------------------------
-__global__ void fill_kernel(double* p, size_t n, double v0, double v1) {
+// A state that steps of any run leave much as it is, so that the bulk terms take
+// their usual branch throughout: grains of one order parameter each (64 cells
+// along x and y), traces of the others, c near 1/2.  (Fields of 0.3 and 0.7
+// everywhere grew without bound at 56 of them.)
+__global__ void fill_kernel(double* phi, double* con, int V, size_t ncell) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) p[i] = (i & 1) ? v1 : v0;
+  if (i >= ncell) return;
+  const int owner = (int)(i / 64 % V);
+  for (int f = 0; f < V; ++f) phi[i * V + f] = f == owner ? 0.95 : 0.02;
+  con[i] = i & 1 ? 0.52 : 0.48;
 }
 
 static std::mutex g_tune_mu;
@@ -572,12 +579,15 @@ static int tune_batch(pf_batch* b) {
       by = std::get<1>(it->second);
       bj = std::get<2>(it->second);
     } else if (env_int("PFGPU_AUTOTUNE", 1) != 0 && (xs.size() > 1 || ys.size() > 1)) {
-      // synthetic non-zero state so that the bulk terms take their usual branches
-      const size_t nfin = (size_t)b->nF * b->Nx * b->Ny * b->Nz;
-      fill_kernel<<<(unsigned)((nfin + 255) / 256), 256, 0, b->stream>>>(b->dstage, nfin, 0.3, 0.7);
+      // every run of the batch holds the synthetic state, in both spaces
       apply_variants(b, xv[xs[0]], yv[ys[0]]);
-      const dim3 g1(b->Nz * (b->Ny / b->xk.wy), 1);
-      b->xk.imp<<<g1, b->xk.threads, b->smem_x, b->stream>>>(b->drp, staged(b));
+      const size_t ncell = (size_t)b->Nx * b->Ny * b->Nz;
+      const Shape in = staged(b);
+      fill_kernel<<<(unsigned)((ncell + 255) / 256), 256, 0, b->stream>>>(in.io_phi, in.io_con, b->V, ncell);
+      const dim3 gi(b->Nz * (b->Ny / b->xk.wy), b->nruns);
+      b->xk.imp<<<gi, b->xk.threads, b->smem_x, b->stream>>>(b->drp, in);
+      const int ri = launch_yz(b, b->yk.imp, b->nF * b->Kx, b->drp, b->nruns, b->stream);
+      if (ri) return ri;
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
@@ -622,6 +632,16 @@ static int tune_batch(pf_batch* b) {
         for (int i : ys)
           fprintf(stderr, "pfgpu autotune %s yz %d cluster=%d threads=%d: %.4f ms/step%s\n", key, i, yv[i].cluster,
                   yv[i].threads, ty[i] / REPS, i == by ? " (chosen)" : "");
+        // and the state that the last of the timed steps found: the least sum phi^2 of its cells
+        for (int r = 0; r < b->nruns; ++r) {
+          int n = 0;
+          double d[DR_COUNT] = {};
+          PF_CUDA(cudaMemcpy(&n, b->hrp[r].counter, sizeof n, cudaMemcpyDeviceToHost));
+          PF_CUDA(cudaMemcpy(d, b->hrp[r].diag + (size_t)((n + b->ring - 1) % b->ring) * DR_COUNT, sizeof d,
+                             cudaMemcpyDeviceToHost));
+          fprintf(stderr, "pfgpu autotune %s run %d: phi_min %.3g, %g non-finite\n", key, r, d[DR_PHIMIN],
+                  d[DR_NONFINITE]);
+        }
       }
       // the xj pass (variable mobility) alone, over every variant that fits one field
       apply_variants(b, xv[bx], yv[by]);
