@@ -169,7 +169,7 @@ int grid_for(size_t n) {
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
     if (e_ != cudaSuccess) {                                                           \
-      set_error(std::string("analysis: ") + #call + ": " + cudaGetErrorString(e_));   \
+      set_cuda_error(std::string("analysis: ") + #call + ": " + cudaGetErrorString(e_)); \
       rc = PF_ECUDA;                                                                   \
       goto done;                                                                       \
     }                                                                                  \
@@ -297,7 +297,7 @@ extern "C" int pf_analyze_fields(const pf_config* cfg, const double* phi_aos, co
       s.con = dev + n * V;
     }
     if (e != cudaSuccess) {
-      set_error(std::string("analysis: ") + cudaGetErrorString(e));
+      set_cuda_error(std::string("analysis: ") + cudaGetErrorString(e));
       rc = e == cudaErrorMemoryAllocation ? PF_ENOMEM : PF_ECUDA;
     }
   }

@@ -24,6 +24,10 @@ namespace pf {
 static thread_local std::string g_err;
 
 void set_error(const std::string& msg) { g_err = msg; }
+void set_cuda_error(const std::string& msg) {
+  g_err = msg;
+  cudaGetLastError();
+}
 
 static int fail(int code, const char* fmt, ...) {
   char buf[512];
@@ -31,7 +35,8 @@ static int fail(int code, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
-  g_err = buf;
+  if (code == PF_ECUDA || code == PF_ENOMEM) set_cuda_error(buf);
+  else set_error(buf);
   return code;
 }
 
@@ -779,11 +784,7 @@ static int create_batch(const pf_config* cfgs, int nruns, pf_batch** out) {
     if (mob_mode(&cfgs[i]) != MOB_CONST) b->mob = mob_mode(&cfgs[i]);
   get_x_kernels(b->Nx, &b->xk);
   get_yz_kernels(b->Ny, b->Nz, &b->yk);
-  auto bail = [&](int rc) {
-    destroy_batch(b);
-    cudaGetLastError();  // reported by rc: not to be taken for another call's
-    return rc;
-  };
+  auto bail = [&](int rc) { destroy_batch(b); return rc; };
   cudaError_t e = cudaSetDevice(b->device);
   if (e != cudaSuccess) return bail(fail(PF_ECUDA, "cudaSetDevice(%d): %s", b->device, cudaGetErrorString(e)));
   int rc = build_tables(b->Nx, b->Ny, b->Nz, b->nF, b->tab);

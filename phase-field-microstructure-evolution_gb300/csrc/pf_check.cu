@@ -115,7 +115,7 @@ extern "C" int pf_check_fp64(const pf_config* cfg, const double* phi_aos, const 
     std::vector<double> h((size_t)kCmpBlocks * kCmpQ);
     if (e == cudaSuccess) e = cudaMemcpy(h.data(), dpart, h.size() * sizeof(double), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
-      set_error(std::string("pf_check_fp64: ") + cudaGetErrorString(e));
+      set_cuda_error(std::string("pf_check_fp64: ") + cudaGetErrorString(e));
       rc = PF_ECUDA;
     } else {
       double q[kCmpQ] = {0, 0, 0, 0, 0, 0, 0, 0};

@@ -114,6 +114,9 @@ constexpr size_t x_smem_bytes(int nF, int wy) {
 }
 
 void set_error(const std::string& msg);
+// ... of a call that failed in CUDA: the runtime's last error has been reported
+// with it and is not to be taken for the next call's.
+void set_cuda_error(const std::string& msg);
 
 // Let kernel `fn` use `bytes` of dynamic shared memory on the current device;
 // false if it cannot.  The limit is the process's, so it is only ever raised.

@@ -176,7 +176,7 @@ int scratch_in_current_context(double** out) {
   void* p = nullptr;
   const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
   if (e != cudaSuccess || !p) {
-    set_error(std::string("pf_diag_fields_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
+    set_cuda_error(std::string("pf_diag_fields_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
     return PF_ECUDA;
   }
   *out = static_cast<double*>(p);
@@ -229,7 +229,7 @@ extern "C" int pf_diag_fields_noalloc(const pf_config* cfg, const float* d_field
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, rec, sizeof h, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
-    set_error(std::string("pf_diag_fields_noalloc: ") + cudaGetErrorString(e));
+    set_cuda_error(std::string("pf_diag_fields_noalloc: ") + cudaGetErrorString(e));
     return PF_ECUDA;
   }
   out->step = 0;

@@ -40,7 +40,8 @@ static int fail64(int code, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
-  set_error(buf);
+  if (code == PF_ECUDA || code == PF_ENOMEM) set_cuda_error(buf);
+  else set_error(buf);
   return code;
 }
 
@@ -371,11 +372,7 @@ int plain64_create(const pf_config* c, Plain64** out) {
   p->Nx = c->nx; p->Ny = c->ny; p->Nz = c->nz; p->Kx = c->nx / 2 + 1; p->V = c->var;
   p->ncell = (size_t)p->Nx * p->Ny * p->Nz;
   p->nspec = (size_t)p->Kx * p->Ny * p->Nz;
-  auto bail = [&](int r) {
-    plain64_destroy(p);
-    cudaGetLastError();  // reported by r: not to be taken for another call's
-    return r;
-  };
+  auto bail = [&](int r) { plain64_destroy(p); return r; };
 #define TRY(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) \
     return bail(fail64(PF_ENOMEM, "%s: %s", #call, cudaGetErrorString(e_))); } while (0)
   TRY(cudaSetDevice(p->device));
@@ -681,7 +678,6 @@ static int shim_plans(int Nx, int Ny, int Nz, ShimCtx::Plans** out) {
     cudaFree(pl.real);
     cudaFree(pl.a);
     cudaFree(pl.b);
-    cudaGetLastError();  // reported: not to be taken for the next call's
     return rc;
   }
   S.plans[key] = pl;

@@ -40,14 +40,14 @@ def _ptr(a):
 
 
 class Run:
-    """A run of 16^3 cells and two order parameters, with host fields."""
+    """A run of 16^3 cells, with host fields."""
 
-    def __init__(self, fake, pkg, oracle, precision=32, **more):
+    def __init__(self, fake, pkg, oracle, precision=32, var=2, **more):
         self.f = fake
-        cfg = pkg.make_config(oracle.Params(16, 16, 16, 2, **more), precision)
+        cfg = pkg.make_config(oracle.Params(16, 16, 16, var, **more), precision)
         self.h = ctypes.c_void_p()
         assert fake.pf_create(ctypes.byref(cfg), ctypes.byref(self.h)) == 0, fake.pf_last_error()
-        self.phi, self.con = np.zeros(16 ** 3 * 2), np.zeros(16 ** 3)
+        self.phi, self.con = np.zeros(16 ** 3 * var), np.zeros(16 ** 3)
 
     def __enter__(self):
         return self
@@ -160,3 +160,23 @@ def test_an_fp64_run_is_one_allocation(fake, pkg, oracle):
     with Run(fake, pkg, oracle, 64, mobility="c1mc"):
         assert fake.fake_count(b"cudaMalloc") == 1 and fake.fake_count(b"cufftPlan") == 4
     assert fake.fake_count(b"cudaFree") == 1
+
+
+@pytest.mark.parametrize("call,step", [("analyze", b"cudaMalloc"), ("analyze_run", b"cudaMalloc"), ("set", b"cudaMemcpyAsync"),
+                                       ("get", b"cudaMemcpyAsync"), ("set64", b"cudaMemcpyAsync"), ("f_trans", b"cudaMemcpy")])
+def test_a_failed_call_is_no_error_of_the_next_one(fake, pkg, oracle, call, step):
+    cfg, counts = pkg.make_config(oracle.Params(16, 16, 16, 3)), pkg.VoxelCounts()
+    more = ctypes.c_double(0.3), None, ctypes.byref(counts)
+    fake.fake_coherent(0)  # fields go in by copies
+    with Run(fake, pkg, oracle) as other, Run(fake, pkg, oracle, 64 if call == "set64" else 32, var=3) as r:
+        fake.fake_fail(step, 1, 2)
+        if call == "analyze":
+            assert fake.pf_analyze_fields(ctypes.byref(cfg), _ptr(r.phi), _ptr(r.con), *more) < 0
+        elif call == "analyze_run":
+            assert fake.pf_analyze_run(r.h, *more) < 0
+        elif call == "f_trans":
+            Shim(fake, 6, 4, 8)()
+        else:
+            assert (fake.pf_get_fields if call == "get" else fake.pf_set_fields)(r.h, _ptr(r.phi), _ptr(r.con)) < 0
+        assert b"FAILED" in fake.fake_order()
+        assert fake.pf_set_fields(other.h, _ptr(other.phi), _ptr(other.con)) == 0, fake.pf_last_error()
