@@ -157,12 +157,12 @@ __global__ void __launch_bounds__(kThreads) grad3_kernel(const double* __restric
   }
 }
 
-int grid_for(size_t n) {
+// Blocks for n items, `per_block` at a time, at most `per_sm` of them an SM.
+unsigned grid_for(size_t n, size_t per_block = kThreads, int per_sm = 8) {
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t want = (n + kThreads - 1) / kThreads;
-  return (int)std::min<size_t>(want, (size_t)sms * 8);
+  return (unsigned)std::min<size_t>((n + per_block - 1) / per_block, (size_t)sms * per_sm);
 }
 
 #define AN_CUDA(call)                                                                  \
@@ -185,8 +185,7 @@ cudaError_t launch_classify(const Src<T>& s, int V, size_t n, double thr, cudaSt
       const int warps = (int)std::max<size_t>(1, std::min<size_t>(kThreads / 32, (48u << 10) / per_warp));
       const size_t smem = warps * per_warp;
       if (smem <= (200u << 10) && (smem <= (48u << 10) || raise_smem((const void*)classify_cells_kernel, smem))) {
-        const size_t want = (n + 32 * warps - 1) / (32 * warps);
-        classify_cells_kernel<<<(unsigned)std::min<size_t>(want, 152 * 4), warps * 32, smem, st>>>(s, V, n, thr, o, counts);
+        classify_cells_kernel<<<grid_for(n, 32 * warps, 4), warps * 32, smem, st>>>(s, V, n, thr, o, counts);
         return cudaGetLastError();
       }
     }

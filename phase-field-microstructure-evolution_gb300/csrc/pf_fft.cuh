@@ -14,10 +14,11 @@
 // takes that order back to natural order.  The spectral update in between is
 // pointwise, so no reordering pass is ever needed.
 //
-// Each DFT of size <= 20 lives in registers (17 as a direct DFT); in shared memory every run of N1
-// consecutive elements is followed by one pad slot and the line pitch is odd,
-// which makes pass A, pass B and line-to-line transposes free of bank
-// conflicts for 8-byte complex elements.
+// Each DFT of size <= 20 lives in registers (17 as a direct DFT).  In shared
+// memory the y and z lines have one pad slot after every run of N1 consecutive
+// elements and an odd pitch (Line), which makes pass A, pass B and
+// line-to-line transposes free of bank conflicts for 8-byte complex elements;
+// the x lines have the odd pitch alone.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -57,7 +58,6 @@ PF_HD float2 cfma(float s, float2 a, float2 b) {
   return make_float2(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y));
 #endif
 }
-PF_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 // a * b
 PF_HD float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));

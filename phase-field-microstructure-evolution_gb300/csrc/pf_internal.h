@@ -107,12 +107,6 @@ inline bool get_yz_kernels(int ny, int nz, YZKernels* out) {
   return true;
 }
 
-// x-pass shared memory for nF fields
-template <int NX>
-constexpr size_t x_smem_bytes(int nF, int wy) {
-  return (size_t)nF * wy * XLine<NX / 2>::PITCH * sizeof(float2);
-}
-
 void set_error(const std::string& msg);
 // ... of a call that failed in CUDA: the runtime's last error has been reported
 // with it and is not to be taken for the next call's.

@@ -327,7 +327,7 @@ __device__ __forceinline__ int x_run_pair(int q) {
 
 // Inverse x transform, first half: read the half spectrum of line (f, yy)
 // for the run pair `pr` (from where SRC says), pre-process, inverse DFT_N1 of
-// each run, store the runs (pass B' output) into the padded line.
+// each run, store the runs (pass B' output) into the line.
 template <int M, int SRC = SPEC_GLOBAL, bool TWS = false>
 __device__ __forceinline__ void x_inv_runs(const float2* src, int ks, float2* line, int pr,
                                            const float2* __restrict__ twN) {  // src may be line (in place)
